@@ -464,6 +464,7 @@ FusedArgs fused_args(const mhd_ctx* ctx, int s, double dt, int in) {
     a.U = ::fields_of(ctx, ctx->U[in]);
     a.Uo = ::fields_of(ctx, ctx->U[1 - in]);
     a.Z = ::fields_of(ctx, ctx->Zb);
+    a.fs = (long long)ctx->ncell;
     a.FT = ctx->Fb ? ctx->Fb + (size_t)F_FT * ctx->ncell : nullptr;
     a.gdt = gam[s] * dt;
     a.zdt = zet[s] * dt;
@@ -556,88 +557,97 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     const double* d1s[3] = {p.dxxdx, p.dyydy, p.dzzdz};
     const double* d2s[3] = {p.d2xxdx2, p.d2yydy2, p.d2zzdz2};
     const int ns[3] = {nx, ny, nz};
-    size_t base_off[3], scaled_off[3];
+    size_t base_off[3], side_off[2];
     for (int ax = 0; ax < 3; ax++) {
         base_off[ax] = h.size();
         for (int i = 0; i < ns[ax]; i++) h.push_back(d1s[ax][i] * hs[ax]);
         for (int i = 0; i < ns[ax]; i++) h.push_back(d2s[ax][i] * hs[ax]);
         for (int i = 0; i < ns[ax]; i++) h.push_back(d1s[ax][i] * d1s[ax][i] * h2s[ax]);
     }
-    const double scales[3] = {ctx->k.ORE, ctx->k.ORE * ctx->k.C43, ctx->k.ORM};
-    for (int ax = 0; ax < 3; ax++) {
-        scaled_off[ax] = h.size();
-        for (int sc = 0; sc < 3; sc++) {
-            for (int i = 0; i < ns[ax]; i++) h.push_back(d2s[ax][i] * hs[ax] * scales[sc]);
-            for (int i = 0; i < ns[ax]; i++) h.push_back(d1s[ax][i] * d1s[ax][i] * h2s[ax] * scales[sc]);
-        }
+    auto c1 = [&](int ax, int i) { return h[base_off[ax] + i]; };
+    auto c2a = [&](int ax, int i) { return h[base_off[ax] + (size_t)ns[ax] + i]; };
+    auto c2b = [&](int ax, int i) { return h[base_off[ax] + 2 * (size_t)ns[ax] + i]; };
+    const double scales[4] = {ctx->k.ORE, ctx->k.ORE * ctx->k.C43, ctx->k.ORM, 1.0};
+    for (int ax = 0; ax < 2; ax++) {
+        side_off[ax] = h.size();
+        for (int k = 0; k < 4; k++)
+            for (int sg = 1; sg >= -1; sg -= 2)
+                for (int i = 0; i < ns[ax]; i++) h.push_back(scales[k] * (c2b(ax, i) + sg * c2a(ax, i)));
     }
-    const size_t kap_off = h.size();
-    const double tmpc = ctx->k.OCV / ctx->k.REPR;
-    for (int i = 0; i < nz; i++) h.push_back(tmpc * p.RKAPA[i]);
-    for (int i = 0; i < nz; i++) h.push_back(tmpc * p.DKAPA[i]);
-    for (int i = 0; i < nz; i++) h.push_back(tmpc * p.DKAPA[i] * h[base_off[2] + i]);
     bool uxy = true;
     for (int i = 0; i < nx; i++) uxy = uxy && p.d2xxdx2[i] == 0.0;
     for (int i = 0; i < ny; i++) uxy = uxy && p.d2yydy2[i] == 0.0;
     // ... and the same first-derivative and 'b' coefficients in every interior column
-    auto same = [&](size_t off, int n) {
-        bool eq = true;
-        for (int i = 2; i <= n - 2; i++) eq = eq && h[off + i] == h[off + 1];
-        return eq;
-    };
-    for (int ax = 0; ax < 2 && uxy; ax++) {
-        uxy = same(base_off[ax], ns[ax]) && same(base_off[ax] + 2 * (size_t)ns[ax], ns[ax]);
-        for (int k = 1; k < 6 && uxy; k += 2) uxy = same(scaled_off[ax] + (size_t)k * ns[ax], ns[ax]);
-    }
-    // Per-z tables of the fused substage on uniform x / y grids (the x / y
-    // coefficients are then the interior column 1's); each records its offset.
-    auto push_z = [&](auto value_at) {
-        const size_t off = h.size();
-        for (int z = 0; z < nz; z++) h.push_back(value_at(z));
-        return off;
-    };
-    auto c1 = [&](int ax, int i) { return h[base_off[ax] + i]; };
-    auto c2a = [&](int ax, int i) { return h[base_off[ax] + (size_t)ns[ax] + i]; };
-    auto c2b = [&](int ax, int i) { return h[base_off[ax] + 2 * (size_t)ns[ax] + i]; };
-    auto s2a = [&](int ax, int k, int i) { return h[scaled_off[ax] + (size_t)(2 * k) * ns[ax] + i]; };
-    auto s2b = [&](int ax, int k, int i) { return h[scaled_off[ax] + (size_t)(2 * k + 1) * ns[ax] + i]; };
-    size_t lapS_off[6], condT_off[5], lapZ_off[8];
-    // S = 2 (sx + sy + sz) of the Laplacians of u, v, w (viscous scales, C43 on the x, y, z
-    // axis), T (unscaled), B (resistive), and 2 (sx + sy) of B on the wall planes
-    {
-        const int kx[6] = {1, 0, 0, -1, 2, 2}, ky[6] = {0, 1, 0, -1, 2, 2}, kz[6] = {0, 0, 1, -1, 2, -2};
-        for (int set = 0; set < 6; set++)
-            lapS_off[set] = push_z([&](int z) {
-                const double sx = kx[set] < 0 ? c2b(0, 1) : s2b(0, kx[set], 1);
-                const double sy = ky[set] < 0 ? c2b(1, 1) : s2b(1, ky[set], 1);
-                const double sz = kz[set] == -2 ? 0.0 : kz[set] < 0 ? c2b(2, z) : s2b(2, kz[set], z);
-                return 2.0 * (sx + sy + sz);
-            });
-    }
-    // the viscous cross-term factors C13*ORE*cx1*cz1, C13*ORE*cy1*cz1 (the kernel's order)
-    const double c13ore = ctx->k.C13 * ctx->k.ORE;
-    const double kx13 = c13ore * c1(0, 1), ky13 = c13ore * c1(1, 1);
-    const size_t kxz_off = push_z([&](int z) { return kx13 * c1(2, z); });
-    const size_t kyz_off = push_z([&](int z) { return ky13 * c1(2, z); });
-    const size_t ocz1_off = push_z([&](int z) { return ctx->k.OBETA * c1(2, z); });
-    // conduction with kapz folded in: kapz cx2b, kapz cy2b, the factors of T(z+1) and
-    // T(z-1) kapz (cz2b +- cz2a) +- dkapz cz1, and kapz S_T
-    {
-        auto kz = [&](int z) { return h[kap_off + z]; };
-        auto dkz = [&](int z) { return h[kap_off + nz + z]; };
-        condT_off[0] = push_z([&](int z) { return kz(z) * c2b(0, 1); });
-        condT_off[1] = push_z([&](int z) { return kz(z) * c2b(1, 1); });
-        condT_off[2] = push_z([&](int z) { return kz(z) * (c2b(2, z) + c2a(2, z)) + dkz(z) * c1(2, z); });
-        condT_off[3] = push_z([&](int z) { return kz(z) * (c2b(2, z) - c2a(2, z)) - dkz(z) * c1(2, z); });
-        condT_off[4] = push_z([&](int z) { return kz(z) * (2.0 * (c2b(0, 1) + c2b(1, 1) + c2b(2, z))); });
-    }
-    // z second-derivative factors b + a and b - a of the planes above and below, for the
-    // scale pairs k = 0, 1, 2 (ORE, ORE*C43, ORM) and unscaled (k = 3)
-    for (int k = 0; k < 4; k++) {
-        auto za = [&](int z) { return k < 3 ? s2a(2, k, z) : c2a(2, z); };
-        auto zb = [&](int z) { return k < 3 ? s2b(2, k, z) : c2b(2, z); };
-        lapZ_off[2 * k] = push_z([&](int z) { return zb(z) + za(z); });
-        lapZ_off[2 * k + 1] = push_z([&](int z) { return zb(z) - za(z); });
+    for (int ax = 0; ax < 2; ax++)
+        for (int i = 2; i <= ns[ax] - 2; i++) uxy = uxy && c1(ax, i) == c1(ax, 1) && c2b(ax, i) == c2b(ax, 1);
+    // the unit of the uniform-grid kernels has to be an ordinary number
+    uxy = uxy && std::isnormal(c1(0, 1)) && std::isnormal(1.0 / c1(0, 1));
+    // The coefficient rows and scalars of the fused kernels (mhd_common.cuh), for
+    // any grid (kappa = 1) and, where it applies, for uniform x / y.
+    const double tmpc = ctx->k.OCV / ctx->k.REPR, c13ore = ctx->k.C13 * ctx->k.ORE;
+    size_t zt_off[2], sc_off[2];
+    for (int u = 0; u < 2; u++) {
+        const double kap = (u && uxy) ? c1(0, 1) : 1.0;
+        const double sT = (p.switches & MHD_SW_LSHR) ? 1.0 : 1.0 / kap;
+        zt_off[u] = h.size();
+        for (int z = 0; z < nz; z++) {
+            double r[ZR_N] = {};
+            const double cz = c1(2, z), za = c2a(2, z), zb = c2b(2, z);
+            const double kz = tmpc * p.RKAPA[z], dkz = tmpc * p.DKAPA[z];
+            const double bx = c2b(0, 1), by = c2b(1, 1);
+            auto centre = [&](int kx, int ky, int kk) {
+                return 2.0 * (scales[kx] * bx + scales[ky] * by + (kk < 0 ? 0.0 : scales[kk] * zb)) / kap;
+            };
+            r[ZR_CZ] = cz / kap;
+            for (int k = 0; k < 3; k++) {
+                r[ZR_SZ0 + 2 * k] = scales[k] * (zb + za) / kap;
+                r[ZR_SZ0 + 2 * k + 1] = scales[k] * (zb - za) / kap;
+            }
+            r[ZR_KZP] = u ? sT * (kz * (zb + za) + dkz * cz) : kz;
+            r[ZR_KZM] = u ? sT * (kz * (zb - za) - dkz * cz) : dkz * cz;
+            r[ZR_KX] = sT * kz * bx;
+            r[ZR_KY] = sT * kz * by;
+            r[ZR_SU] = centre(1, 0, 0);
+            r[ZR_SV] = centre(0, 1, 0);
+            r[ZR_SW] = centre(0, 0, 1);
+            r[ZR_ST] = sT * kz * (2.0 * (bx + by + zb));
+            r[ZR_SB] = centre(2, 2, 2);
+            r[ZR_SBW] = centre(2, 2, -1);
+            r[ZR_KQZ] = c13ore * cz;
+            r[ZR_OCZ] = ctx->k.OBETA * cz / kap;
+            r[ZR_TZP] = zb + za;
+            r[ZR_TZM] = zb - za;
+            r[ZR_STL] = 2.0 * (bx + by + zb);
+            r[ZR_WD2] = ctx->k.ORM * za / kap;
+            r[ZR_WD1] = ctx->k.ORM * zb / kap;
+            h.insert(h.end(), r, r + ZR_N);
+        }
+        double s[SC_N] = {};
+        s[SC_ONE] = 1.0;
+        s[SC_NZ] = -0.0;
+        s[SC_KAPPA] = kap;
+        s[SC_ST] = sT;
+        s[SC_CY] = c1(1, 1) / kap;
+        for (int k = 0; k < 3; k++) {
+            s[SC_SX0 + k] = scales[k] * c2b(0, 1) / kap;
+            s[SC_SY0 + k] = scales[k] * c2b(1, 1) / kap;
+        }
+        s[SC_KQX] = u ? c13ore * c1(0, 1) : c13ore;
+        s[SC_KQY] = u ? c13ore * c1(1, 1) : c13ore;
+        s[SC_GRAV] = p.GRAV / kap;
+        s[SC_OMZ] = ctx->k.OMZ / kap;
+        s[SC_OMX] = ctx->k.OMX / kap;
+        s[SC_HQ] = ctx->k.OCV * ctx->k.ORE * kap * kap * sT;
+        s[SC_MOCV] = -ctx->k.OCV * (kap * sT);
+        s[SC_C43] = ctx->k.C43;
+        s[SC_C43X3] = 3.0 * ctx->k.C43;
+        s[SC_OB] = ctx->k.OBETA;
+        s[SC_OHM] = ctx->k.OBETA != 0.0 ? ctx->k.ORM * ctx->k.OCV * kap * kap * sT / ctx->k.OBETA : 0.0;
+        s[SC_TX] = c2b(0, 1);
+        s[SC_TY] = c2b(1, 1);
+        s[SC_TMPC] = tmpc * sT;
+        sc_off[u] = h.size();
+        h.insert(h.end(), s, s + SC_N);
     }
     if (cudaMalloc(&ctx->d_metric, h.size() * sizeof(double)) != cudaSuccess ||
         cudaMemcpyAsync(ctx->d_metric, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream) !=
@@ -654,26 +664,21 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     c.dzzdz = m; c.d2zzdz2 = m + nz; c.DDZ = m + 2 * nz; c.RKAPA = m + 3 * nz; c.DKAPA = m + 4 * nz; m += 5 * nz;
     {
         const double* b0 = ctx->d_metric;
-        const double** c1s[3] = {&ctx->coef.cx1, &ctx->coef.cy1, &ctx->coef.cz1};
-        const double** c2as[3] = {&ctx->coef.cx2a, &ctx->coef.cy2a, &ctx->coef.cz2a};
-        const double** c2bs[3] = {&ctx->coef.cx2b, &ctx->coef.cy2b, &ctx->coef.cz2b};
-        for (int ax = 0; ax < 3; ax++) {
+        const double** c1s[2] = {&ctx->coef.cx1, &ctx->coef.cy1};
+        const double** c2as[2] = {&ctx->coef.cx2a, &ctx->coef.cy2a};
+        const double** c2bs[2] = {&ctx->coef.cx2b, &ctx->coef.cy2b};
+        for (int ax = 0; ax < 2; ax++) {
             *c1s[ax] = b0 + base_off[ax];
             *c2as[ax] = b0 + base_off[ax] + ns[ax];
             *c2bs[ax] = b0 + base_off[ax] + 2 * ns[ax];
-            for (int k = 0; k < 6; k++) ctx->coef.s2[ax][k] = b0 + scaled_off[ax] + (size_t)k * ns[ax];
+            for (int k = 0; k < 8; k++) (ax ? ctx->coef.yt : ctx->coef.xt)[k] = b0 + side_off[ax] + (size_t)k * ns[ax];
         }
-        ctx->coef.kapz = b0 + kap_off;
-        ctx->coef.dkapz = b0 + kap_off + nz;
-        ctx->coef.dkz = b0 + kap_off + 2 * (size_t)nz;
+        for (int u = 0; u < 2; u++) {
+            ctx->coef.zt[u] = b0 + zt_off[u];
+            ctx->coef.sc[u] = b0 + sc_off[u];
+        }
         ctx->coef.uniform_xy = uxy ? 1 : 0;
         ctx->coef.isotropic_xy = (uxy && c1(0, 1) == c1(1, 1)) ? 1 : 0;
-        for (int set = 0; set < 6; set++) ctx->coef.lapS[set] = b0 + lapS_off[set];
-        ctx->coef.kxz = b0 + kxz_off;
-        ctx->coef.kyz = b0 + kyz_off;
-        ctx->coef.ocz1 = b0 + ocz1_off;
-        for (int t = 0; t < 5; t++) ctx->coef.condT[t] = b0 + condT_off[t];
-        for (int t = 0; t < 8; t++) ctx->coef.lapZ[t] = b0 + lapZ_off[t];
     }
     c.C13 = ctx->k.C13; c.C23 = ctx->k.C23; c.C43 = ctx->k.C43;
     c.hx = ctx->k.hx; c.h2x = ctx->k.h2x; c.hy = ctx->k.hy; c.h2y = ctx->k.h2y; c.hz = ctx->k.hz; c.h2z = ctx->k.h2z;

@@ -117,6 +117,7 @@ void fill_args(const mhd_batch* b, const std::vector<double*>& U0, const std::ve
                 a.U = ctxops::fields_of(c, ubuf[cur]);
                 a.Uo = ctxops::fields_of(c, ubuf[1 - cur]);
                 a.Z = ctxops::fields_of(c, Z[i]);
+                a.fs = (long long)c->ncell;
                 a.FT = FT[i];
                 a.gdt = gam[s] * b->dt[i];
                 a.zdt = zet[s] * b->dt[i];

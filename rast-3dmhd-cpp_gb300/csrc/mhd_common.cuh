@@ -70,38 +70,63 @@ struct Fields8 {
     double* p[8];
 };
 
-// Metric coefficients premultiplied for the fused kernels:
-//   c1 = duudu*hu, c2a = d2uudu2*hu, c2b = duudu^2*h2u   per axis.
+// Coefficients of the fused FP64 kernels.  The kernels for uniform x and y
+// grids work in units of kappa = cx1 (the x metric factor duudu*hu, the same
+// in every column): every equation is divided by it and the RK coefficients
+// multiplied by it, except the temperature's with lShr, whose right-hand side
+// is kept from call to call in true units.  `sT` below is the scale of the
+// temperature equation, 1/kappa or (lShr) 1.  On other grids kappa = 1.
+//
+// One row per z (kZt rows follow one another, ZR_N doubles each):
+enum ZRow {
+    ZR_CZ = 0,    // cz1 / kappa (cz1 = dzzdz*hz)
+    ZR_SZ0,       // z second-derivative factors of the planes above and below, b + a and b - a
+                  // (a = d2zzdz2*hz, b = dzzdz^2*h2z), scaled by ORE, ORE*C43, ORM, over kappa: 6 entries
+    ZR_KZP = ZR_SZ0 + 6,  // conduction: the factors of T(z+1) and T(z-1), kapz (b +- a) +- dkapz cz1, with
+    ZR_KZM,               // kapz, dkapz = OCV/REPR * (RKAPA, DKAPA), times sT; other grids: kapz and dkapz cz1
+    ZR_KX, ZR_KY,         // kapz cx2b, kapz cy2b (cx2b = duudu^2*h2u), times sT
+    ZR_SU, ZR_SV, ZR_SW,  // centre coefficients 2 (sx + sy + sz) of the Laplacians of u, v, w,
+    ZR_ST, ZR_SB, ZR_SBW, // T (kapz and sT included) and B, and 2 (sx + sy) of B for the wall planes
+    ZR_KQZ,               // C13*ORE*cz1
+    ZR_OCZ,               // OBETA*cz1 / kappa
+    ZR_TZP, ZR_TZM, ZR_STL,  // the unscaled Laplacian's b + a, b - a and centre coefficient (lRem; other grids)
+    ZR_WD2, ZR_WD1,          // ORM a and ORM b over kappa: the one-sided d2B/dz2 on the walls
+    ZR_N
+};
+// Scalars, read through shared memory (a constant-bank operand makes a DFMA
+// slower); SC_ONE and SC_NZ are the 1 and -0 of the sums and products.
+enum Scalar {
+    SC_ONE = 0, SC_NZ,
+    SC_KAPPA, SC_ST,
+    SC_CY,                   // cy1 / kappa
+    SC_SX0,                  // cx2b scaled by ORE, ORE*C43, ORM, over kappa: 3 entries
+    SC_SY0 = SC_SX0 + 3,     // the same of y
+    SC_KQX = SC_SY0 + 3, SC_KQY,  // C13*ORE*cx1, C13*ORE*cy1; other grids: C13*ORE
+    SC_GRAV, SC_OMZ, SC_OMX,      // over kappa
+    SC_HQ,                   // OCV*ORE*kappa^2*sT, viscous heating
+    SC_MOCV,                 // -OCV*kappa*sT, pdV work
+    SC_C43, SC_C43X3,        // C43 and 3*C43
+    SC_OB,                   // OBETA
+    SC_OHM,                  // ORM*OCV*kappa^2*sT/OBETA (0 for OBETA = 0), Ohmic heating of OBETA j
+    SC_TX, SC_TY,            // cx2b, cy2b (lRem)
+    SC_TMPC,                 // OCV/REPR*sT (lRem)
+    SC_G, SC_Z, SC_GT, SC_ZT,  // filled by the kernel: gamma dt and zeta dt times kappa; of the temperature
+    SC_N
+};
 struct Coefs {
+    const double* zt[2];  // [nz][ZR_N]: any grid, uniform x / y
+    const double* sc[2];  // [SC_N]
+    // per column (any grid): first-derivative factors duudu*hu, second-derivative coefficients
+    // c2a = d2uudu2*hu, c2b = duudu^2*h2u
     const double *cx1, *cx2a, *cx2b;
     const double *cy1, *cy2a, *cy2b;
-    const double *cz1, *cz2a, *cz2b;
-    // second-derivative coefficients with the viscous and resistive scales
-    // folded in, per axis: ORE*c2a, ORE*c2b, ORE*C43*c2a, ORE*C43*c2b, ORM*c2a, ORM*c2b
-    const double* s2[3][6];
-    const double *kapz, *dkapz;  // (OCV/REPR)*RKAPA[z], (OCV/REPR)*DKAPA[z]
-    const double* dkz;           // dkapz[z] * cz1[z]
-    const double* ocz1;          // OBETA * cz1[z]
-    // with uniform_xy, per z: kapz*cx2b, kapz*cy2b, then the factors of T(z+1) and T(z-1)
-    // kapz*(cz2b + cz2a) + dkapz*cz1 and kapz*(cz2b - cz2a) - dkapz*cz1, and kapz*S_T
-    const double* condT[5];
-    // per z, for the scale pairs k = 0, 1, 2 (ORE, ORE*C43, ORM) and unscaled (k = 3):
-    // lapZ[2k] = b + a, lapZ[2k+1] = b - a of the z second-derivative coefficients
-    const double* lapZ[8];
+    // per column (any grid): c2b + c2a and c2b - c2a, scaled by ORE, ORE*C43, ORM and unscaled
+    const double *xt[8], *yt[8];
     // uniform x and y grids: d2xxdx2 and d2yydy2 vanish and the x / y
     // coefficients are the same in every interior column
     int uniform_xy;
-    // with uniform_xy: the same first-derivative coefficient on x and y
-    // (cx1 = cy1, equal spacings), so the x and y advection and induction
-    // terms of a component can share one metric product
+    // with uniform_xy: the same first-derivative coefficient on x and y (equal spacings)
     int isotropic_xy;
-    // with uniform_xy, per z: S = 2 (sx + sy + sz) of the second-derivative
-    // coefficients (the 'b' ones) of the Laplacians of u, v, w (viscous,
-    // C43 on the x, y, z axis respectively), T (plain), B (resistive), and
-    // 2 (sx + sy) of B for the wall planes
-    const double* lapS[6];
-    // with uniform_xy, per z: the viscous cross-term factors C13*ORE*cx1*cz1 and C13*ORE*cy1*cz1
-    const double *kxz, *kyz;
 };
 
 // ---- launchers implemented in the .cu files ----------------------------
@@ -139,6 +164,7 @@ struct FusedArgs {
     Fields8 U;     // state read (with ghosts)
     Fields8 Uo;    // state written (interior + x/y ghost images)
     Fields8 Z;     // RK register (read when substage > 0, written when substage < 2)
+    long long fs;  // the fields of U, Uo and Z each follow one another at this distance (elements)
     double* FT;    // persistent temperature right-hand side (lShr only)
     double gdt;    // GAM_k * dt
     double zdt;    // ZETA_k * dt

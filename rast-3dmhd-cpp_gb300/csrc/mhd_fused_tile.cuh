@@ -1,49 +1,50 @@
 // mhd_fused_tile.cuh -- the fused FP64 RK3 substage for one tile of columns.
 //
 // A CTA owns a TX x TY tile of (x, y) columns and marches down a range of z
-// planes.  Three z-planes of the tile plus a one-cell halo live in a
-// shared-memory ring; when plane z+2 is loaded its derived quantities (1/rho,
-// the velocities u = RU/rho, v, w and the diagonal momentum fluxes
-// p + RU u, p + RV v, p + RW w with the pressure p = rho*T) are computed once
-// per point, so every stencil reads them instead of recomputing them.
-// One thread per column then evaluates the whole right-hand side of fluxes()
-// (3dmhdsub.h:194-696) for cell (z, y, x), applies the RK update of
-// step_block_GAM (3dmhdsub.h:181-192), forms the next substage's register
-// Z' = U' + zeta*dt*F (step_block_ZETA, 3dmhdsub.h:168-179) and writes U'
-// together with its periodic ghost images (communicate(), 3dmhdmpi.h:11-143,
-// as dual stores).  BCON (3dmhdsub.h:720-873) on the wall planes follows in a
-// separate small kernel.
+// planes.  Three z planes of the tile plus a one-cell halo live in a
+// shared-memory ring; a plane's raw fields arrive by cp.async one plane ahead
+// and its derived quantities (1/rho, the velocities u = RU/rho, v, w and the
+// diagonal momentum fluxes p + RU u, p + RV v, p + RW w with p = rho T) are
+// computed once per point.  One thread per column then evaluates the whole
+// right-hand side of fluxes() (3dmhdsub.h:194-696) for cell (z, y, x), applies
+// the RK update of step_block_GAM (3dmhdsub.h:181-192), forms the next
+// substage's register Z' = U' + zeta*dt*F (step_block_ZETA, 3dmhdsub.h:168-179)
+// and writes U' together with its periodic ghost images (communicate(),
+// 3dmhdmpi.h:11-143, as dual stores).
 //
-// GB300 executes two FP64 FMAs per clock per SM, so this kernel is bound by
-// its FP64 instruction count, not by HBM; the right-hand side is regrouped for
-// the fewest FP64 instructions:
-//   * metric factors are premultiplied (c1 = duudu*hu, c2a = d2uudu2*hu,
-//     c2b = duudu^2*h2u), and the viscous (ORE, ORE*C43) and resistive (ORM)
-//     scales are folded into copies of c2a/c2b, so a scaled second derivative
-//     accumulates with three FMAs (five where d2uudu2 does not vanish);
-//   * UXY (uniform x and y grids: d2uudu2 = 0, the same coefficients in
-//     every column) drops the first-derivative part of the x/y second
-//     derivatives at compile time and sums each Laplacian as
-//     sx (px + mx) + sy (py + my) + pz (szb + sza) + mz (szb - sza) - c S with
-//     S = 2 (sx + sy + szb) and the z factors from per-z tables: one -2c
-//     product instead of one per axis, no (pz - mz) / (pz + mz); the
-//     conduction coefficient kappa(z) and the DKAPA dT/dz term are folded
-//     into the temperature's tables, and the cross-term factors are per-z
-//     tables too; with equal x and y spacings (cx1 = cy1) the x and y parts
-//     of each advection and induction component share one metric product;
-//   * with lShr (no temperature advection or heating) the velocity gradients
-//     feed only the induction terms, which are grouped per axis over raw
-//     differences with the metric factor applied once per group; without
-//     lShr the B differences stay raw and the metric factors ride in u cx1,
-//     v cy1, w cz1; OBETA rides in the current density;
-//   * the pressure is differenced together with the diagonal momentum flux
-//     (P + RU_i u_i, formed once per point, not once per neighbour), and the
-//     temperature terms proportional to 1/rho are summed before one multiply;
-//   * load_plane forms per point the z differences of u, v, w and the x
-//     differences of u, v (difference arrays after the ring), from which the
-//     viscous mixed derivatives are one subtraction of two neighbours' values;
-//   * repeated gradients are computed once; 1/rho is Newton's iteration
-//     r <- r + r(1 - rho r), twice, from the hardware reciprocal estimate.
+// GB300's FP64 unit takes 16 cycles of an SM for a warp's DFMA with three
+// register operands, but 19 for a DADD, a DMUL or a DFMA with a constant-bank
+// operand, whatever the number of active lanes (measured with one CTA per SM:
+// 2.00 against 1.68 lanes per clock).  The kernel is bound by that unit, so
+//   * every sum is fma(a, 1, b) and every product fma(a, b, -0), with the 1
+//     and the -0 read from memory so that they stay register operands; both
+//     are exactly a + b and a * b;
+//   * scalars and per-z coefficients come through shared memory instead of
+//     the constant bank;
+//   * points of the halo are packed into as few warps as they fill.
+// and the right-hand side is grouped for the fewest FP64 instructions:
+//   * advection and diffusion along one axis share their operands:
+//       -D(q RU) + s D2 q = q[+] (s+ - c RU[+]) + q[-] (s- + c RU[-]) - S q,
+//     where the two coefficients (formed once per axis) serve every momentum
+//     component without a C43 on that axis, and in the induction equation
+//     (with u instead of RU) all three components of B;
+//   * the diagonal momentum flux is differenced together with the pressure,
+//     before any product, as the two nearly cancel against gravity;
+//   * the viscous mixed derivatives are differences of sums of 1-D
+//     differences, Q1 = D_y v + D_z w (at x +- 1), Q2 = D_x u + D_z w (at
+//     y +- 1) and Q3 = D_x u + D_y v (at z +- 1, carried along the column),
+//     formed once per point;
+//   * uniform x and y grids (UXY) divide the equations by the x metric factor
+//     kappa, which the RK coefficients put back: x derivatives are then plain
+//     differences, and with equal x and y spacings (ISO) y derivatives too;
+//   * 1/rho is the hardware estimate (relative error e below 2^-20) times
+//     1 + e + e^2, three instructions for a remainder of order e^3.
+// Measured against the version before it (the same terms per cell with each
+// neighbour's products formed anew, plain sums and products, about 200 FP64
+// instructions per cell): a step at 512x512x256 (lMag, lRot, lShr) 68.9 ->
+// 55.4 ms, a batch of 24 instances 10.3 -> 8.3 ms per step, at 32x32x32 181 ->
+// 138 us; the FP64 unit is 90 % busy (184 instructions per cell and substage
+// at 256x256x128 with lMag).
 // Results agree with the reference to rounding (1e-12 of each field's
 // max-norm after a step, checked against the oracle).
 //
@@ -67,92 +68,45 @@ struct Tile {
     static constexpr int kPX = TX + 2;
     static constexpr int kPY = TY + 2;
     static constexpr int kPlane = kPX * kPY;
+    static constexpr int kHalo = kPlane - kThreads;
+    static_assert(kHalo <= kThreads, "one halo point per thread at most");
 };
 
-// quantities held per plane point; Q_PX, Q_PY, Q_PZ are the diagonal momentum
-// fluxes P + RU u, P + RV v, P + RW w (P = rho T), which both neighbours of a
-// point difference
-enum Q { Q_RU = 0, Q_RV, Q_RW, Q_TT, Q_RO, Q_RI, Q_U, Q_V, Q_W, Q_PX, Q_PY, Q_PZ, Q_BX, Q_BY, Q_BZ, Q_N };
+// quantities of a ring plane, with halo; Q_PX, Q_PY are the diagonal momentum
+// fluxes P + RU u, P + RV v (P = rho T), which both neighbours difference
+enum Q { Q_RU = 0, Q_RV, Q_TT, Q_U, Q_V, Q_W, Q_PX, Q_PY, Q_BX, Q_BY, Q_BZ, Q_N };
+// quantities kept for the thread's own column only: RW and P + RW w
+enum O { O_RW = 0, O_PZ, O_N };
 
 template <class SW>
 constexpr int nq() {
     return SW::lMag ? Q_N : Q_BX;
 }
+template <class SW>
+constexpr int nraw() {
+    return SW::lMag ? 8 : 5;
+}
 
-// per-point differences of the plane being computed, after the ring: the z
-// differences of u, v, w and the x differences of u, v (the viscous cross
-// terms difference them once more between neighbours)
-enum D { D_UZ = 0, D_VZ, D_WZ, D_UX, D_VX, D_N };
+constexpr int kZRing = 4;  // per-z coefficient rows in flight (z, z + 1 in use, z + 2 arriving)
 
+// shared memory, in doubles: ring [3][nq][plane], Q1 and Q2 [2][2][plane], raw
+// staging [nraw][plane], own columns [3][O_N][threads], coefficient rows, scalars
+template <class SW, class T>
+constexpr size_t ring_doubles() {
+    return (size_t)(3 * nq<SW>() + 4 + nraw<SW>()) * T::kPlane + (size_t)3 * O_N * T::kThreads + kZRing * ZR_N + SC_N;
+}
 template <class SW, class T>
 constexpr size_t ring_bytes() {
-    return ((size_t)3 * nq<SW>() + D_N) * T::kPlane * sizeof(double);
+    return ring_doubles<SW, T>() * sizeof(double);
 }
 
-// 1/x by Newton's iteration for the reciprocal, r <- r + r(1 - x r), applied
-// twice to the hardware estimate (each step doubles the correct bits).
-__device__ __forceinline__ double recip(double x) {
+// 1/x: r is the hardware estimate, e = 1 - x r, and 1/x = r / (1 - e) = r (1 + e + e^2) + O(e^3)
+__device__ __forceinline__ double recip(double x, double one) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-x, r, 1.0);
+    double e = fma(-x, r, one);
+    e = fma(e, e, e);
     return fma(r, e, r);
-}
-
-// Load plane z into ring slot `slot` with its derived quantities.  With
-// `diffs`, also the differences of plane z-1 into the difference arrays: the
-// z differences at each point from this plane and plane z-2, which the same
-// thread loaded at the same point, and the x differences from plane z-1,
-// which a barrier has made visible since its load.
-template <class SW, class T>
-__device__ __forceinline__ void load_plane(const FusedArgs& a, double* ring, int slot, int z, int x0, int y0,
-                                           bool diffs) {
-    constexpr int NQ = nq<SW>();
-    constexpr int kPlane = T::kPlane, kPX = T::kPX, kThreads = T::kThreads;
-    double* base = ring + (size_t)slot * NQ * kPlane;
-    const Grid& g = a.g;
-    for (int k = threadIdx.x; k < kPlane; k += kThreads) {
-        const int hx = k % kPX, hy = k / kPX;
-        const int gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-        if (gx >= g.nx || gy >= g.ny) continue;
-        const long long i = (long long)z * g.sz + (long long)gy * g.sy + gx;
-        const double ru = a.U.p[S_RU][i], rv = a.U.p[S_RV][i], rw = a.U.p[S_RW][i];
-        const double tt = a.U.p[S_TT][i], ro = a.U.p[S_RO][i];
-        const double ri = recip(ro);
-        base[Q_RU * kPlane + k] = ru;
-        base[Q_RV * kPlane + k] = rv;
-        base[Q_RW * kPlane + k] = rw;
-        base[Q_TT * kPlane + k] = tt;
-        base[Q_RO * kPlane + k] = ro;
-        base[Q_RI * kPlane + k] = ri;
-        // the stored, rounded products (not contracted into the differences below)
-        const double uu = __dmul_rn(ru, ri), vv = __dmul_rn(rv, ri), ww = __dmul_rn(rw, ri);
-        base[Q_U * kPlane + k] = uu;
-        base[Q_V * kPlane + k] = vv;
-        base[Q_W * kPlane + k] = ww;
-        const double p = __dmul_rn(ro, tt);
-        base[Q_PX * kPlane + k] = fma(ru, uu, p);
-        base[Q_PY * kPlane + k] = fma(rv, vv, p);
-        base[Q_PZ * kPlane + k] = fma(rw, ww, p);
-        if (diffs) {
-            const double* Pm2 = ring + (size_t)((slot + 1) % 3) * NQ * kPlane;  // plane z-2
-            const double* Pm1 = ring + (size_t)((slot + 2) % 3) * NQ * kPlane;  // plane z-1
-            double* Dp = ring + (size_t)3 * NQ * kPlane;
-            Dp[D_UZ * kPlane + k] = uu - Pm2[Q_U * kPlane + k];
-            Dp[D_VZ * kPlane + k] = vv - Pm2[Q_V * kPlane + k];
-            Dp[D_WZ * kPlane + k] = ww - Pm2[Q_W * kPlane + k];
-            if (hx >= 1 && hx <= kPX - 2) {
-                Dp[D_UX * kPlane + k] = Pm1[Q_U * kPlane + k + 1] - Pm1[Q_U * kPlane + k - 1];
-                Dp[D_VX * kPlane + k] = Pm1[Q_V * kPlane + k + 1] - Pm1[Q_V * kPlane + k - 1];
-            }
-        }
-        if constexpr (SW::lMag) {
-            base[Q_BX * kPlane + k] = a.U.p[S_BX][i];
-            base[Q_BY * kPlane + k] = a.U.p[S_BY][i];
-            base[Q_BZ * kPlane + k] = a.U.p[S_BZ][i];
-        }
-    }
 }
 
 // Store v at (z, y, x) and at every periodic ghost image of that cell.
@@ -168,70 +122,211 @@ __device__ __forceinline__ void store_with_images(double* F, const Grid& g, int 
     }
 }
 
-// acc + s * D2 F at a node from F[+1], F[-1], F[0], with s folded into
-// (c2a_s, c2b_s); HAS_A = false when d2uudu2 vanishes on this axis.
-template <bool HAS_A>
-__device__ __forceinline__ double acc_d2(double acc, double p, double m, double c, double c2a_s, double c2b_s) {
-    acc = fma(fma(-2.0, c, p + m), c2b_s, acc);
-    if constexpr (HAS_A) acc = fma(p - m, c2a_s, acc);
-    return acc;
-}
-
 // One tile (bx, by) of one instance, z planes [zb, ze) of the interior.
 // EXTRA: the instantiation with the optional temperature terms (the iTCon 2
 // plume heat sink, lRem); the others carry no code for them.  ISO (with UXY):
-// cx1 = cy1, the x and y parts of the advection and induction terms summed
-// before one metric product.
+// cx1 = cy1.
 template <class SW, class T, bool UXY, bool EXTRA = false, bool ISO = false>
-__device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by, int zb, int ze, double* ring) {
-    constexpr int NQ = nq<SW>();
-    constexpr int kTX = T::kTX, kPX = T::kPX, kPlane = T::kPlane, kTY = T::kTY;
+__device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by, int zb, int ze, double* smem) {
+    constexpr int NQ = nq<SW>(), NRAW = nraw<SW>();
+    constexpr int kTX = T::kTX, kPX = T::kPX, kPlane = T::kPlane, kTY = T::kTY, kThreads = T::kThreads;
+    constexpr int kOwn = O_N * kThreads, kRing = NQ * kPlane;
     const Grid& g = a.g;
     const Consts& c = a.c;
     const Coefs& K = a.k;
+    double* ring = smem;
+    double* qbuf = ring + 3 * kRing;           // [parity][Q1, Q2][plane]
+    double* stage = qbuf + 4 * kPlane;         // [nraw][plane]
+    double* own = stage + NRAW * kPlane;       // [slot][O_N][thread]
+    double* zrow = own + 3 * kOwn;             // [kZRing][ZR_N]
+    double* sc = zrow + kZRing * ZR_N;         // [SC_N]
+    const double* zt = K.zt[UXY ? 1 : 0];
+    const int tid = threadIdx.x;
     const int x0 = 1 + bx * kTX, y0 = 1 + by * kTY;
-    const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
+    const int tx = tid % kTX, ty = tid / kTX;
     const int x = x0 + tx, y = y0 + ty;
     const bool active = (x <= g.nx - 2) && (y <= g.ny - 2);
     const int zl = 1, zr = g.nz - 1;
 
-    // per-column coefficients
-    const int xc = active ? x : 1, yc = active ? y : 1;
-    const double cx1 = K.cx1[xc], cy1 = K.cy1[yc];
-    const double cx2a = K.cx2a[xc], cx2b = K.cx2b[xc], cy2a = K.cy2a[yc], cy2b = K.cy2b[yc];
-    // folded viscous / resistive coefficients: [ORE a, ORE b, ORE43 a, ORE43 b, ORM a, ORM b]
-    double sx[6], sy[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        sx[k] = K.s2[0][k][xc];
-        sy[k] = K.s2[1][k][yc];
+    // this thread's points of a plane: its own column, and one halo point of
+    // the rows below and above the tile (in x), then of the columns left and
+    // right, then of the corners
+    const int pc = (ty + 1) * kPX + (tx + 1);
+    const bool own_in = x < g.nx && y < g.ny;
+    int hk = 0, hkind = -1;  // halo point, 0: y halo (needs Q2), 1: x halo (Q1), 2: corner
+    if (tid < 2 * kTX) {
+        hk = (tid < kTX ? 0 : (kTY + 1) * kPX) + 1 + tid % kTX;
+        hkind = 0;
+    } else if (tid < 2 * kTX + 2 * kTY) {
+        const int r = tid - 2 * kTX;
+        hk = (1 + r % kTY) * kPX + (r < kTY ? 0 : kPX - 1);
+        hkind = 1;
+    } else if (tid < T::kHalo) {
+        const int r = tid - 2 * kTX - 2 * kTY;
+        hk = ((r & 2) ? (kTY + 1) * kPX : 0) + ((r & 1) ? kPX - 1 : 0);
+        hkind = 2;
     }
-    const double c13ore = c.C13 * c.ORE;
-    const double kxy = c13ore * cx1 * cy1;
-    const double kx13 = c13ore * cx1, ky13 = c13ore * cy1;
-    // RK coefficients: from the host, or from the device time-step record; a
-    // halted record (dt below 1e-8) turns the substage into a copy of U
-    const double gdt = a.dtp ? a.gam * a.dtp[0] : a.gdt;
-    const double zdt = a.dtp ? a.zet * a.dtp[0] : a.zdt;
+    const int hgx = x0 - 1 + hk % kPX, hgy = y0 - 1 + hk / kPX;
+    if (hgx >= g.nx || hgy >= g.ny) hkind = -1;
+    const long long ocol = (long long)y * g.sy + x, hcol = (long long)hgy * g.sy + hgx;
+    const double* U0 = a.U.p[0];
+    const long long fs = a.fs;  // distance of the fields, in elements
+
+    // raw fields of point k (column offset col) of plane z into an [nraw][plane] area
+    auto copy_point = [&](double* to, int k, long long col, int z) {
+        const double* src = U0 + (long long)z * g.sz + col;
+#pragma unroll
+        for (int f = 0; f < NRAW; f++) {
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(to + f * kPlane + k);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+            src += fs;
+        }
+    };
+    // every thread copies the points it later derives itself, so its own wait
+    // is the only one the derivation needs
+    auto copy_plane = [&](double* to, int z) {
+        if (own_in) copy_point(to, pc, ocol, z);
+        if (hkind >= 0) copy_point(to, hk, hcol, z);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // ring slots of planes z - 1, z, z + 1
+    double *Pm = ring + (size_t)((zb - 1) % 3) * kRing, *P0 = ring + (size_t)(zb % 3) * kRing,
+           *Pp = ring + (size_t)((zb + 1) % 3) * kRing;
+    double *Om = own + (size_t)((zb - 1) % 3) * kOwn, *O0 = own + (size_t)(zb % 3) * kOwn,
+           *Op = own + (size_t)((zb + 1) % 3) * kOwn;
+    // the first three planes, each into its own slot, where it is derived; then
+    // the scalars and the first two coefficient rows
+    copy_plane(Pm, zb - 1);
+    copy_plane(P0, zb);
+    copy_plane(Pp, zb + 1);
+    if (tid < SC_N) sc[tid] = K.sc[UXY ? 1 : 0][tid];
+    for (int k = tid; k < 2 * ZR_N; k += kThreads)
+        zrow[((zb + k / ZR_N) & (kZRing - 1)) * ZR_N + k % ZR_N] = zt[(size_t)(zb + k / ZR_N) * ZR_N + k % ZR_N];
+
+    __syncthreads();
+    const double one = sc[SC_ONE], nzero = sc[SC_NZ];
+    auto add = [&](double p, double q) { return fma(p, one, q); };
+    auto sub = [&](double p, double q) { return fma(-q, one, p); };
+    auto mul = [&](double p, double q) { return fma(p, q, nzero); };
+    // derivatives of raw x / y differences in units of kappa
+    const int xc = own_in ? x : 1, yc = own_in ? y : 1;  // (ghost columns form Q1, Q2 too)
+    const double gcx = UXY ? 1.0 : K.cx1[xc];
+    const double gcy = ISO ? 1.0 : UXY ? sc[SC_CY] : K.cy1[yc];
+    auto SX = [&](double d) { return UXY ? d : mul(gcx, d); };
+    auto SY = [&](double d) { return ISO ? d : mul(gcy, d); };
+    auto AX = [&](double d, double q) { return UXY ? add(d, q) : fma(gcx, d, q); };  // q + D_x
+    auto AY = [&](double d, double q) { return ISO ? add(d, q) : fma(gcy, d, q); };
+    // RK coefficients, kappa included: from the host, or from the device
+    // time-step record; a halted record (dt below 1e-8) turns the substage
+    // into a copy of U.  With lShr the temperature equation keeps true units.
     const bool halted = a.dtp && a.dtp[3] != 0.0;
-    const double ocvore = c.OCV * c.ORE;
-    // the current density carries OBETA (j' = OBETA j): the Lorentz force is
-    // B x j' and the Ohmic heating (ORM OCV / OBETA) |j'|^2
-    const double ocx1 = c.OBETA * cx1, ocy1 = c.OBETA * cy1;
-    const double ohm2 = c.OBETA != 0.0 ? c.ORM * c.OCV / c.OBETA : 0.0;
+    {
+        const double gdt = a.dtp ? a.gam * a.dtp[0] : a.gdt;
+        const double zdt = a.dtp ? a.zet * a.dtp[0] : a.zdt;
+        if (tid == 0) {
+            sc[SC_G] = gdt * sc[SC_KAPPA];
+            sc[SC_Z] = zdt * sc[SC_KAPPA];
+            sc[SC_GT] = SW::lShr ? gdt : gdt * sc[SC_KAPPA];
+            sc[SC_ZT] = SW::lShr ? zdt : zdt * sc[SC_KAPPA];
+        }
+    }
 
-    load_plane<SW, T>(a, ring, (zb - 1) % 3, zb - 1, x0, y0, false);
-    load_plane<SW, T>(a, ring, zb % 3, zb, x0, y0, false);
-    __syncthreads();  // plane zb complete: its x differences come with the next load
-    load_plane<SW, T>(a, ring, (zb + 1) % 3, zb + 1, x0, y0, true);
+    double ro0 = 1.0, ri0 = 1.0, ro1 = 1.0, ri1 = 1.0, ro2 = 1.0, ri2 = 1.0;  // rho, 1/rho of planes z, z + 1, z + 2
 
-    const int pc = (ty + 1) * kPX + (tx + 1);  // centre offset inside a plane
+    // ring quantities of a copied point (the copy may lie in P itself: all of
+    // it is read first); returns rho, 1/rho and w, and leaves RW and P + RW w
+    // of the own column in ow
+    auto derive_point = [&](const double* from, int k, double* P, double* ow, double& ro, double& ri, double& ww) {
+        double r[NRAW];
+#pragma unroll
+        for (int f = 0; f < NRAW; f++) r[f] = from[f * kPlane + k];
+        ro = r[S_RO];
+        ri = recip(ro, one);
+        const double uu = mul(r[S_RU], ri), vv = mul(r[S_RV], ri), p = mul(ro, r[S_TT]);
+        ww = mul(r[S_RW], ri);
+        P[Q_RU * kPlane + k] = r[S_RU];
+        P[Q_RV * kPlane + k] = r[S_RV];
+        P[Q_TT * kPlane + k] = r[S_TT];
+        P[Q_U * kPlane + k] = uu;
+        P[Q_V * kPlane + k] = vv;
+        P[Q_W * kPlane + k] = ww;
+        P[Q_PX * kPlane + k] = fma(r[S_RU], uu, p);
+        P[Q_PY * kPlane + k] = fma(r[S_RV], vv, p);
+        if (ow) {
+            ow[O_RW * kThreads + tid] = r[S_RW];
+            ow[O_PZ * kThreads + tid] = fma(r[S_RW], ww, p);
+        }
+        if constexpr (SW::lMag) {
+            P[Q_BX * kPlane + k] = r[S_BX];
+            P[Q_BY * kPlane + k] = r[S_BY];
+            P[Q_BZ * kPlane + k] = r[S_BZ];
+        }
+    };
+    double dux = 0.0, dvy = 0.0, wzc = 0.0;  // the own column's raw D_x u and D_y v, and D_z w, of plane z
+    double q3m = 0.0, q3c = 0.0, q3p = 0.0;  // Q3 of planes z - 1, z, z + 1
+    // the own column's D_x u and D_y v of a ring plane, and their sum Q3
+    auto own_q3 = [&](const double* P, double& du, double& dv) {
+        du = sub(P[Q_U * kPlane + pc + 1], P[Q_U * kPlane + pc - 1]);
+        dv = sub(P[Q_V * kPlane + pc + kPX], P[Q_V * kPlane + pc - kPX]);
+        return AX(du, SY(dv));
+    };
+    // Q1 = D_y v + D_z w and Q2 = D_x u + D_z w of plane z (ring plane P) at this
+    // thread's points, from w of planes z + 1 (wp, hwp) and z - 1 (wm, hwm) there;
+    // leaves dux, dvy, wzc of plane z
+    auto put_q = [&](const double* P, int z, double du, double dv, double wp, double wm, double hwp, double hwm) {
+        double* q1 = qbuf + (z & 1) * 2 * kPlane;
+        double* q2 = q1 + kPlane;
+        const double cz = zrow[(z & (kZRing - 1)) * ZR_N + ZR_CZ];
+        if (own_in) {
+            dux = du;
+            dvy = dv;
+            wzc = mul(cz, sub(wp, wm));
+            q1[pc] = AY(dv, wzc);
+            q2[pc] = AX(du, wzc);
+        }
+        if (hkind == 0) {
+            const double d = sub(P[Q_U * kPlane + hk + 1], P[Q_U * kPlane + hk - 1]);
+            const double s = UXY ? d : mul(K.cx1[hgx], d);
+            q2[hk] = fma(cz, sub(hwp, hwm), s);
+        } else if (hkind == 1) {
+            const double d = sub(P[Q_V * kPlane + hk + kPX], P[Q_V * kPlane + hk - kPX]);
+            const double s = ISO ? d : mul(UXY ? gcy : K.cy1[hgy], d);
+            q1[hk] = fma(cz, sub(hwp, hwm), s);
+        }
+    };
+
+    {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        double wm = 0.0, wp = 0.0, hwm = 0.0, hwp = 0.0, t0, t1, t2;
+        if (own_in) {
+            derive_point(Pm, pc, Pm, Om, t0, t1, wm);
+            derive_point(P0, pc, P0, O0, ro0, ri0, t2);
+            derive_point(Pp, pc, Pp, Op, ro1, ri1, wp);
+        }
+        if (hkind >= 0) {
+            derive_point(Pm, hk, Pm, nullptr, t0, t1, hwm);
+            derive_point(P0, hk, P0, nullptr, t0, t1, t2);
+            derive_point(Pp, hk, Pp, nullptr, t0, t1, hwp);
+        }
+        __syncthreads();
+        if (zb + 2 <= ze) copy_plane(stage, zb + 2);
+        double du = 0.0, dv = 0.0;
+        if (own_in) {
+            // (inactive columns inside the grid are neighbours too)
+            q3m = own_q3(Pm, du, dv);
+            q3c = own_q3(P0, du, dv);
+        }
+        put_q(P0, zb, du, dv, wp, wm, hwp, hwm);
+    }
+
     for (int z = zb; z < ze; z++) {
         __syncthreads();
+        const double* R = zrow + (z & (kZRing - 1)) * ZR_N;
+        // row z + 2 lands before the next plane's barrier
+        if (tid < ZR_N && z + 2 <= ze) zrow[((z + 2) & (kZRing - 1)) * ZR_N + tid] = zt[(size_t)(z + 2) * ZR_N + tid];
+        double dux1 = 0.0, dvy1 = 0.0;
+        if (own_in) q3p = own_q3(Pp, dux1, dvy1);
         if (active) {
-            const double* Pm = ring + (size_t)((z - 1) % 3) * NQ * kPlane;
-            const double* P0 = ring + (size_t)(z % 3) * NQ * kPlane;
-            const double* Pp = ring + (size_t)((z + 1) % 3) * NQ * kPlane;
             auto C0 = [&](int q) { return P0[q * kPlane + pc]; };
             auto XP = [&](int q) { return P0[q * kPlane + pc + 1]; };
             auto XM = [&](int q) { return P0[q * kPlane + pc - 1]; };
@@ -239,33 +334,8 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
             auto YM = [&](int q) { return P0[q * kPlane + pc - kPX]; };
             auto ZP = [&](int q) { return Pp[q * kPlane + pc]; };
             auto ZM = [&](int q) { return Pm[q * kPlane + pc]; };
-            const double* Dp = ring + (size_t)3 * NQ * kPlane;  // differences of plane z
-            auto DD = [&](int d, int off) { return Dp[d * kPlane + pc + off]; };
-            const double cz1 = K.cz1[z], cz2a = K.cz2a[z], cz2b = K.cz2b[z];
-            double sz[6];
-#pragma unroll
-            for (int k = 0; k < 6; k++) sz[k] = K.s2[2][k][z];
-            auto Dx = [&](int q) { return (XP(q) - XM(q)) * cx1; };
-            auto Dy = [&](int q) { return (YP(q) - YM(q)) * cy1; };
-            // acc + s * (D2x + D2y + D2z) q with scale pair k (0: ORE, 1: ORE*C43, 2: ORM)
-            auto lapx = [&](double acc, int q, int k) { return acc_d2<!UXY>(acc, XP(q), XM(q), C0(q), sx[2 * k], sx[2 * k + 1]); };
-            auto lapy = [&](double acc, int q, int k) { return acc_d2<!UXY>(acc, YP(q), YM(q), C0(q), sy[2 * k], sy[2 * k + 1]); };
-            auto lapz = [&](double acc, int q, int k) { return acc_d2<true>(acc, ZP(q), ZM(q), C0(q), sz[2 * k], sz[2 * k + 1]); };
-            // uniform x / y: acc + sxb (px + mx) + syb (py + my) + pz (szb + sza) + mz (szb - sza) - c S,
-            // i.e. the scaled Laplacian with its z part sza (pz - mz) + szb (pz + mz) regrouped;
-            // szpm points at the per-z pair of tables (szb + sza, szb - sza), and S = 2 (sxb + syb
-            // + szb) comes from a per-z table: one -2c product for the three axes
-            auto lap3 = [&](double acc, int q, double sxb, double syb, const double* const* szpm, double S) {
-                acc = fma(ZP(q), szpm[0][z], acc);
-                acc = fma(ZM(q), szpm[1][z], acc);
-                acc = fma(XP(q) + XM(q), sxb, acc);
-                acc = fma(YP(q) + YM(q), syb, acc);
-                return fma(-C0(q), S, acc);
-            };
-
-            const double ro = C0(Q_RO), ri = C0(Q_RI), tt = C0(Q_TT);
-            const double u = C0(Q_U), v = C0(Q_V), w = C0(Q_W);
-            const long long i = (long long)z * g.sz + (long long)y * g.sy + x;
+            const double cz = R[ZR_CZ];
+            const long long i = (long long)z * g.sz + ocol;
             // the RK register (read by substages 2 and 3) and FT of this column's
             // next plane into L2, so the next iteration's epilogue does not wait
             // on DRAM for them
@@ -273,285 +343,272 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
                 const long long inx = i + g.sz;
                 if (a.substage != 0) {
 #pragma unroll
-                    for (int f = 0; f < 8; f++)
-                        if (f < (SW::lMag ? 8 : 5)) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.Z.p[f] + inx));
+                    for (int f = 0; f < NRAW; f++)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.Z.p[0] + f * fs + inx));
                 }
                 if constexpr (SW::lShr) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.FT + inx));
             }
+            // second-derivative coefficients of the planes / columns above (p) and
+            // below (m): scale k = 0 ORE, 1 ORE*C43, 2 ORM, 3 unscaled (T)
+            auto pxs = [&](int k) { return UXY ? sc[SC_SX0 + k] : K.xt[2 * k][xc]; };
+            auto mxs = [&](int k) { return UXY ? sc[SC_SX0 + k] : K.xt[2 * k + 1][xc]; };
+            auto pys = [&](int k) { return UXY ? sc[SC_SY0 + k] : K.yt[2 * k][yc]; };
+            auto mys = [&](int k) { return UXY ? sc[SC_SY0 + k] : K.yt[2 * k + 1][yc]; };
+            // ... and their sum, the coefficient of the centre (kx, ky, kz: scale per axis)
+            auto centre = [&](int kx, int ky, int kz, int row) {
+                if constexpr (UXY) return R[row];
+                else return (pxs(kx) + mxs(kx)) + (pys(ky) + mys(ky)) + (kz < 0 ? 0.0 : R[ZR_SZ0 + 2 * kz] + R[ZR_SZ0 + 2 * kz + 1]);
+            };
+
+            const double rwp = Op[O_RW * kThreads + tid], rwm = Om[O_RW * kThreads + tid];
+            const double u = C0(Q_U), v = C0(Q_V), w = C0(Q_W), tt = C0(Q_TT);
 
             // ---- continuity (3dmhdsub.h:204-227), one-sided dRW/dz on the walls
-            double rwz = ZP(Q_RW) - ZM(Q_RW);
-            if (z == zl) rwz = 4.0 * ZP(Q_RW) - a.U.p[S_RW][i + 2 * g.sz];
-            if (z == zr - 1) rwz = a.U.p[S_RW][i - 2 * g.sz] - 4.0 * ZM(Q_RW);
-            const double fr = -fma(rwz, cz1, fma(YP(Q_RV) - YM(Q_RV), cy1, (XP(Q_RU) - XM(Q_RU)) * cx1));
+            const double rup = XP(Q_RU), rum = XM(Q_RU), rvp = YP(Q_RV), rvm = YM(Q_RV);
+            double rwz = sub(rwp, rwm);
+            if (z == zl) rwz = 4.0 * rwp - U0[S_RW * fs + i + 2 * g.sz];
+            if (z == zr - 1) rwz = U0[S_RW * fs + i - 2 * g.sz] - 4.0 * rwm;
+            const double fr = fma(-cz, rwz, AY(sub(rvm, rvp), SX(sub(rum, rup))));
 
-            // ---- pressure, gravity (3dmhdsub.h:266-272) and momentum advection
-            // (3dmhdsub.h:279-289): F_i = -D_i P - D_j(RU_i u_j), + GRAV rho in z; the
-            // diagonal terms difference P + RU_i u_i, formed once per point by load_plane
-            double fu, fv;
-            double fw = fma(ro, c.GRAV, -cz1 * (ZP(Q_PZ) - ZM(Q_PZ)));
-            if constexpr (ISO) {
-                // cx1 = cy1: each component's x and y fluxes are summed before one metric product
-                double tu = XP(Q_PX) - XM(Q_PX);
-                tu = fma(-YM(Q_RU), YM(Q_V), fma(YP(Q_RU), YP(Q_V), tu));
-                double tv = YP(Q_PY) - YM(Q_PY);
-                tv = fma(-XM(Q_RV), XM(Q_U), fma(XP(Q_RV), XP(Q_U), tv));
-                double tw = fma(XP(Q_RW), XP(Q_U), -XM(Q_RW) * XM(Q_U));
-                tw = fma(-YM(Q_RW), YM(Q_V), fma(YP(Q_RW), YP(Q_V), tw));
-                fu = -cx1 * tu;
-                fv = -cx1 * tv;
-                fw = fma(-cx1, tw, fw);
-            } else {
-                fu = -cx1 * (XP(Q_PX) - XM(Q_PX));
-                fv = -cy1 * (YP(Q_PY) - YM(Q_PY));
-                fu = fma(-cy1, fma(YP(Q_RU), YP(Q_V), -YM(Q_RU) * YM(Q_V)), fu);
-                fv = fma(-cx1, fma(XP(Q_RV), XP(Q_U), -XM(Q_RV) * XM(Q_U)), fv);
-                fw = fma(-cx1, fma(XP(Q_RW), XP(Q_U), -XM(Q_RW) * XM(Q_U)), fw);
-                fw = fma(-cy1, fma(YP(Q_RW), YP(Q_V), -YM(Q_RW) * YM(Q_V)), fw);
+            // ---- momentum: pressure and gravity (3dmhdsub.h:266-272), advection
+            // (3dmhdsub.h:279-289), viscous Laplacians (3dmhdsub.h:462-472)
+            double fu = SX(sub(XM(Q_PX), XP(Q_PX)));
+            double fv = SY(sub(YM(Q_PY), YP(Q_PY)));
+            double fw = fma(cz, sub(Om[O_PZ * kThreads + tid], Op[O_PZ * kThreads + tid]), mul(sc[SC_GRAV], ro0));
+            {
+                const double ap = UXY ? sub(pxs(0), rup) : fma(-gcx, rup, pxs(0));
+                const double am = UXY ? add(mxs(0), rum) : fma(gcx, rum, mxs(0));
+                fu = fma(pxs(1), XP(Q_U), fma(mxs(1), XM(Q_U), fu));
+                fv = fma(ap, XP(Q_V), fma(am, XM(Q_V), fv));
+                fw = fma(ap, XP(Q_W), fma(am, XM(Q_W), fw));
             }
-            fu = fma(-cz1, fma(ZP(Q_RU), ZP(Q_W), -ZM(Q_RU) * ZM(Q_W)), fu);
-            fv = fma(-cz1, fma(ZP(Q_RV), ZP(Q_W), -ZM(Q_RV) * ZM(Q_W)), fv);
+            {
+                const double ap = ISO ? sub(pys(0), rvp) : fma(-gcy, rvp, pys(0));
+                const double am = ISO ? add(mys(0), rvm) : fma(gcy, rvm, mys(0));
+                fu = fma(ap, YP(Q_U), fma(am, YM(Q_U), fu));
+                fv = fma(pys(1), YP(Q_V), fma(mys(1), YM(Q_V), fv));
+                fw = fma(ap, YP(Q_W), fma(am, YM(Q_W), fw));
+            }
+            {
+                const double ap = fma(-cz, rwp, R[ZR_SZ0]), am = fma(cz, rwm, R[ZR_SZ0 + 1]);
+                fu = fma(ap, ZP(Q_U), fma(am, ZM(Q_U), fu));
+                fv = fma(ap, ZP(Q_V), fma(am, ZM(Q_V), fv));
+                fw = fma(R[ZR_SZ0 + 2], ZP(Q_W), fma(R[ZR_SZ0 + 3], ZM(Q_W), fw));
+            }
+            fu = fma(-centre(1, 0, 0, ZR_SU), u, fu);
+            fv = fma(-centre(0, 1, 0, ZR_SV), v, fv);
+            fw = fma(-centre(0, 0, 1, ZR_SW), w, fw);
+
+            // ---- viscous cross terms (3dmhdsub.h:486-487,517-518,531-532)
+            {
+                const double* q1 = qbuf + (z & 1) * 2 * kPlane + pc;
+                const double* q2 = q1 + kPlane;
+                const double kqx = UXY ? sc[SC_KQX] : sc[SC_KQX] * gcx, kqy = UXY ? sc[SC_KQY] : sc[SC_KQY] * gcy;
+                fu = fma(kqx, sub(q1[1], q1[-1]), fu);
+                fv = fma(kqy, sub(q2[kPX], q2[-kPX]), fv);
+                fw = fma(R[ZR_KQZ], sub(q3p, q3m), fw);
+            }
 
             // ---- temperature: advection (3dmhdsub.h:293-296), conduction (:315-319)
-            const double dTz = ZP(Q_TT) - ZM(Q_TT);
             double ft;
-            double qr = 0.0;  // the temperature terms proportional to 1/rho, applied once at the end
-            // the velocities with their axis' metric factor (the T advection here
-            // and the advective induction terms below)
-            double cxu = 0.0, cyv = 0.0, czw = 0.0;
+            double qr;  // the temperature terms proportional to 1/rho, applied once at the end
+            const double czw = mul(cz, w);
+            double dTz = 0.0;
+            if constexpr (!SW::lShr || !UXY) dTz = sub(ZP(Q_TT), ZM(Q_TT));
             if constexpr (!SW::lShr) {
-                cxu = cx1 * u;
-                cyv = cy1 * v;
-                czw = cz1 * w;
-                ft = -fma(cxu, XP(Q_TT) - XM(Q_TT), fma(cyv, YP(Q_TT) - YM(Q_TT), czw * dTz));
+                const double dTx = sub(XP(Q_TT), XM(Q_TT)), dTy = sub(YP(Q_TT), YM(Q_TT));
+                ft = UXY ? mul(-u, dTx) : mul(-gcx * u, dTx);
+                ft = ISO ? fma(-v, dTy, ft) : fma(-gcy * v, dTy, ft);
+                ft = fma(-czw, dTz, ft);
             } else {
                 ft = a.FT[i];  // the reference never re-initialises FT with lShr
             }
             {
                 double lapT = 0.0;
-                if constexpr (UXY) {
-                    if (EXTRA && c.lrem && !SW::lShr) lapT = lap3(0.0, Q_TT, cx2b, cy2b, K.lapZ + 6, K.lapS[3][z]);
-                } else {
-                    lapT = acc_d2<true>(0.0, XP(Q_TT), XM(Q_TT), C0(Q_TT), cx2a, cx2b);
-                    lapT = acc_d2<true>(lapT, YP(Q_TT), YM(Q_TT), C0(Q_TT), cy2a, cy2b);
-                    lapT = acc_d2<true>(lapT, ZP(Q_TT), ZM(Q_TT), C0(Q_TT), cz2a, cz2b);
+                if ((EXTRA && c.lrem && !SW::lShr) || !UXY) {
+                    lapT = mul(UXY ? sc[SC_TX] : pxs(3), XP(Q_TT));
+                    lapT = fma(UXY ? sc[SC_TX] : mxs(3), XM(Q_TT), lapT);
+                    lapT = fma(UXY ? sc[SC_TY] : pys(3), YP(Q_TT), lapT);
+                    lapT = fma(UXY ? sc[SC_TY] : mys(3), YM(Q_TT), lapT);
+                    lapT = fma(R[ZR_TZP], ZP(Q_TT), fma(R[ZR_TZM], ZM(Q_TT), lapT));
+                    double S;
+                    if constexpr (UXY) S = R[ZR_STL];
+                    else S = (pxs(3) + mxs(3)) + (pys(3) + mys(3)) + (R[ZR_TZP] + R[ZR_TZM]);
+                    lapT = fma(-S, tt, lapT);
                 }
                 if (EXTRA && c.lrem && !SW::lShr) {
                     // lRem: conduction of T - TTM(z) plus HRAD (3dmhdsub.h:297-313),
                     // as lap T + (HRAD - d2 TTM/dz2), the latter precomputed per z
-                    ft = fma(ri * (c.OCV / c.REPR), lapT + c.lrem_g[z], ft);
+                    qr = sc[SC_TMPC] * (lapT + c.lrem_g[z]);
                 } else if constexpr (UXY) {
-                    // kapz lap T + dkapz dT/dz with kapz folded into per-z coefficients:
-                    // condT = kapz (cx2b, cy2b), the pz and mz factors kapz (cz2b + cz2a) + dkapz cz1
-                    // and kapz (cz2b - cz2a) - dkapz cz1, and kapz S
-                    double q = ZP(Q_TT) * K.condT[2][z];
-                    q = fma(ZM(Q_TT), K.condT[3][z], q);
-                    q = fma(XP(Q_TT) + XM(Q_TT), K.condT[0][z], q);
-                    q = fma(YP(Q_TT) + YM(Q_TT), K.condT[1][z], q);
-                    qr = fma(-C0(Q_TT), K.condT[4][z], q);
+                    // kapz lap T + dkapz dT/dz with kapz folded into the per-z coefficients
+                    qr = mul(R[ZR_KX], XP(Q_TT));
+                    qr = fma(R[ZR_KX], XM(Q_TT), qr);
+                    qr = fma(R[ZR_KY], YP(Q_TT), qr);
+                    qr = fma(R[ZR_KY], YM(Q_TT), qr);
+                    qr = fma(R[ZR_KZP], ZP(Q_TT), qr);
+                    qr = fma(R[ZR_KZM], ZM(Q_TT), qr);
+                    qr = fma(-R[ZR_ST], tt, qr);
                 } else {
-                    ft = fma(ri, fma(K.kapz[z], lapT, K.dkz[z] * dTz), ft);  // dkz = dkapz cz1
+                    qr = fma(R[ZR_KZP], lapT, R[ZR_KZM] * dTz);  // kapz, dkapz cz1
                 }
             }
             // internal plume heat sink (iTCon 2, 3dmhdsub.h:443-459)
             if constexpr (EXTRA) {
-                if (c.pl_mode == 3) qr = fma(-c.pl_s, c.plx[x] * c.ply[y] * c.plz[z], qr);
+                if (c.pl_mode == 3) qr = fma(-c.pl_s * sc[SC_ST], c.plx[x] * c.ply[y] * c.plz[z], qr);
             }
 
-            // ---- viscous Laplacians (3dmhdsub.h:462-472); scale pairs sx[2k], sx[2k+1]
-            if constexpr (UXY) {
-                fu = lap3(fu, Q_U, sx[3], sy[1], K.lapZ + 0, K.lapS[0][z]);
-                fv = lap3(fv, Q_V, sx[1], sy[3], K.lapZ + 0, K.lapS[1][z]);
-                fw = lap3(fw, Q_W, sx[1], sy[1], K.lapZ + 2, K.lapS[2][z]);
-            } else {
-                fu = lapz(lapy(lapx(fu, Q_U, 1), Q_U, 0), Q_U, 0);
-                fv = lapz(lapy(lapx(fv, Q_V, 0), Q_V, 1), Q_V, 0);
-                fw = lapz(lapy(lapx(fw, Q_W, 0), Q_W, 0), Q_W, 1);
+            // velocity gradients in units of kappa (heating and induction); the z
+            // gradients of u and v stay raw
+            double ux = 0, uy = 0, dUz = 0, vx = 0, vy = 0, dVz = 0, wx = 0, wy = 0;
+            if constexpr (!SW::lShr || SW::lMag) {
+                ux = SX(dux);
+                vx = SX(sub(XP(Q_V), XM(Q_V)));
+                wx = SX(sub(XP(Q_W), XM(Q_W)));
+                uy = SY(sub(YP(Q_U), YM(Q_U)));
+                vy = SY(dvy);
+                wy = SY(sub(YP(Q_W), YM(Q_W)));
+                dUz = sub(ZP(Q_U), ZM(Q_U));
+                dVz = sub(ZP(Q_V), ZM(Q_V));
             }
-
-            // ---- viscous cross terms (3dmhdsub.h:486-487,517-518,531-532)
-            {
-                double kxz, kyz;
-                if constexpr (UXY) {
-                    kxz = K.kxz[z];
-                    kyz = K.kyz[z];
-                } else {
-                    kxz = kx13 * cz1;
-                    kyz = ky13 * cz1;
-                }
-                // mixed differences as differences of the neighbours' 1-D differences
-                const double dyxv = DD(D_VX, kPX) - DD(D_VX, -kPX);
-                const double dyxu = DD(D_UX, kPX) - DD(D_UX, -kPX);
-                const double dxzw = DD(D_WZ, 1) - DD(D_WZ, -1);
-                const double dyzw = DD(D_WZ, kPX) - DD(D_WZ, -kPX);
-                const double dxzu = DD(D_UZ, 1) - DD(D_UZ, -1);
-                const double dyzv = DD(D_VZ, kPX) - DD(D_VZ, -kPX);
-                fu = fma(kxy, dyxv, fma(kxz, dxzw, fu));
-                fv = fma(kxy, dyxu, fma(kyz, dyzw, fv));
-                fw = fma(kxz, dxzu, fma(kyz, dyzv, fw));
-            }
-
-            // velocity gradients (heating and, without lShr, induction)
-            double ux = 0, uy = 0, uz = 0, vx = 0, vy = 0, vz = 0, wx = 0, wy = 0, wz = 0;
+            // ---- viscous heating and pdV work (3dmhdsub.h:477-538, not with lShr):
+            // ux^2 + vy^2 + wz^2 - ux vy - (ux + vy) wz = div^2 - 3 (ux vy + (ux + vy) wz)
             if constexpr (!SW::lShr) {
-                ux = DD(D_UX, 0) * cx1; uy = Dy(Q_U); uz = DD(D_UZ, 0) * cz1;
-                vx = DD(D_VX, 0) * cx1; vy = Dy(Q_V); vz = DD(D_VZ, 0) * cz1;
-                wx = Dx(Q_W); wy = Dy(Q_W); wz = DD(D_WZ, 0) * cz1;
-            }
-            // ---- viscous heating and pdV work (3dmhdsub.h:477-538, not with lShr)
-            if constexpr (!SW::lShr) {
-                double dg = ux * ux;
-                dg = fma(vy, vy, dg);
-                dg = fma(wz, wz, dg);
-                dg = fma(-ux, vy, dg);
-                dg = fma(-ux, wz, dg);
-                dg = fma(-vy, wz, dg);
-                const double s1 = uy + vx, s2 = uz + wx, s3 = vz + wy;
-                const double sh = fma(s1, s1, fma(s2, s2, s3 * s3));
-                const double phi = fma(c.C43, dg, sh);
-                qr = fma(ocvore, phi, qr);
-                ft = fma(-c.OCV * tt, ux + vy + wz, ft);
+                const double div = add(q3c, wzc);
+                const double s1 = add(uy, vx), s2 = fma(cz, dUz, wx), s3 = fma(cz, dVz, wy);
+                double phi = fma(s1, s1, fma(s2, s2, mul(s3, s3)));
+                phi = fma(sc[SC_C43], mul(div, div), phi);
+                phi = fma(-sc[SC_C43X3], fma(wzc, q3c, mul(ux, vy)), phi);
+                qr = fma(sc[SC_HQ], phi, qr);
+                ft = fma(mul(sc[SC_MOCV], tt), div, ft);
             }
 
             // ---- Coriolis (3dmhdsub.h:540-545)
             if constexpr (SW::lRot) {
-                fu = fma(c.OMZ, C0(Q_RV), fu);
-                fv = fma(-c.OMZ, C0(Q_RU), fv);
-                fv = fma(c.OMX, C0(Q_RW), fv);
-                fw = fma(-c.OMX, C0(Q_RV), fw);
+                const double omz = sc[SC_OMZ], omx = sc[SC_OMX], rv = C0(Q_RV);
+                fu = fma(omz, rv, fu);
+                fv = fma(-omz, C0(Q_RU), fv);
+                fv = fma(omx, O0[O_RW * kThreads + tid], fv);
+                fw = fma(-omx, rv, fw);
             }
 
             // ---- induction, Lorentz force, Ohmic heating (3dmhdsub.h:547-695)
             double w1 = 0, w2 = 0, w3 = 0;
             if constexpr (SW::lMag) {
                 const double bx = C0(Q_BX), by = C0(Q_BY), bz = C0(Q_BZ);
-                double jx, jy, jz;
-                if constexpr (SW::lShr) {
-                    // the velocity gradients feed the induction terms only: group each
-                    // component's terms by axis over raw differences and apply the axis'
-                    // metric factor once per group
-                    const double dUx = DD(D_UX, 0), dUy = YP(Q_U) - YM(Q_U), dUz = DD(D_UZ, 0);
-                    const double dVx = DD(D_VX, 0), dVy = YP(Q_V) - YM(Q_V), dVz = DD(D_VZ, 0);
-                    const double dWx = XP(Q_W) - XM(Q_W), dWy = YP(Q_W) - YM(Q_W);
-                    double dWz = DD(D_WZ, 0);
-                    // one-sided dw/dz on the walls for the induction terms (3dmhdsub.h:572-584)
-                    if (z == zl) {
-                        const long long j = i + 2 * g.sz;
-                        dWz = 4.0 * ZP(Q_W) - a.U.p[S_RW][j] / a.U.p[S_RO][j];
-                    }
-                    if (z == zr - 1) {
-                        const long long j = i - 2 * g.sz;
-                        dWz = a.U.p[S_RW][j] / a.U.p[S_RO][j] - 4.0 * ZM(Q_W);
-                    }
-                    const double dBXx = XP(Q_BX) - XM(Q_BX), dBXy = YP(Q_BX) - YM(Q_BX), dBXz = ZP(Q_BX) - ZM(Q_BX);
-                    const double dBYx = XP(Q_BY) - XM(Q_BY), dBYy = YP(Q_BY) - YM(Q_BY), dBYz = ZP(Q_BY) - ZM(Q_BY);
-                    const double dBZx = XP(Q_BZ) - XM(Q_BZ), dBZy = YP(Q_BZ) - YM(Q_BZ), dBZz = ZP(Q_BZ) - ZM(Q_BZ);
-                    czw = cz1 * w;
-                    if constexpr (ISO) {
-                        // cx1 = cy1: each component's x and y terms share one metric product
-                        w1 = fma(cx1, fma(-u, dBXx, fma(by, dUy, fma(-v, dBXy, -bx * dVy))),
-                                 cz1 * fma(bz, dUz, fma(-w, dBXz, -bx * dWz)));
-                        w2 = fma(cx1, fma(-v, dBYy, fma(bx, dVx, fma(-u, dBYx, -by * dUx))),
-                                 cz1 * fma(bz, dVz, fma(-w, dBYz, -by * dWz)));
-                        w3 = fma(cx1, fma(by, dWy, fma(-v, dBZy, fma(-bz, dVy, fma(bx, dWx, fma(-u, dBZx, -bz * dUx))))),
-                                 -czw * dBZz);
-                    } else {
-                        cxu = cx1 * u;
-                        cyv = cy1 * v;
-                        w1 = fma(-cxu, dBXx, fma(cy1, fma(by, dUy, fma(-v, dBXy, -bx * dVy)),
-                                                 cz1 * fma(bz, dUz, fma(-w, dBXz, -bx * dWz))));
-                        w2 = fma(cx1, fma(bx, dVx, fma(-u, dBYx, -by * dUx)),
-                                 fma(-cyv, dBYy, cz1 * fma(bz, dVz, fma(-w, dBYz, -by * dWz))));
-                        w3 = fma(cx1, fma(bx, dWx, fma(-u, dBZx, -bz * dUx)),
-                                 fma(cy1, fma(by, dWy, fma(-v, dBZy, -bz * dVy)), -czw * dBZz));
-                    }
-                    const double ocz1 = K.ocz1[z];  // OBETA cz1
-                    jz = fma(ocx1, dBYx, -ocy1 * dBXy);
-                    jy = fma(ocz1, dBXz, -ocx1 * dBZx);
-                    jx = fma(ocy1, dBZy, -ocz1 * dBYz);
-                } else {
-                    // one-sided dw/dz on the walls for the induction terms (3dmhdsub.h:572-584)
-                    double wzm = wz;
-                    if (z == zl) {
-                        const long long j = i + 2 * g.sz;
-                        wzm = (4.0 * ZP(Q_W) - a.U.p[S_RW][j] / a.U.p[S_RO][j]) * cz1;
-                    }
-                    if (z == zr - 1) {
-                        const long long j = i - 2 * g.sz;
-                        wzm = (a.U.p[S_RW][j] / a.U.p[S_RO][j] - 4.0 * ZM(Q_W)) * cz1;
-                    }
-                    // raw B differences: the metric factor rides in u cx1, v cy1, w cz1
-                    // for the advective terms and in OBETA c for the current density
-                    const double dBXx = XP(Q_BX) - XM(Q_BX), dBXy = YP(Q_BX) - YM(Q_BX), dBXz = ZP(Q_BX) - ZM(Q_BX);
-                    const double dBYx = XP(Q_BY) - XM(Q_BY), dBYy = YP(Q_BY) - YM(Q_BY), dBYz = ZP(Q_BY) - ZM(Q_BY);
-                    const double dBZx = XP(Q_BZ) - XM(Q_BZ), dBZy = YP(Q_BZ) - YM(Q_BZ), dBZz = ZP(Q_BZ) - ZM(Q_BZ);
-                    w1 = fma(by, uy, fma(bz, uz, -bx * (vy + wzm)));
-                    w1 = fma(-cxu, dBXx, fma(-cyv, dBXy, fma(-czw, dBXz, w1)));
-                    w2 = fma(bx, vx, fma(bz, vz, -by * (ux + wzm)));
-                    w2 = fma(-cxu, dBYx, fma(-cyv, dBYy, fma(-czw, dBYz, w2)));
-                    w3 = fma(bx, wx, fma(by, wy, -bz * (ux + vy)));
-                    w3 = fma(-cxu, dBZx, fma(-cyv, dBZy, fma(-czw, dBZz, w3)));
-                    const double ocz1 = K.ocz1[z];  // OBETA cz1
-                    jz = fma(ocx1, dBYx, -ocy1 * dBXy);
-                    jy = fma(ocz1, dBXz, -ocx1 * dBZx);
-                    jx = fma(ocy1, dBZy, -ocz1 * dBYz);
-                }
                 const bool wall = (z == zl || z == zr - 1);
-                if constexpr (UXY) {
-                    w3 = lap3(w3, Q_BZ, sx[5], sy[5], K.lapZ + 4, K.lapS[4][z]);
-                    if (wall) {
-                        // x and y parts only: acc + sxb (px + mx) + syb (py + my) - c 2 (sxb + syb)
-                        w1 = fma(-bx, K.lapS[5][z], fma(YP(Q_BX) + YM(Q_BX), sy[5], fma(XP(Q_BX) + XM(Q_BX), sx[5], w1)));
-                        w2 = fma(-by, K.lapS[5][z], fma(YP(Q_BY) + YM(Q_BY), sy[5], fma(XP(Q_BY) + XM(Q_BY), sx[5], w2)));
-                    } else {
-                        w1 = lap3(w1, Q_BX, sx[5], sy[5], K.lapZ + 4, K.lapS[4][z]);
-                        w2 = lap3(w2, Q_BY, sx[5], sy[5], K.lapZ + 4, K.lapS[4][z]);
-                    }
-                } else {
-                    w1 = lapy(lapx(w1, Q_BX, 2), Q_BX, 2);
-                    w2 = lapy(lapx(w2, Q_BY, 2), Q_BY, 2);
-                    w3 = lapz(lapy(lapx(w3, Q_BZ, 2), Q_BZ, 2), Q_BZ, 2);
-                    if (!wall) {
-                        w1 = lapz(w1, Q_BX, 2);
-                        w2 = lapz(w2, Q_BY, 2);
-                    }
-                }
-                // d2B/dz2 with the one-sided wall stencils (3dmhdsub.h:640-654,673-687)
+                // stretching; one-sided dw/dz on the walls (3dmhdsub.h:572-584)
+                double wzm = wzc;
                 if (wall) {
-                    const int s = (z == zl) ? 1 : -1;
-                    const long long j2 = i + 2 * s * g.sz, j3 = i + 3 * s * g.sz;
-                    const double d2 = c.d2zzdz2[z] * c.hz * c.ORM, d1 = c.dzzdz[z] * c.dzzdz[z] * c.h2z * c.ORM;
-                    const double X1 = (s > 0) ? ZP(Q_BX) : ZM(Q_BX), X2 = a.U.p[S_BX][j2], X3 = a.U.p[S_BX][j3];
-                    const double Y1 = (s > 0) ? ZP(Q_BY) : ZM(Q_BY), Y2 = a.U.p[S_BY][j2], Y3 = a.U.p[S_BY][j3];
-                    const double sg = (double)s;
-                    w1 += sg * (-3.0 * bx + 4.0 * X1 - X2) * d2 + (2.0 * bx - 5.0 * X1 + 4.0 * X2 - X3) * d1;
-                    w2 += sg * (-3.0 * by + 4.0 * Y1 - Y2) * d2 + (2.0 * by - 5.0 * Y1 + 4.0 * Y2 - Y3) * d1;
+                    const long long j = z == zl ? i + 2 * g.sz : i - 2 * g.sz;
+                    const double w2nd = U0[S_RW * fs + j] / U0[S_RO * fs + j];
+                    wzm = z == zl ? (4.0 * ZP(Q_W) - w2nd) * cz : (w2nd - 4.0 * ZM(Q_W)) * cz;
                 }
+                const double bzc = mul(cz, bz);
+                w1 = fma(by, uy, fma(bzc, dUz, mul(-bx, add(vy, wzm))));
+                w2 = fma(bx, vx, fma(bzc, dVz, mul(-by, add(ux, wzm))));
+                w3 = fma(bx, wx, fma(by, wy, mul(-bz, q3c)));
+                // advection and resistive Laplacians
+                {
+                    const double ap = UXY ? sub(pxs(2), u) : fma(-gcx, u, pxs(2));
+                    const double am = UXY ? add(mxs(2), u) : fma(gcx, u, mxs(2));
+                    w1 = fma(ap, XP(Q_BX), fma(am, XM(Q_BX), w1));
+                    w2 = fma(ap, XP(Q_BY), fma(am, XM(Q_BY), w2));
+                    w3 = fma(ap, XP(Q_BZ), fma(am, XM(Q_BZ), w3));
+                }
+                {
+                    const double ap = ISO ? sub(pys(2), v) : fma(-gcy, v, pys(2));
+                    const double am = ISO ? add(mys(2), v) : fma(gcy, v, mys(2));
+                    w1 = fma(ap, YP(Q_BX), fma(am, YM(Q_BX), w1));
+                    w2 = fma(ap, YP(Q_BY), fma(am, YM(Q_BY), w2));
+                    w3 = fma(ap, YP(Q_BZ), fma(am, YM(Q_BZ), w3));
+                }
+                {
+                    const double ap = sub(R[ZR_SZ0 + 4], czw), am = add(R[ZR_SZ0 + 5], czw);
+                    w3 = fma(ap, ZP(Q_BZ), fma(am, ZM(Q_BZ), w3));
+                    w3 = fma(-centre(2, 2, 2, ZR_SB), bz, w3);
+                    if (!wall) {
+                        const double S = centre(2, 2, 2, ZR_SB);
+                        w1 = fma(ap, ZP(Q_BX), fma(am, ZM(Q_BX), fma(-S, bx, w1)));
+                        w2 = fma(ap, ZP(Q_BY), fma(am, ZM(Q_BY), fma(-S, by, w2)));
+                    } else {
+                        // d2B/dz2 with the one-sided wall stencils (3dmhdsub.h:640-654,673-687)
+                        const double S = centre(2, 2, -1, ZR_SBW);
+                        const int s = (z == zl) ? 1 : -1;
+                        const long long j2 = i + 2 * s * g.sz, j3 = i + 3 * s * g.sz;
+                        const double d2 = R[ZR_WD2], d1 = R[ZR_WD1];
+                        const double X1 = (s > 0) ? ZP(Q_BX) : ZM(Q_BX), X2 = U0[S_BX * fs + j2], X3 = U0[S_BX * fs + j3];
+                        const double Y1 = (s > 0) ? ZP(Q_BY) : ZM(Q_BY), Y2 = U0[S_BY * fs + j2], Y3 = U0[S_BY * fs + j3];
+                        const double sg = (double)s;
+                        w1 = fma(-czw, ZP(Q_BX) - ZM(Q_BX), fma(-S, bx, w1));
+                        w2 = fma(-czw, ZP(Q_BY) - ZM(Q_BY), fma(-S, by, w2));
+                        w1 += sg * (-3.0 * bx + 4.0 * X1 - X2) * d2 + (2.0 * bx - 5.0 * X1 + 4.0 * X2 - X3) * d1;
+                        w2 += sg * (-3.0 * by + 4.0 * Y1 - Y2) * d2 + (2.0 * by - 5.0 * Y1 + 4.0 * Y2 - Y3) * d1;
+                    }
+                }
+                // current density j' = OBETA j (in units of kappa): the Lorentz force is
+                // B x j' and the Ohmic heating proportional to |j'|^2
+                const double ob = sc[SC_OB], ocz = R[ZR_OCZ];
+                const double obx = UXY ? ob : ob * gcx, oby = ISO ? ob : ob * gcy;
+                const double dBYx = sub(XP(Q_BY), XM(Q_BY)), dBXy = sub(YP(Q_BX), YM(Q_BX));
+                const double dBZx = sub(XP(Q_BZ), XM(Q_BZ)), dBXz = sub(ZP(Q_BX), ZM(Q_BX));
+                const double dBZy = sub(YP(Q_BZ), YM(Q_BZ)), dBYz = sub(ZP(Q_BY), ZM(Q_BY));
+                const double jz = ISO ? mul(ob, sub(dBYx, dBXy)) : fma(obx, dBYx, mul(-oby, dBXy));
+                const double jy = fma(ocz, dBXz, mul(-obx, dBZx));
+                const double jx = fma(oby, dBZy, mul(-ocz, dBYz));
                 fu = fma(bz, jy, fma(-by, jz, fu));
                 fv = fma(bx, jz, fma(-bz, jx, fv));
                 fw = fma(by, jx, fma(-bx, jy, fw));
-                qr = fma(ohm2, fma(jx, jx, fma(jy, jy, jz * jz)), qr);
+                qr = fma(sc[SC_OHM], fma(jx, jx, fma(jy, jy, mul(jz, jz))), qr);
             }
 
-            ft = fma(ri, qr, ft);
+            ft = fma(ri0, qr, ft);
 
-            // ---- RK3 substage update and the next register (3dmhdsub.h:168-192)
+            // ---- RK3 substage update and the next register (3dmhdsub.h:168-192); the
+            // register is read before anything is written, as the stores may alias
+            // the loads as far as the compiler knows
             const double fl[8] = {fu, fv, fw, ft, fr, w1, w2, w3};
-            constexpr int nf = SW::lMag ? 8 : 5;
-            constexpr int ring_of[8] = {Q_RU, Q_RV, Q_RW, Q_TT, Q_RO, Q_BX, Q_BY, Q_BZ};
+            double zf[NRAW];
 #pragma unroll
-            for (int f = 0; f < nf; f++) {
-                const double zf = (a.substage == 0) ? C0(ring_of[f]) : a.Z.p[f][i];
-                const double un = halted ? C0(ring_of[f]) : fma(gdt, fl[f], zf);
-                store_with_images(a.Uo.p[f], g, z, y, x, un);
-                if (a.substage < 2) a.Z.p[f][i] = halted ? un : fma(zdt, fl[f], un);
+            for (int f = 0; f < NRAW; f++) {
+                constexpr int ring_of[8] = {Q_RU, Q_RV, 0, Q_TT, 0, Q_BX, Q_BY, Q_BZ};
+                if (a.substage == 0 || halted) zf[f] = f == S_RW ? O0[O_RW * kThreads + tid] : f == S_RO ? ro0 : C0(ring_of[f]);
+                else zf[f] = a.Z.p[0][f * fs + i];
+            }
+#pragma unroll
+            for (int f = 0; f < NRAW; f++) {
+                const double un = halted ? zf[f] : fma(sc[f == S_TT ? SC_GT : SC_G], fl[f], zf[f]);
+                store_with_images(a.Uo.p[0] + f * fs, g, z, y, x, un);
+                if (a.substage < 2) a.Z.p[0][f * fs + i] = halted ? un : fma(sc[f == S_TT ? SC_ZT : SC_Z], fl[f], un);
             }
             if constexpr (SW::lShr) {
                 if (!halted) a.FT[i] = ft;
             }
         }
-        __syncthreads();
-        if (z + 2 <= ze) load_plane<SW, T>(a, ring, (z + 2) % 3, z + 2, x0, y0, true);
+        if (z + 1 < ze) {
+            // plane z + 2 into the slot of plane z - 1, of which every thread reads
+            // its own points only; then Q1 and Q2 of plane z + 1
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            double w2 = 0.0, hw2 = 0.0, hr, hi;
+            if (own_in) derive_point(stage, pc, Pm, Om, ro2, ri2, w2);
+            if (hkind >= 0) derive_point(stage, hk, Pm, nullptr, hr, hi, hw2);
+            if (z + 3 <= ze) copy_plane(stage, z + 3);
+            put_q(Pp, z + 1, dux1, dvy1, w2, P0[Q_W * kPlane + pc], hw2, P0[Q_W * kPlane + hk]);
+            q3m = q3c;
+            q3c = q3p;
+            ro0 = ro1;
+            ri0 = ri1;
+            ro1 = ro2;
+            ri1 = ri2;
+            double* t = Pm;
+            Pm = P0;
+            P0 = Pp;
+            Pp = t;
+            t = Om;
+            Om = O0;
+            O0 = Op;
+            Op = t;
+        }
     }
 }
 
