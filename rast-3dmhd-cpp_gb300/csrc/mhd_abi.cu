@@ -190,8 +190,6 @@ int fused_step(mhd_ctx* ctx, double dt, const double* dtp = nullptr) {
         int e = fused_substage(ctx->sw, a, ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "fused substage launch");
         if (ev) CK(cudaEventRecord(ev[1], ctx->stream));
-        e = fused_bcon_ghost(ctx->sw, ctx->g, ctx->c, a.Uo, ctx->timt, ctx->stream);
-        if (e) return cuda_fail(ctx, (cudaError_t)e, "BCON launch");
         ctx->cur = 1 - ctx->cur;
     }
     return MHD_OK;
@@ -470,6 +468,7 @@ FusedArgs fused_args(const mhd_ctx* ctx, int s, double dt, int in) {
     a.zdt = zet[s] * dt;
     a.gam = gam[s];
     a.zet = zet[s];
+    a.timt = ctx->timt;
     a.substage = s;
     return a;
 }

@@ -95,9 +95,21 @@ std::string signature(const mhd_batch* b) {
     return s;
 }
 
-// Per-instance arguments of every (parity, substage) given each instance's
-// state buffers; U0/U1 may be a scratch copy (autotuner).
-void fill_args(const mhd_batch* b, const std::vector<double*>& U0, const std::vector<double*>& U1,
+// First interior plane of z range k when nPz planes are cut into ranges of at most zmax.
+int range_count(int nPz, int zmax) { return (nPz + zmax - 1) / zmax; }
+int range_begin(int nPz, int k, int zmax) { return 1 + nPz * k / range_count(nPz, zmax); }
+
+// Whether the substage kernels apply BCON themselves (FusedArgs::walls): the
+// z ranges next to both walls then hold its planes.
+bool walls_inside(const mhd_batch* b, const Grid& g, int zmax) {
+    const int nPz = g.nz - 2, n = range_count(nPz, zmax);
+    return !b->fp32 && range_begin(nPz, 1, zmax) - 1 >= kWallPlanes &&
+           1 + nPz - range_begin(nPz, n - 1, zmax) >= kWallPlanes;
+}
+
+// Per-instance arguments of every (parity, substage) for z ranges of at most
+// zmax given each instance's state buffers; U0/U1 may be a scratch copy (autotuner).
+void fill_args(const mhd_batch* b, int zmax, const std::vector<double*>& U0, const std::vector<double*>& U1,
                const std::vector<double*>& Z, const std::vector<double*>& FT, const std::vector<int>& cur0,
                std::vector<FusedArgs>& out) {
     const int n = (int)b->ctx.size();
@@ -123,6 +135,7 @@ void fill_args(const mhd_batch* b, const std::vector<double*>& U0, const std::ve
                 a.zdt = zet[s] * b->dt[i];
                 a.timt = c->timt;
                 a.substage = s;
+                a.walls = walls_inside(b, c->g, zmax) ? 3 : 0;
             }
 }
 
@@ -176,9 +189,9 @@ void make_items(const mhd_batch* b, int tile, int zmax, std::vector<int4>& items
     for (size_t i = 0; i < b->ctx.size(); i++) {
         const Grid& g = b->ctx[i]->g;
         const int nbx = (g.nx - 2 + tx - 1) / tx, nby = (g.ny - 2 + ty - 1) / ty;
-        const int nPz = g.nz - 2, chunks = (nPz + zmax - 1) / zmax;
+        const int nPz = g.nz - 2, chunks = range_count(nPz, zmax);
         for (int ch = 0; ch < chunks; ch++) {
-            const int zb = 1 + nPz * ch / chunks, ze = 1 + nPz * (ch + 1) / chunks;
+            const int zb = range_begin(nPz, ch, zmax), ze = range_begin(nPz, ch + 1, zmax);
             for (int by = 0; by < nby; by++)
                 for (int bx = 0; bx < nbx; bx++) items.push_back(make_int4((int)i, bx, by, zb | (ze << 16)));
         }
@@ -215,10 +228,12 @@ int check_items(mhd_batch* b, int tile, const std::vector<int4>& items) {
     return MHD_OK;
 }
 
-void make_bcon_items(const mhd_batch* b, std::vector<int2>& items) {
+// Wall cells left to the separate BCON kernel, 128 per item.
+void make_bcon_items(const mhd_batch* b, int zmax, std::vector<int2>& items) {
     items.clear();
     for (size_t i = 0; i < b->ctx.size(); i++) {
         const Grid& g = b->ctx[i]->g;
+        if (walls_inside(b, g, zmax)) continue;
         const int cells = 2 * (g.nx - 2) * (g.ny - 2);
         for (int s = 0; s < cells; s += 128) items.push_back(make_int2((int)i, s));
     }
@@ -235,9 +250,9 @@ int persistent_grid(mhd_batch* b, int tile, int nitems) {
     return std::max(1, std::min(nitems, sms * per_sm));
 }
 
-// Capture the two step graphs for `tile` over the given argument array.
+// Capture the two step graphs for `tile` over the given argument array and work lists.
 int capture(mhd_batch* b, int tile, const FusedArgs* d_args, const Fused32Args* d_args32, int4* d_items, int nitems,
-            int* d_counters, cudaGraphExec_t out[2]) {
+            int2* d_bitems, int nbitems, int* d_counters, cudaGraphExec_t out[2]) {
     const int n = (int)b->ctx.size();
     const int grid = persistent_grid(b, tile, nitems);
     const BatchCtl ctl{b->d_left, b->d_err, n};
@@ -251,7 +266,7 @@ int capture(mhd_batch* b, int tile, const FusedArgs* d_args, const Fused32Args* 
                 const Fused32Args* a32 = d_args32 + ((size_t)p * 3 + s) * n;
                 rc = fused32_batch_substage(b->sw, a32, d_items, nitems, d_counters + 3 * p + s, ctl, grid,
                                             b->stream);
-                if (!rc) rc = fused32_batch_bcon(b->sw, a32, b->d_bitems, ctl, b->nbitems, b->stream);
+                if (!rc && nbitems) rc = fused32_batch_bcon(b->sw, a32, d_bitems, ctl, nbitems, b->stream);
                 continue;
             }
             const FusedArgs* args = d_args + ((size_t)p * 3 + s) * n;
@@ -259,7 +274,7 @@ int capture(mhd_batch* b, int tile, const FusedArgs* d_args, const Fused32Args* 
                                                    ctl, grid, b->stream)
                         : fused_batch_substage_gen(b->sw, tile, args, d_items, nitems, d_counters + 3 * p + s,
                                                    ctl, grid, b->stream);
-            if (!rc) rc = fused_batch_bcon(b->sw, args, b->d_bitems, ctl, b->nbitems, b->stream);
+            if (!rc && nbitems) rc = fused_batch_bcon(b->sw, args, d_bitems, ctl, nbitems, b->stream);
         }
         if (!rc) rc = batch_tick(b->d_left, n, b->stream);
         const cudaError_t ec = cudaStreamEndCapture(b->stream, &graph);
@@ -319,7 +334,7 @@ int build(mhd_batch* b) {
         BCK(cudaStreamSynchronize(b->stream));
     } else {
         std::vector<FusedArgs> args;
-        fill_args(b, U0, U1, Z, FT, cur, args);
+        fill_args(b, b->zmax, U0, U1, Z, FT, cur, args);
         BCK(cudaMemcpyAsync(b->d_args, args.data(), sizeof(FusedArgs) * args.size(), cudaMemcpyHostToDevice, b->stream));
         BCK(cudaStreamSynchronize(b->stream));
     }
@@ -334,8 +349,20 @@ int build(mhd_batch* b) {
     BCK(cudaMemcpyAsync(b->d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
     b->nitems = (int)items.size();
+    std::vector<int2> bitems;
+    make_bcon_items(b, b->zmax, bitems);
+    cudaFree(b->d_bitems);
+    b->d_bitems = nullptr;
+    b->nbitems = (int)bitems.size();
+    if (b->nbitems) {
+        BCK(cudaMalloc(&b->d_bitems, sizeof(int2) * bitems.size()));
+        BCK(cudaMemcpyAsync(b->d_bitems, bitems.data(), sizeof(int2) * bitems.size(), cudaMemcpyHostToDevice,
+                            b->stream));
+        BCK(cudaStreamSynchronize(b->stream));
+    }
     drop_graphs(b->exec);
-    int rc = capture(b, b->tile, b->d_args, b->d_args32, b->d_items, b->nitems, b->d_counters, b->exec);
+    int rc = capture(b, b->tile, b->d_args, b->d_args32, b->d_items, b->nitems, b->d_bitems, b->nbitems,
+                     b->d_counters, b->exec);
     if (rc) return rc;
     b->expect_cur = cur;
     b->phase = 0;
@@ -398,12 +425,19 @@ int autotune(mhd_batch* b, double* ms_out) {
     }
     FusedArgs* d_args = nullptr;
     Fused32Args* d_args32 = nullptr;
+    int2* d_bitems = nullptr;
+    std::vector<int2> bitems;
+    make_bcon_items(b, kZMax[kZChoices - 1], bitems);
     int* d_cnt = nullptr;
     int best = 0;
     double best_ms = 1e300;
     if (!rc && cudaMalloc(&d_args, sizeof(FusedArgs) * 6 * n) != cudaSuccess) rc = MHD_ERR_NOMEM;
     if (!rc && cudaMalloc(&d_args32, sizeof(Fused32Args) * 6 * n) != cudaSuccess) rc = MHD_ERR_NOMEM;
     if (!rc && cudaMalloc(&d_cnt, sizeof(int) * 6) != cudaSuccess) rc = MHD_ERR_NOMEM;
+    if (!rc && !bitems.empty()) {
+        if (cudaMalloc(&d_bitems, sizeof(int2) * bitems.size()) != cudaSuccess) rc = MHD_ERR_NOMEM;
+        else cudaMemcpyAsync(d_bitems, bitems.data(), sizeof(int2) * bitems.size(), cudaMemcpyHostToDevice, b->stream);
+    }
     if (!rc) {
         if (b->fp32) {
             std::vector<Fused32Args> a32;
@@ -412,7 +446,7 @@ int autotune(mhd_batch* b, double* ms_out) {
             cudaStreamSynchronize(b->stream);
         } else {
             std::vector<FusedArgs> args;
-            fill_args(b, U0, U1, Z, FT, cur, args);
+            fill_args(b, kZMax[kZChoices - 1], U0, U1, Z, FT, cur, args);  // the shortest ranges
             cudaMemcpyAsync(d_args, args.data(), sizeof(FusedArgs) * args.size(), cudaMemcpyHostToDevice, b->stream);
             cudaStreamSynchronize(b->stream);
         }
@@ -441,7 +475,7 @@ int autotune(mhd_batch* b, double* ms_out) {
             cudaMemcpyAsync(d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, b->stream);
             cudaStreamSynchronize(b->stream);
             cudaGraphExec_t ex[2] = {nullptr, nullptr};
-            rc = capture(b, t, d_args, d_args32, d_items, (int)items.size(), d_cnt, ex);
+            rc = capture(b, t, d_args, d_args32, d_items, (int)items.size(), d_bitems, (int)bitems.size(), d_cnt, ex);
             if (!rc) {
                 for (int w = 0; w < 2; w++) cudaGraphLaunch(ex[w], b->stream);
                 cudaEventRecord(e0, b->stream);
@@ -467,6 +501,7 @@ int autotune(mhd_batch* b, double* ms_out) {
     cudaStreamSynchronize(b->stream);
     cudaFree(d_args);
     cudaFree(d_args32);
+    cudaFree(d_bitems);
     cudaFree(d_cnt);
     for (void* p : owned) cudaFree(p);
     if (rc) return rc;
@@ -522,15 +557,9 @@ int mhd_batch_create(mhd_ctx* const* ctxs, const double* dts, int n, void* strea
         delete b;
         return MHD_ERR_CUDA;
     }
-    std::vector<int2> bitems;
-    make_bcon_items(b, bitems);
-    b->nbitems = (int)bitems.size();
     if (cudaMalloc(&b->d_args, sizeof(FusedArgs) * 6 * n) != cudaSuccess ||
         cudaMalloc(&b->d_args32, sizeof(Fused32Args) * 6 * n) != cudaSuccess ||
         cudaMalloc(&b->d_counters, sizeof(int) * 6) != cudaSuccess ||
-        cudaMalloc(&b->d_bitems, sizeof(int2) * bitems.size()) != cudaSuccess ||
-        cudaMemcpyAsync(b->d_bitems, bitems.data(), sizeof(int2) * bitems.size(), cudaMemcpyHostToDevice, b->stream) !=
-            cudaSuccess ||
         cudaMalloc(&b->d_left, sizeof(int) * n) != cudaSuccess ||
         cudaMalloc(&b->d_err, sizeof(int) * 4) != cudaSuccess ||
         cudaMemsetAsync(b->d_err, 0, sizeof(int) * 4, b->stream) != cudaSuccess ||

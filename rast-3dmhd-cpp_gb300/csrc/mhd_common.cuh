@@ -176,16 +176,22 @@ struct FusedArgs {
     double gam, zet;
     // interior z planes [zlo, zhi) of a single-instance launch (zhi = 0: all)
     int zlo, zhi;
+    // BCON of the wall cells by the thread that computed them (bit 0: plane 1,
+    // bit 1: plane nz - 2): only where the z range next to that wall holds the
+    // kWallPlanes planes that BCON involves
+    int walls;
 };
+constexpr int kWallPlanes = 3;
 // Device time-step record of mhd_steps_cfl: [0] DT in use (0 once halted),
 // [1] TIMT, [2] UMACH, [3] halt flag (DT < 1e-8), [4] the CFL DT computed
 // last, [5] completed steps, [6] TIMI, [7] TIMC.
 constexpr int kDtRecord = 8;
 int cfl_dt_on_device(bool mag, const Grid& g, const Consts& c, Fields8 U, double* partials, int max_blocks,
                      double* rec, cudaStream_t st);
+// One substage over planes [zlo, zhi) and BCON of the walls they touch (a.walls is set here).
 int fused_substage(unsigned sw, const FusedArgs& a, cudaStream_t st);
 // the instantiation with the optional temperature terms (fused_substage calls it)
-int fused_substage_xp(unsigned sw, const FusedArgs& a, cudaStream_t st);
+int fused_substage_xp(unsigned sw, const FusedArgs& a, int chunks, cudaStream_t st);
 // Ragged batches: persistent CTAs take (instance, tile x, tile y) items from a
 // counter that must be zero at launch.  Tile shapes: 0 = 32x4, 1 = 32x8, 2 = 16x8.
 constexpr int kBatchTiles = 3;
@@ -246,9 +252,6 @@ int fused_batch_bcon(unsigned sw, const FusedArgs* args, const int2* items, Batc
                      cudaStream_t st);
 // end of a batched step: left[i] -= 1 where positive
 int batch_tick(int* left, int n, cudaStream_t st);
-int fused_bcon_ghost(unsigned sw, const Grid& g, const Consts& c, Fields8 U, double timt, cudaStream_t st);
-// BCON of one wall (0 = bottom plane 1, 1 = top plane nz-2) or both (wall = -1)
-int fused_bcon_wall(unsigned sw, const Grid& g, const Consts& c, Fields8 U, double timt, int wall, cudaStream_t st);
 
 // FP32-storage path (fields stored in FP32, RO and TT as deviations from FP64
 // reference profiles rho0(z), T0(z)).

@@ -1,13 +1,10 @@
 // mhd_fused.cu -- launches of the fused FP64 RK3 substage for one instance
 // (the per-tile work is in mhd_fused_tile.cuh) and of the wall kernel.
 //
-// The grid is (x tiles, y tiles, z chunks): splitting every column into a few
-// z ranges turns the tail wave of a large grid into many short work units.
-// The number of chunks minimises (waves needed / waves of work) x (planes
-// loaded / planes computed) for the occupancy the device reports.
+// The grid is (x tiles, y tiles, z chunks): splitting every column into z
+// ranges spreads a small grid over the SMs and turns the tail wave of a large
+// one into many short work units (choose_chunks).
 #include "mhd_fused_tile.cuh"
-
-#include <cmath>
 
 namespace mhd {
 namespace {
@@ -52,14 +49,42 @@ __global__ void k_bcon_ghost(Grid g, Consts c, Fields8 U, double timt, int wall0
     bcon_cell<SW>(g, c, U, timt, wall0 + t / (nPx * nPy), 1 + r % nPx, 1 + r / nPx);
 }
 
-int choose_chunks(long long tiles, int slots, int nPz) {
+// First plane of z range k of n over `planes` planes (the kernel's split).
+int chunk_begin(int planes, int k, int n) { return (int)((long long)planes * k / n); }
+
+// Whether the z ranges next to the walls hold the planes of BCON.
+int fused_walls(const FusedArgs& a, int lo, int planes, int chunks) {
+    int w = 0;
+    if (lo == 1 && chunk_begin(planes, 1, chunks) >= kWallPlanes) w |= 1;
+    if (lo + planes == a.g.nz - 1 && planes - chunk_begin(planes, chunks - 1, chunks) >= kWallPlanes) w |= 2;
+    return w;
+}
+
+// Number of z ranges per column.  In units of the time the SM's one FP64 unit
+// takes for a plane of a tile (6.2 us with lMag), a launch of n CTAs with P
+// planes each lasts, measured at 32^3 .. 256x256x128 for 1 .. 64 ranges:
+//   n <= 152 (one per SM)          1.7 + 1.24 P   one CTA alone does not keep the unit busy
+//   n <= 304                       1.7 + 2.13 P
+//   n <= 456 (all resident)        1.7 + 3.05 P
+//   more                           5.0 + ceil(n / 456) (0.55 + 2.83 P)
+// with the constants for the planes around a range and its start-up; the last
+// wave counts in full because its CTAs are not spread evenly over the SMs.  A
+// range too short for BCON at the walls adds a launch (0.8).  Against at most
+// eight ranges of four planes: a step at 32x32x32 138 -> 87 us (32 ranges of
+// one plane), 97x45x61 (no field) 344 -> 272 us, 128x128x64 1146 -> 1094 us
+// (BCON inside the launch included).
+int choose_chunks(const FusedArgs& a, long long tiles, int sms, int lo, int planes) {
     int best = 1;
     double best_cost = 1e300;
-    for (int c = 1; c <= 8 && c <= nPz / 4; c++) {
-        const double units = (double)tiles * c;
-        const double waves = std::ceil(units / slots);
-        const double eff = units / (waves * slots);
-        const double cost = (1.0 + 2.0 * c / nPz) / eff;
+    const int need = (lo == 1 ? 1 : 0) | (lo + planes == a.g.nz - 1 ? 2 : 0);
+    for (int c = 1; c <= planes; c++) {
+        const long long n = tiles * c, wave = (long long)kMinBlocks * sms;
+        const double most = (planes + c - 1) / c, avg = (double)planes / c;
+        double cost = n <= sms       ? 1.7 + 1.24 * most
+                      : n <= 2 * sms ? 1.7 + 2.13 * most
+                      : n <= wave    ? 1.7 + 3.05 * most
+                                     : 5.0 + (double)((n + wave - 1) / wave) * (0.55 + 2.83 * avg);
+        if (fused_walls(a, lo, planes, c) != need) cost += 0.8;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = c;
@@ -68,63 +93,64 @@ int choose_chunks(long long tiles, int slots, int nPz) {
     return best;
 }
 
-template <class SW, bool UXY, bool ISO>
-int launch_t(const FusedArgs& a, cudaStream_t st) {
-    using T = DefaultTile;
-    const size_t smem = ring_bytes<SW, T>();
-    static int slots = 0;
-    if (!slots) {
-        cudaFuncSetAttribute(k_substage<SW, UXY, ISO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        int dev = 0, sms = 0, per_sm = 1;
+int sm_count() {
+    static const int n = [] {
+        int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_substage<SW, UXY, ISO>, T::kThreads, smem);
-        slots = sms * (per_sm > 0 ? per_sm : 1);
-    }
+        return sms > 0 ? sms : 1;
+    }();
+    return n;
+}
+
+template <class SW, bool UXY, bool ISO>
+int launch_t(const FusedArgs& a, int chunks, cudaStream_t st) {
+    using T = DefaultTile;
+    const size_t smem = ring_bytes<SW, T>();
+    static const cudaError_t set =
+        cudaFuncSetAttribute(k_substage<SW, UXY, ISO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (set != cudaSuccess) return (int)set;
     const int nbx = (a.g.nx - 2 + T::kTX - 1) / T::kTX, nby = (a.g.ny - 2 + T::kTY - 1) / T::kTY;
-    const int planes = a.zhi > 0 ? a.zhi - a.zlo : a.g.nz - 2;
-    const int chunks = choose_chunks((long long)nbx * nby, slots, planes);
     k_substage<SW, UXY, ISO><<<dim3(nbx, nby, chunks), T::kThreads, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
 
 template <class SW>
-void launch_substage(const FusedArgs& a, cudaStream_t st, int* rc) {
+void launch_substage(const FusedArgs& a, int chunks, cudaStream_t st, int* rc) {
     // the instantiation with the optional temperature terms has no isotropic variant
-    if (!kExtra && a.k.uniform_xy && a.k.isotropic_xy) *rc = launch_t<SW, true, !kExtra>(a, st);
-    else *rc = a.k.uniform_xy ? launch_t<SW, true, false>(a, st) : launch_t<SW, false, false>(a, st);
+    if (!kExtra && a.k.uniform_xy && a.k.isotropic_xy) *rc = launch_t<SW, true, !kExtra>(a, chunks, st);
+    else *rc = a.k.uniform_xy ? launch_t<SW, true, false>(a, chunks, st) : launch_t<SW, false, false>(a, chunks, st);
 }
 
 template <class SW>
-void launch_bcon_ghost(const Grid& g, const Consts& c, Fields8 U, double timt, int wall, cudaStream_t st) {
-    const int nwalls = wall < 0 ? 2 : 1, wall0 = wall < 0 ? 0 : wall;
-    const int n = nwalls * (g.nx - 2) * (g.ny - 2);
-    k_bcon_ghost<SW><<<(n + 127) / 128, 128, 0, st>>>(g, c, U, timt, wall0, nwalls);
+void launch_bcon_ghost(const FusedArgs& a, int wall0, int nwalls, cudaStream_t st) {
+    const int n = nwalls * (a.g.nx - 2) * (a.g.ny - 2);
+    k_bcon_ghost<SW><<<(n + 127) / 128, 128, 0, st>>>(a.g, a.c, a.Uo, a.timt, wall0, nwalls);
 }
 
 }  // namespace
 
 #if MHD_FUSED_XP
-int fused_substage_xp(unsigned sw, const FusedArgs& a, cudaStream_t st) {
+int fused_substage_xp(unsigned sw, const FusedArgs& a, int chunks, cudaStream_t st) {
     int rc = 0;
-    MHD_DISPATCH_SW(sw, launch_substage, a, st, &rc);
+    MHD_DISPATCH_SW(sw, launch_substage, a, chunks, st, &rc);
     return rc;
 }
 #else
-int fused_substage(unsigned sw, const FusedArgs& a, cudaStream_t st) {
-    if (a.c.pl_mode == 3 || a.c.lrem) return fused_substage_xp(sw, a, st);
+int fused_substage(unsigned sw, const FusedArgs& args, cudaStream_t st) {
+    FusedArgs a = args;
+    const int lo = a.zhi > 0 ? a.zlo : 1, planes = (a.zhi > 0 ? a.zhi : a.g.nz - 1) - lo;
+    const long long tiles = (long long)((a.g.nx - 2 + DefaultTile::kTX - 1) / DefaultTile::kTX) *
+                            ((a.g.ny - 2 + DefaultTile::kTY - 1) / DefaultTile::kTY);
+    const int chunks = choose_chunks(a, tiles, sm_count(), lo, planes);
+    a.walls = fused_walls(a, lo, planes, chunks);
     int rc = 0;
-    MHD_DISPATCH_SW(sw, launch_substage, a, st, &rc);
-    return rc;
-}
-
-int fused_bcon_ghost(unsigned sw, const Grid& g, const Consts& c, Fields8 U, double timt, cudaStream_t st) {
-    MHD_DISPATCH_SW(sw, launch_bcon_ghost, g, c, U, timt, -1, st);
-    return (int)cudaGetLastError();
-}
-
-int fused_bcon_wall(unsigned sw, const Grid& g, const Consts& c, Fields8 U, double timt, int wall, cudaStream_t st) {
-    MHD_DISPATCH_SW(sw, launch_bcon_ghost, g, c, U, timt, wall, st);
+    if (a.c.pl_mode == 3 || a.c.lrem) rc = fused_substage_xp(sw, a, chunks, st);
+    else MHD_DISPATCH_SW(sw, launch_substage, a, chunks, st, &rc);
+    if (rc) return rc;
+    // the walls that the substage left
+    const bool first = lo == 1 && !(a.walls & 1), last = lo + planes == a.g.nz - 1 && !(a.walls & 2);
+    if (first || last) MHD_DISPATCH_SW(sw, launch_bcon_ghost, a, first ? 0 : 1, (first ? 1 : 0) + (last ? 1 : 0), st);
     return (int)cudaGetLastError();
 }
 #endif

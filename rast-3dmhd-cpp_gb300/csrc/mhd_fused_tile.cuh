@@ -10,7 +10,9 @@
 // the RK update of step_block_GAM (3dmhdsub.h:181-192), forms the next
 // substage's register Z' = U' + zeta*dt*F (step_block_ZETA, 3dmhdsub.h:168-179)
 // and writes U' together with its periodic ghost images (communicate(),
-// 3dmhdmpi.h:11-143, as dual stores).
+// 3dmhdmpi.h:11-143, as dual stores).  The wall conditions BCON
+// (3dmhdsub.h:720-873) follow in the same thread where its z range reaches
+// three planes into the grid, else in a separate small kernel.
 //
 // GB300's FP64 unit takes 16 cycles of an SM for a warp's DFMA with three
 // register operands, but 19 for a DADD, a DMUL or a DFMA with a constant-bank
@@ -119,6 +121,61 @@ __device__ __forceinline__ void store_with_images(double* F, const Grid& g, int 
     if (yb >= 0) {
         F[zo + (long long)yb * g.sy + x] = v;
         if (xb >= 0) F[zo + (long long)yb * g.sy + xb] = v;
+    }
+}
+
+// BCON (3dmhdsub.h:720-873) for one wall cell of U' plus its periodic ghost images.
+template <class SW>
+__device__ __forceinline__ void bcon_cell(const Grid& g, const Consts& c, const Fields8& U, double timt, int wall, int x,
+                                          int y) {
+    const long long sz = g.sz;
+    const double RRT = 1.0, RRB = -1.0, RPP = 0.0;
+    const int z = wall == 0 ? 1 : g.nz - 2;
+    const int s = wall == 0 ? 1 : -1;
+    const long long i = (long long)z * sz + (long long)y * g.sy + x;
+    const long long i1 = i + s * sz, i2 = i + 2 * s * sz;
+    const double *RU = U.p[S_RU], *RV = U.p[S_RV], *TT = U.p[S_TT], *RO = U.p[S_RO];
+    double ru, rv, tt;
+    if constexpr (SW::lShr) {
+        ru = 0.0;
+        rv = (wall == 0 ? RRT : RRB) * cos(RPP * timt) * RO[i];
+    } else {
+        ru = RO[i] * (c.C43 * RU[i1] / RO[i1] - c.C13 * RU[i2] / RO[i2]);
+        rv = RO[i] * (c.C43 * RV[i1] / RO[i1] - c.C13 * RV[i2] / RO[i2]);
+    }
+    if (wall == 0) {
+        if (c.pl_mode == 1) {
+            // cooling spot on the top wall (3dmhdsub.h:750-766)
+            tt = 1.0f - (1.0f - c.pl_tpr) * c.plx[x] / c.pl_hh * c.ply[y] / c.pl_hh;
+        } else if (c.pl_mode == 2) {
+            const double DZ = 1.0f / (double)(g.nPz - 1) / c.dzzdz[z];
+            tt = c.C43 * TT[i1] - c.C13 * TT[i2] -
+                 c.C23 * DZ * (c.THETA - (c.THETA - c.pl_tpr) * c.plx[x] / c.pl_hh * c.ply[y] / c.pl_hh);
+        } else if (c.iTCon == 1) {
+            const double DZ = 1.0f / (float)(g.nPz - 1) / c.dzzdz[z];
+            tt = c.lrem ? c.C43 * TT[i1] - c.C13 * TT[i2] + c.DZTU : c.C43 * TT[i1] - c.C13 * TT[i2] - c.C23 * DZ * c.THETA;
+        } else if (c.lrem) {
+            tt = c.TU;
+        } else {
+            tt = 1.0;
+            if (c.iTCon == 4 && x < g.nx / 2) tt = 1.0f - c.TP;
+        }
+    } else {
+        if (c.izCon == 0) {
+            tt = c.TB;
+        } else if (c.lrem) {
+            tt = c.C43 * TT[i1] - c.C13 * TT[i2] + c.DZTB;
+        } else {
+            const double DZ = 1.0f / (float)(g.nPz - 1) / c.dzzdz[z];
+            tt = c.C43 * TT[i1] - c.C13 * TT[i2] - c.C23 * DZ * c.THETA / c.RKAPA[z];
+        }
+    }
+    store_with_images(U.p[S_RU], g, z, y, x, ru);
+    store_with_images(U.p[S_RV], g, z, y, x, rv);
+    store_with_images(U.p[S_RW], g, z, y, x, 0.0);
+    store_with_images(U.p[S_TT], g, z, y, x, tt);
+    if constexpr (SW::lMag) {
+        if (c.iBCon == 0) store_with_images(U.p[S_BZ], g, z, y, x, 0.0);
     }
 }
 
@@ -610,60 +667,11 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
             Op = t;
         }
     }
-}
-
-// BCON (3dmhdsub.h:720-873) for one wall cell of U' plus its periodic ghost images.
-template <class SW>
-__device__ __forceinline__ void bcon_cell(const Grid& g, const Consts& c, const Fields8& U, double timt, int wall, int x,
-                                          int y) {
-    const long long sz = g.sz;
-    const double RRT = 1.0, RRB = -1.0, RPP = 0.0;
-    const int z = wall == 0 ? 1 : g.nz - 2;
-    const int s = wall == 0 ? 1 : -1;
-    const long long i = (long long)z * sz + (long long)y * g.sy + x;
-    const long long i1 = i + s * sz, i2 = i + 2 * s * sz;
-    const double *RU = U.p[S_RU], *RV = U.p[S_RV], *TT = U.p[S_TT], *RO = U.p[S_RO];
-    double ru, rv, tt;
-    if constexpr (SW::lShr) {
-        ru = 0.0;
-        rv = (wall == 0 ? RRT : RRB) * cos(RPP * timt) * RO[i];
-    } else {
-        ru = RO[i] * (c.C43 * RU[i1] / RO[i1] - c.C13 * RU[i2] / RO[i2]);
-        rv = RO[i] * (c.C43 * RV[i1] / RO[i1] - c.C13 * RV[i2] / RO[i2]);
-    }
-    if (wall == 0) {
-        if (c.pl_mode == 1) {
-            // cooling spot on the top wall (3dmhdsub.h:750-766)
-            tt = 1.0f - (1.0f - c.pl_tpr) * c.plx[x] / c.pl_hh * c.ply[y] / c.pl_hh;
-        } else if (c.pl_mode == 2) {
-            const double DZ = 1.0f / (double)(g.nPz - 1) / c.dzzdz[z];
-            tt = c.C43 * TT[i1] - c.C13 * TT[i2] -
-                 c.C23 * DZ * (c.THETA - (c.THETA - c.pl_tpr) * c.plx[x] / c.pl_hh * c.ply[y] / c.pl_hh);
-        } else if (c.iTCon == 1) {
-            const double DZ = 1.0f / (float)(g.nPz - 1) / c.dzzdz[z];
-            tt = c.lrem ? c.C43 * TT[i1] - c.C13 * TT[i2] + c.DZTU : c.C43 * TT[i1] - c.C13 * TT[i2] - c.C23 * DZ * c.THETA;
-        } else if (c.lrem) {
-            tt = c.TU;
-        } else {
-            tt = 1.0;
-            if (c.iTCon == 4 && x < g.nx / 2) tt = 1.0f - c.TP;
-        }
-    } else {
-        if (c.izCon == 0) {
-            tt = c.TB;
-        } else if (c.lrem) {
-            tt = c.C43 * TT[i1] - c.C13 * TT[i2] + c.DZTB;
-        } else {
-            const double DZ = 1.0f / (float)(g.nPz - 1) / c.dzzdz[z];
-            tt = c.C43 * TT[i1] - c.C13 * TT[i2] - c.C23 * DZ * c.THETA / c.RKAPA[z];
-        }
-    }
-    store_with_images(U.p[S_RU], g, z, y, x, ru);
-    store_with_images(U.p[S_RV], g, z, y, x, rv);
-    store_with_images(U.p[S_RW], g, z, y, x, 0.0);
-    store_with_images(U.p[S_TT], g, z, y, x, tt);
-    if constexpr (SW::lMag) {
-        if (c.iBCon == 0) store_with_images(U.p[S_BZ], g, z, y, x, 0.0);
+    // BCON of a wall reads the new values of its column two planes in, all
+    // written by this thread when the z range holds them
+    if (active) {
+        if ((a.walls & 1) && zb == 1) bcon_cell<SW>(g, c, a.Uo, a.timt, 0, x, y);
+        if ((a.walls & 2) && ze == g.nz - 1) bcon_cell<SW>(g, c, a.Uo, a.timt, 1, x, y);
     }
 }
 

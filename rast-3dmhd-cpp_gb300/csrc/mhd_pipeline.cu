@@ -17,8 +17,7 @@
 // in-place ping-pong writes (S2(j) overwrites U[cur] planes that S1 of slabs
 // j-1..j+1 read, S3(j) overwrites U[1-cur] planes that S2 of slabs j-1..j+1
 // read), and the substages of one slab follow one another through it.  The
-// wall BCON of each substage follows its first / last slab on the same
-// stream.  Kernels of different substages run concurrently, so one kernel's
+// wall BCON of each substage belongs to its first / last slab.  Kernels of different substages run concurrently, so one kernel's
 // last wave overlaps the next kernel's first instead of draining the GPU; the
 // later substages have the higher stream priority, so the pipeline drains
 // early.  Every cell goes through the same arithmetic as in mhd_step, so the
@@ -161,9 +160,6 @@ int issue_step(mhd_ctx* ctx, const std::vector<int>& b, const double* in, double
         a.zhi = b[j + 1];
         int e = fused_substage(ctx->sw, a, st);
         if (e) return fail_cuda(ctx, (cudaError_t)e, "fused substage launch");
-        if (j == 0) e = fused_bcon_wall(ctx->sw, ctx->g, ctx->c, a.Uo, ctx->timt, 0, st);
-        if (!e && j == ns - 1) e = fused_bcon_wall(ctx->sw, ctx->g, ctx->c, a.Uo, ctx->timt, 1, st);
-        if (e) return fail_cuda(ctx, (cudaError_t)e, "BCON launch");
         return MHD_OK;
     };
     // issue in wavefront order (S1 of slab t, S2 of t-1, S3 of t-2), so each

@@ -6,11 +6,12 @@ x / y spacings, and on a stretched x / y grid.  One step against the oracle;
 1e-12 of each field's max-norm, the bound of every fused-path comparison:
 regrouped sums of about 200 FP64 operations per cell differ by rounding only.
 """
+import numpy as np
 import pytest
 
 from gpu_util import METRIC_NAMES, rel_err
 from mhd_gb300.case import STATE_FIELDS, initial_state, small_cases, tanh_metric
-from mhd_gb300.sim import Simulation
+from mhd_gb300.sim import Batch, Simulation
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,35 @@ def test_one_step_at_tile_edges(size, grid, sw):
     o.steps(1)
     for k in STATE_FIELDS[:case.nfields]:
         assert rel_err(got[k], o.arr[k]) <= 1e-12, (k, rel_err(got[k], o.arr[k]))
+
+
+@pytest.mark.parametrize("zmax", [1, 2, 3, 5])
+def test_batch_walls_for_short_z_ranges(zmax):
+    """Z ranges of fewer than three planes leave BCON to its own kernel, longer
+    ones apply it where the wall cells are computed: the same values either
+    way, as each cell's arithmetic does not depend on the range it lies in."""
+    base = small_cases()["mhd_fixedT"].replace(izCon=1, iTCon=1)
+    cases = [base.replace(nPx=nx, nPy=ny, nPz=nz, seed=i) for i, (nx, ny, nz) in
+             enumerate([(20, 12, 4), (17, 9, 7), (32, 8, 11)])]
+
+    def run(z):
+        sims = []
+        for c in cases:
+            s = Simulation(c)
+            s.upload_state(initial_state(c))
+            s.communicate()
+            sims.append(s)
+        b = Batch(sims)
+        b.set_tile(2)
+        b.set_zrange(z)
+        b.steps(3)
+        b.sync()
+        out = [s.download_state() for s in sims]
+        b.close()
+        for s in sims:
+            s.close()
+        return out
+
+    for got, ref in zip(run(zmax), run(64)):
+        for k in STATE_FIELDS:
+            assert np.array_equal(got[k], ref[k]), k
