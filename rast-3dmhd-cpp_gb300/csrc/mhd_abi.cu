@@ -263,25 +263,26 @@ int profiles_from_means(mhd_ctx* ctx) {
     const double* r0 = ctx->h_bg.data();
     const double* cz1 = ctx->h_cz.data();
     for (int z = 0; z < nz; z++) {
-        ctx->h_zf[3 * (size_t)nz + z] = (float)ctx->h_bg[2 * (size_t)nz + z];
-        ctx->h_zf[4 * (size_t)nz + z] = (float)ctx->h_bg[3 * (size_t)nz + z];
+        float* row = ctx->h_zf.data() + (size_t)z * ZF_N;
+        row[ZF_DZT] = (float)ctx->h_bg[2 * (size_t)nz + z];
+        row[ZF_D2T] = (float)ctx->h_bg[3 * (size_t)nz + z];
         double hz = 0.0;
         if (z > 0 && z < nz - 1) hz = r0[z] * ctx->prm.GRAV - (r0[z + 1] * bg[z + 1] - r0[z - 1] * bg[z - 1]) * cz1[z];
-        ctx->h_zf[7 * (size_t)nz + z] = (float)hz;
+        row[ZF_HZ] = (float)hz;
         // rho0 and T0 as float pairs hi + lo (hi the nearest float, lo the
         // nearest float to the exact remainder): about 48 significant bits,
         // for the FP32 kernels' compensated reconstruction of rho and p
         const float rh = (float)r0[z], th = (float)bg[z];
-        ctx->h_zf[8 * (size_t)nz + z] = rh;
-        ctx->h_zf[9 * (size_t)nz + z] = (float)(r0[z] - (double)rh);
-        ctx->h_zf[10 * (size_t)nz + z] = th;
-        ctx->h_zf[11 * (size_t)nz + z] = (float)(bg[z] - (double)th);
+        row[ZF_RH] = rh;
+        row[ZF_RL] = (float)(r0[z] - (double)rh);
+        row[ZF_TH] = th;
+        row[ZF_TL] = (float)(bg[z] - (double)th);
     }
     // on the context's stream: its kernels read the profiles (a plain cudaMemcpy
     // runs on the legacy stream, which the non-blocking context stream does not
     // wait for); the sync keeps h_bg / h_zf stable until the copies are done
     CK(cudaMemcpyAsync(ctx->d_bg, ctx->h_bg.data(), sizeof(double) * 4 * nz, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_bg + 4 * nz, ctx->h_zf.data(), sizeof(float) * kZfRows * nz, cudaMemcpyHostToDevice,
+    CK(cudaMemcpyAsync(ctx->d_bg + 4 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz, cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
@@ -360,14 +361,13 @@ int fused32_step(mhd_ctx* ctx, double dt, const double* dtp = nullptr) {
         a.FT = ctx->FT64;
         a.bgR = ctx->d_bg;
         a.bgT = ctx->d_bg + nz;
-        a.dzT0 = ctx->d_bg + 2 * nz;
-        a.d2zT0 = ctx->d_bg + 3 * nz;
         a.zf = reinterpret_cast<const float*>(ctx->d_bg + 4 * nz);
         a.gdt = gam[s] * dt;
         a.zdt = zet[s] * dt;
         a.dtp = dtp;
         a.gam = gam[s];
         a.zet = zet[s];
+        a.timt = ctx->timt;
         a.substage = s;
         if (ctx->c.lrem) {
             // horizontal means of the substage's input T (3dmhdsub.h:297-313), in FP64
@@ -390,8 +390,6 @@ int fused32_step(mhd_ctx* ctx, double dt, const double* dtp = nullptr) {
         int e = fused32_substage(ctx->sw, a, ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "FP32 substage launch");
         if (ev) CK(cudaEventRecord(ev[1], ctx->stream));
-        e = fused32_bcon_ghost(ctx->sw, ctx->g, ctx->c, a.Uo, a.Z, a.bgR, a.bgT, ctx->timt, ctx->stream);
-        if (e) return cuda_fail(ctx, (cudaError_t)e, "FP32 BCON launch");
         ctx->cur = 1 - ctx->cur;
     }
     return MHD_OK;
@@ -573,6 +571,19 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
             for (int sg = 1; sg >= -1; sg -= 2)
                 for (int i = 0; i < ns[ax]; i++) h.push_back(scales[k] * (c2b(ax, i) + sg * c2a(ax, i)));
     }
+    // the FP32 kernels' column coefficients, two floats per double
+    size_t sidef_off[2];
+    for (int ax = 0; ax < 2; ax++) {
+        std::vector<float> t((size_t)8 * ns[ax]);
+        for (int k = 0; k < 4; k++)
+            for (int i = 0; i < ns[ax]; i++) {
+                t[(size_t)(2 * k) * ns[ax] + i] = (float)(scales[k] * c2b(ax, i));
+                t[(size_t)(2 * k + 1) * ns[ax] + i] = (float)(scales[k] * c2a(ax, i));
+            }
+        sidef_off[ax] = h.size();
+        h.resize(h.size() + (size_t)4 * ns[ax]);
+        memcpy(h.data() + sidef_off[ax], t.data(), sizeof(float) * t.size());
+    }
     bool uxy = true;
     for (int i = 0; i < nx; i++) uxy = uxy && p.d2xxdx2[i] == 0.0;
     for (int i = 0; i < ny; i++) uxy = uxy && p.d2yydy2[i] == 0.0;
@@ -670,6 +681,9 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
             *c1s[ax] = b0 + base_off[ax];
             *c2as[ax] = b0 + base_off[ax] + ns[ax];
             *c2bs[ax] = b0 + base_off[ax] + 2 * ns[ax];
+            for (int k = 0; k < 8; k++)
+                (ax ? ctx->coef.yf : ctx->coef.xf)[k] =
+                    reinterpret_cast<const float*>(b0 + sidef_off[ax]) + (size_t)k * ns[ax];
             for (int k = 0; k < 8; k++) (ax ? ctx->coef.yt : ctx->coef.xt)[k] = b0 + side_off[ax] + (size_t)k * ns[ax];
         }
         for (int u = 0; u < 2; u++) {
@@ -699,17 +713,25 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     int arc = MHD_OK;
     if (ctx->fp32) {
         arc = alloc_f32(ctx, &ctx->U32[0]);
-        // 4 x nz double profiles, then the [kZfRows][nz] float coefficient table
-        const size_t bg_bytes = sizeof(double) * 4 * nz + sizeof(float) * kZfRows * nz;
+        // 4 x nz double profiles, then the [nz][ZF_N] float coefficient table
+        const size_t bg_bytes = sizeof(double) * 4 * nz + sizeof(float) * ZF_N * nz;
         if (!arc && cudaMalloc(&ctx->d_bg, bg_bytes) != cudaSuccess) arc = MHD_ERR_NOMEM;
         if (!arc && cudaMemsetAsync(ctx->d_bg, 0, bg_bytes, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
-        ctx->h_zf.assign(kZfRows * (size_t)nz, 0.0f);
+        ctx->h_zf.assign(ZF_N * (size_t)nz, 0.0f);
         for (int z = 0; z < nz; z++) {
-            for (int r = 0; r < 3; r++) ctx->h_zf[(size_t)r * nz + z] = (float)ctx->h_cz[(size_t)r * nz + z];
-            ctx->h_zf[5 * (size_t)nz + z] = (float)p.RKAPA[z];
-            ctx->h_zf[6 * (size_t)nz + z] = (float)p.DKAPA[z];
+            float* row = ctx->h_zf.data() + (size_t)z * ZF_N;
+            const double cz = c1(2, z), za = c2a(2, z), zb = c2b(2, z);
+            row[ZF_CZ] = (float)cz;
+            row[ZF_NCZ] = (float)-cz;
+            for (int k = 0; k < 4; k++) {
+                row[ZF_SZ0 + 2 * k] = (float)(scales[k] * zb);
+                row[ZF_SZ0 + 2 * k + 1] = (float)(scales[k] * za);
+            }
+            row[ZF_KQZ] = (float)(c13ore * cz);
+            row[ZF_KAP] = (float)(tmpc * p.RKAPA[z]);
+            row[ZF_DKAP] = (float)(tmpc * p.DKAPA[z]);
         }
-        if (!arc && cudaMemcpyAsync(ctx->d_bg + 4 * nz, ctx->h_zf.data(), sizeof(float) * kZfRows * nz,
+        if (!arc && cudaMemcpyAsync(ctx->d_bg + 4 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz,
                                     cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
     } else {
         arc = alloc_block(ctx, &ctx->U[0], 8);

@@ -101,9 +101,9 @@ int range_begin(int nPz, int k, int zmax) { return 1 + nPz * k / range_count(nPz
 
 // Whether the substage kernels apply BCON themselves (FusedArgs::walls): the
 // z ranges next to both walls then hold its planes.
-bool walls_inside(const mhd_batch* b, const Grid& g, int zmax) {
+bool walls_inside(const Grid& g, int zmax) {
     const int nPz = g.nz - 2, n = range_count(nPz, zmax);
-    return !b->fp32 && range_begin(nPz, 1, zmax) - 1 >= kWallPlanes &&
+    return range_begin(nPz, 1, zmax) - 1 >= kWallPlanes &&
            1 + nPz - range_begin(nPz, n - 1, zmax) >= kWallPlanes;
 }
 
@@ -135,13 +135,13 @@ void fill_args(const mhd_batch* b, int zmax, const std::vector<double*>& U0, con
                 a.zdt = zet[s] * b->dt[i];
                 a.timt = c->timt;
                 a.substage = s;
-                a.walls = walls_inside(b, c->g, zmax) ? 3 : 0;
+                a.walls = walls_inside(c->g, zmax) ? 3 : 0;
             }
 }
 
 // The same for FP32-storage instances; U0/U1 (FP32 state), Z and FT (FP64)
 // may be a scratch copy (autotuner).
-void fill_args32(const mhd_batch* b, const std::vector<float*>& U0, const std::vector<float*>& U1,
+void fill_args32(const mhd_batch* b, int zmax, const std::vector<float*>& U0, const std::vector<float*>& U1,
                  const std::vector<double*>& Z, const std::vector<double*>& FT, const std::vector<int>& cur0,
                  std::vector<Fused32Args>& out) {
     const int n = (int)b->ctx.size();
@@ -165,13 +165,12 @@ void fill_args32(const mhd_batch* b, const std::vector<float*>& U0, const std::v
                 a.FT = FT[i];
                 a.bgR = c->d_bg;
                 a.bgT = c->d_bg + nz;
-                a.dzT0 = c->d_bg + 2 * nz;
-                a.d2zT0 = c->d_bg + 3 * nz;
                 a.zf = reinterpret_cast<const float*>(c->d_bg + 4 * nz);
                 a.gdt = gam[s] * b->dt[i];
                 a.zdt = zet[s] * b->dt[i];
                 a.timt = c->timt;
                 a.substage = s;
+                a.walls = walls_inside(c->g, zmax) ? 3 : 0;
             }
 }
 
@@ -233,7 +232,7 @@ void make_bcon_items(const mhd_batch* b, int zmax, std::vector<int2>& items) {
     items.clear();
     for (size_t i = 0; i < b->ctx.size(); i++) {
         const Grid& g = b->ctx[i]->g;
-        if (walls_inside(b, g, zmax)) continue;
+        if (walls_inside(g, zmax)) continue;
         const int cells = 2 * (g.nx - 2) * (g.ny - 2);
         for (int s = 0; s < cells; s += 128) items.push_back(make_int2((int)i, s));
     }
@@ -328,7 +327,7 @@ int build(mhd_batch* b) {
             FT32[i] = b->ctx[i]->FT64;
         }
         std::vector<Fused32Args> a32;
-        fill_args32(b, V0, V1, Z32, FT32, cur, a32);
+        fill_args32(b, b->zmax, V0, V1, Z32, FT32, cur, a32);
         BCK(cudaMemcpyAsync(b->d_args32, a32.data(), sizeof(Fused32Args) * a32.size(), cudaMemcpyHostToDevice,
                             b->stream));
         BCK(cudaStreamSynchronize(b->stream));
@@ -441,7 +440,7 @@ int autotune(mhd_batch* b, double* ms_out) {
     if (!rc) {
         if (b->fp32) {
             std::vector<Fused32Args> a32;
-            fill_args32(b, V0, V1, Z, FT, cur, a32);
+            fill_args32(b, kZMax[kZChoices - 1], V0, V1, Z, FT, cur, a32);  // the shortest ranges
             cudaMemcpyAsync(d_args32, a32.data(), sizeof(Fused32Args) * a32.size(), cudaMemcpyHostToDevice, b->stream);
             cudaStreamSynchronize(b->stream);
         } else {

@@ -122,6 +122,8 @@ struct Coefs {
     const double *cy1, *cy2a, *cy2b;
     // per column (any grid): c2b + c2a and c2b - c2a, scaled by ORE, ORE*C43, ORM and unscaled
     const double *xt[8], *yt[8];
+    // for the FP32 kernels: c2b and c2a as floats, scaled alike
+    const float *xf[8], *yf[8];
     // uniform x and y grids: d2xxdx2 and d2yydy2 vanish and the x / y
     // coefficients are the same in every interior column
     int uniform_xy;
@@ -258,8 +260,17 @@ int batch_tick(int* left, int n, cudaStream_t st);
 struct Fields8f {
     float* p[8];
 };
-// rows of the FP32 kernels' per-z float table (Fused32Args::zf)
-constexpr int kZfRows = 12;
+// the FP32 kernels' per-z coefficients, one row of ZF_N floats per z
+enum ZFloat {
+    ZF_CZ = 0, ZF_NCZ,   // +-cz1
+    ZF_SZ0,              // b and a of the z second derivative, scaled by ORE, ORE*C43, ORM and unscaled: 8 entries
+    ZF_KQZ = ZF_SZ0 + 8, // C13*ORE*cz1
+    ZF_KAP, ZF_DKAP,     // OCV/REPR * (RKAPA, DKAPA)
+    // from the profiles: their hydrostatic residual rho0 GRAV - D_z(rho0 T0), T0's first and second z
+    // derivatives, and rho0, T0 as float pairs hi, lo
+    ZF_HZ, ZF_DZT, ZF_D2T, ZF_RH, ZF_RL, ZF_TH, ZF_TL,
+    ZF_N
+};
 struct Fused32Args {
     Grid g;
     Consts c;
@@ -269,20 +280,17 @@ struct Fused32Args {
     Fields8 Z;     // FP64 RK register (full values)
     double* FT;    // FP64 persistent temperature right-hand side (lShr only)
     const double *bgR, *bgT;     // reference profiles rho0(z), T0(z)
-    const double *dzT0, *d2zT0;  // their premultiplied first and second z derivatives
-    const float* zf;             // [kZfRows][nz] float cz1, cz2a, cz2b, dzT0, d2zT0, RKAPA, DKAPA, the
-                                 // profiles' hydrostatic residual rho0 GRAV - D_z(rho0 T0), and
-                                 // rho0, T0 as float pairs (rows 8, 9 and 10, 11: hi, lo)
+    const float* zf;             // [nz][ZF_N]
     double gdt, zdt;
     double timt;
     int substage;
     // device time-step record of mhd_steps_cfl (as FusedArgs)
     const double* dtp;
     double gam, zet;
+    int walls;  // as FusedArgs
 };
+// One substage and BCON (a.walls is set here).
 int fused32_substage(unsigned sw, const Fused32Args& a, cudaStream_t st);
-int fused32_bcon_ghost(unsigned sw, const Grid& g, const Consts& c, Fields8f U, Fields8 Z, const double* bgR,
-                       const double* bgT, double timt, cudaStream_t st);
 int communicate32(int nf, const Grid& g, Fields8f U, cudaStream_t st);
 // lRem profiles (as lrem_profiles) of an FP32-storage temperature: the plane
 // means T0(z) + mean(dT) summed in FP64

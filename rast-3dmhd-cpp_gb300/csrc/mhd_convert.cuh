@@ -59,4 +59,23 @@ __device__ __forceinline__ float narrow_f64(double d) {
     return __uint_as_float(sign | (q + up));
 }
 
+// f 2^-896 exactly, for every finite f: the float's fields taken as a double's
+// (zero and subnormal floats come out as zero and subnormal doubles).
+__device__ __forceinline__ double widen_scaled(float f) {
+    const unsigned b = __float_as_uint(f);
+    return __hiloint2double((int)((unsigned)((int)b >> 3) & 0x8fffffffu), (int)(b << 29));
+}
+// (float)d, rounded to nearest even, in fewer instructions, where
+// narrow_ordinary: the result is a normal float, whichever way it rounds
+__device__ __forceinline__ bool narrow_ordinary(double d) {
+    // exponent field 897 .. 1149: 2^-126 up to below 2^127
+    return (((unsigned)__double2hiint(d) & 0x7fffffffu) - 0x38100000u) < 0x0fd00000u;
+}
+__device__ __forceinline__ float narrow_fast(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const unsigned q = __funnelshift_l(lo, hi, 3);  // exponent (9 bits), the 23 bits kept
+    const unsigned up = ((lo << 3) | (q & 1u)) > 0x80000000u ? 1u : 0u;  // above half, or half and odd
+    return __uint_as_float(((q + 0x40000000u + up) & 0x7fffffffu) | (hi & 0x80000000u));
+}
+
 }  // namespace mhd

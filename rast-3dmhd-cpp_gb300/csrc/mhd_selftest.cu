@@ -45,6 +45,9 @@ __global__ void k_selftest(long long n, unsigned long long seed, unsigned long l
         if (!same_f32(mhd::narrow_f64(d), __double2float_rn(d))) nb++;
         const float f = __double2float_rn(d);
         if (!same_f64(mhd::widen_f32(f), (double)f)) nb++;
+        // the substage's forms: f 2^-896 for finite f, and the rounding of ordinary values
+        if (isfinite(f) && !same_f64(mhd::widen_scaled(f) * 0x1p896, (double)f)) nb++;
+        if (mhd::narrow_ordinary(d) && !same_f32(mhd::narrow_fast(d), f)) nb++;
     }
     if (nb) atomicAdd(bad, nb);
 }
