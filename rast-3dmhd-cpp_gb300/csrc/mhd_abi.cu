@@ -12,6 +12,7 @@
 // Buffers that a call sequence never needs are allocated on first use.
 #include "mhd_context.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -310,14 +311,34 @@ int upload32(mhd_ctx* ctx, int field, const double* host) {
     return MHD_OK;
 }
 
-int download32(mhd_ctx* ctx, int field, double* host) {
-    std::vector<float> tmp(ctx->ncell);
+// Fields [field, field + nf) of the state to the host, widened on the device in
+// pieces of kStage elements.  Widening on the host (a copy of each field into a
+// fresh buffer, then one thread's loop) took 67 ms for the eight fields of
+// 256x256x128; the copy alone takes 3.
+constexpr size_t kStage = 2u << 20;  // 16 MB: a piece's copy takes far longer than its kernel
+
+int download32(mhd_ctx* ctx, int field, int nf, double* host) {
+    if (!ctx->d_stage) {
+        const size_t len = std::min(kStage, ctx->ncell * (size_t)ctx->nf);
+        if (cudaMalloc(&ctx->d_stage, len * sizeof(double)) == cudaSuccess) {
+            ctx->stage_len = len;
+            ctx->bytes += len * sizeof(double);
+        } else {
+            ctx->d_stage = nullptr;
+            cudaGetLastError();
+        }
+    }
+    // without memory for it: the reduction scratch, which this stream's work does not hold
+    double* const buf = ctx->d_stage ? ctx->d_stage : ctx->red;
+    const long long len = ctx->d_stage ? (long long)ctx->stage_len : 8LL * ctx->red_blocks;
+    const long long first = (long long)field * (long long)ctx->ncell, total = (long long)nf * (long long)ctx->ncell;
+    for (long long at = 0; at < total; at += len) {
+        const int n = (int)std::min(len, total - at);
+        const int e = widen32(ctx->g, ctx->U32[ctx->cur], ctx->d_bg, ctx->d_bg + ctx->g.nz, first + at, n, buf, ctx->stream);
+        if (e) return cuda_fail(ctx, (cudaError_t)e, "widening launch");
+        CK(cudaMemcpyAsync(host + at, buf, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaMemcpy(tmp.data(), ctx->U32[ctx->cur] + (size_t)field * ctx->ncell, ctx->ncell * sizeof(float),
-                  cudaMemcpyDeviceToHost));
-    const double* bg = profile_host(ctx, field);
-    const size_t plane = (size_t)ctx->g.sz;
-    for (size_t i = 0; i < ctx->ncell; i++) host[i] = (double)tmp[i] + (bg ? bg[i / plane] : 0.0);
     return MHD_OK;
 }
 
@@ -786,6 +807,7 @@ int mhd_destroy(mhd_ctx* ctx) {
     cudaFree(ctx->U32[0]);
     cudaFree(ctx->U32[1]);
     cudaFree(ctx->FT64);
+    cudaFree(ctx->d_stage);
     cudaFree(ctx->d_bg);
     cudaFree(ctx->d_plume);
     cudaFree(ctx->d_lrem);
@@ -857,7 +879,7 @@ int mhd_upload(mhd_ctx* ctx, int field, const double* host) {
 
 int mhd_download(mhd_ctx* ctx, int field, double* host) {
     if (!ctx || !host) return MHD_ERR_INVALID;
-    if (ctx->fp32 && field >= 0 && field < 8) return download32(ctx, field, host);
+    if (ctx->fp32 && field >= 0 && field < 8) return download32(ctx, field, 1, host);
     int rc;
     double* d = field_ptr(ctx, field, false, &rc);
     if (!d) return rc;
@@ -882,13 +904,7 @@ int mhd_upload_state(mhd_ctx* ctx, const double* host) {
 
 int mhd_download_state(mhd_ctx* ctx, double* host) {
     if (!ctx || !host) return MHD_ERR_INVALID;
-    if (ctx->fp32) {
-        for (int f = 0; f < ctx->nf; f++) {
-            int rc = download32(ctx, f, host + (size_t)f * ctx->ncell);
-            if (rc) return rc;
-        }
-        return MHD_OK;
-    }
+    if (ctx->fp32) return download32(ctx, 0, ctx->nf, host);
     CK(cudaMemcpyAsync(host, ctx->U[ctx->cur], field_bytes(ctx) * ctx->nf, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return MHD_OK;

@@ -292,6 +292,9 @@ struct Fused32Args {
 // One substage and BCON (a.walls is set here).
 int fused32_substage(unsigned sw, const Fused32Args& a, cudaStream_t st);
 int communicate32(int nf, const Grid& g, Fields8f U, cudaStream_t st);
+// elements [first, first + n) of an FP32-storage state (fields one after another) as FP64 values in out
+int widen32(const Grid& g, const float* U, const double* bgR, const double* bgT, long long first, int n, double* out,
+            cudaStream_t st);
 // lRem profiles (as lrem_profiles) of an FP32-storage temperature: the plane
 // means T0(z) + mean(dT) summed in FP64
 int lrem_profiles32(const Grid& g, const Consts& c, const float* dT, const double* bgT, double* buf, cudaStream_t st);

@@ -244,6 +244,30 @@ __global__ void k_lrem_ttm32(Grid g, const float* dT, const double* bgT, double*
 
 }  // namespace
 
+namespace {
+
+// Elements [first, first + n) of the state, fields one after another, as FP64:
+// the stored deviation plus its profile (rho0, T0; zero for the other fields).
+__global__ void k_widen32(Grid g, const float* U, const double* bgR, const double* bgT, long long first, int n,
+                          double* out) {
+    const long long ncell = g.sz * g.nz;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const long long e = first + k;
+        const int f = (int)(e / ncell);
+        const int z = (int)((e - f * ncell) / g.sz);
+        out[k] = widen_f32(U[e]) + (f == S_RO ? bgR[z] : f == S_TT ? bgT[z] : 0.0);
+    }
+}
+
+}  // namespace
+
+int widen32(const Grid& g, const float* U, const double* bgR, const double* bgT, long long first, int n, double* out,
+            cudaStream_t st) {
+    const int b = (n + 255) / 256;
+    k_widen32<<<b < 152 * 16 ? b : 152 * 16, 256, 0, st>>>(g, U, bgR, bgT, first, n, out);
+    return (int)cudaGetLastError();
+}
+
 int lrem_profiles32(const Grid& g, const Consts& c, const float* dT, const double* bgT, double* buf, cudaStream_t st) {
     k_lrem_ttm32<<<g.nz, 256, 0, st>>>(g, dT, bgT, buf);
     const int e = (int)cudaGetLastError();

@@ -66,3 +66,25 @@ def test_non_finite_cells_stay_non_finite(value):
         zz, yy, xx = np.nonzero(bad)
         assert bad.any()
         assert np.abs(zz - 8).max() <= 3 and np.abs(yy - 10).max() <= 3 and np.abs(xx - 12).max() <= 3, k
+
+
+def test_download_widens_every_piece():
+    """The state comes back as its stored floats plus the profiles, in pieces:
+    a grid of more elements than one piece holds, whole and field by field, is
+    what was uploaded to the rounding of one float of the deviation (and
+    exactly the same values either way)."""
+    case = small_cases()["mhd_fixedT"].replace(nPx=100, nPy=90, nPz=60)
+    st = initial_state(case)
+    sim = Simulation(case, precision="fp32")
+    sim.upload_state(st)
+    got = sim.download_state()
+    whole = np.empty((8,) + case.shape)
+    import ctypes as C
+    assert sim.L.mhd_download_state(sim.ctx, whole.ctypes.data_as(C.POINTER(C.c_double))) == 0
+    sim.close()
+    assert whole.size > 2 << 20  # the piece length, in elements
+    for i, k in enumerate(STATE_FIELDS):
+        assert np.array_equal(whole[i], got[k]), k
+        mean = st[k][:, 1:-1, 1:-1].mean(axis=(1, 2))[:, None, None] if k in ("RO", "TT") else 0.0
+        bound = 2.0 ** -24 * np.abs(st[k] - mean) + 2.0 ** -50 * np.abs(st[k]) + 2.0 ** -149
+        assert (np.abs(got[k] - st[k]) <= bound).all(), k
