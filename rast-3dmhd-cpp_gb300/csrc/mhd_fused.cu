@@ -6,6 +6,8 @@
 // one into many short work units (choose_chunks).
 #include "mhd_fused_tile.cuh"
 
+#include <algorithm>
+
 namespace mhd {
 namespace {
 
@@ -77,8 +79,14 @@ int choose_chunks(const FusedArgs& a, long long tiles, int sms, int lo, int plan
     int best = 1;
     double best_cost = 1e300;
     const int need = (lo == 1 ? 1 : 0) | (lo + planes == a.g.nz - 1 ? 2 : 0);
+    const long long wave = (long long)kMinBlocks * sms;
+    // A slab of a host-to-host step runs beside the slabs of other substages,
+    // which fill its last wave: where a plane has a wave of tiles, about two waves
+    // of long ranges (256x256x128: 8.65 ms per step with 2 ranges, 9.24 with the 8
+    // of the model below; 512x512x256: 57.3 ms with 1)
+    if (planes < a.g.nz - 2 && tiles >= wave) return (int)std::max(1LL, std::min<long long>(planes, (2 * wave + tiles / 2) / tiles));
     for (int c = 1; c <= planes; c++) {
-        const long long n = tiles * c, wave = (long long)kMinBlocks * sms;
+        const long long n = tiles * c;
         const double most = (planes + c - 1) / c, avg = (double)planes / c;
         double cost = n <= sms       ? 1.7 + 1.24 * most
                       : n <= 2 * sms ? 1.7 + 2.13 * most
