@@ -721,6 +721,8 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     c.RM = p.RM; c.ORM = ctx->k.ORM; c.OBETA = ctx->k.OBETA; c.TB = p.TB; c.TP = p.TP; c.SFF = p.SFF;
     c.DDXmin = HUGE_VAL;
     for (int x = 1; x <= nx - 2; x++) c.DDXmin = (p.DDX[x] < c.DDXmin) ? p.DDX[x] : c.DDXmin;
+    c.DDXsame = 1;
+    for (int x = 1; x <= nx - 2; x++) c.DDXsame = c.DDXsame && p.DDX[x] == c.DDXmin;
     c.izCon = p.izCon; c.iTCon = p.iTCon; c.iBCon = p.iBCon;
     c.lrem = (p.switches & MHD_SW_LREM) ? 1 : 0;
     c.TU = p.TU; c.DZTU = p.DZTU; c.DZTB = p.DZTB;

@@ -526,19 +526,24 @@ struct CflFields64 {
     __device__ double f(int k, long long i) const { return U.p[k][i]; }
     __device__ double ro(long long i, int) const { return U.p[S_RO][i]; }
     __device__ double tt(long long i, int) const { return U.p[S_TT][i]; }
-    // the estimate's float input of field k (truncated to 23 bits) and whether it is nonzero
-    __device__ float fe(int k, long long i) const { return trunc_to_f32(U.p[k][i]); }
-    __device__ bool nz(int k, long long i) const { return nonzero_bits(U.p[k][i]); }
+    // a cell's fields as they are stored, loaded apart from their use so that
+    // several cells' loads are in flight at once
+    using Val = double;
+    __device__ Val load(int k, long long i) const { return U.p[k][i]; }
+    static constexpr int kGroup = 2;  // cells of a lane loaded together
+    // the estimate's float input of a field (truncated to 23 bits) and whether it is nonzero
+    static __device__ float fe(Val v) { return trunc_to_f32(v); }
+    static __device__ bool nz(Val v) { return nonzero_bits(v); }
     // Estimate inputs ro, tt of a filtered row (truncated to 23 bits: relative
     // error below 2^-23) and m, the value whose row minimum gives the row's
     // smallest ro: here ro itself.
     struct Row {};
     using Min = double;
     __device__ Row row(int) const { return {}; }
-    __device__ void est_in(const Row&, long long i, float& ro, float& tt, bool& ok, double& m) const {
-        m = U.p[S_RO][i];
-        ro = trunc_to_f32(m);
-        tt = trunc_to_f32(U.p[S_TT][i]);
+    __device__ void est_in(const Row&, Val vro, Val vtt, float& ro, float& tt, bool& ok, double& m) const {
+        m = vro;
+        ro = trunc_to_f32(vro);
+        tt = trunc_to_f32(vtt);
         ok = true;
     }
     __device__ double ro_min(double m, int) const { return m; }
@@ -550,8 +555,11 @@ struct CflFields32 {
     __device__ double ro(long long i, int z) const { return bgR[z] + widen_f32(U.p[S_RO][i]); }
     __device__ double tt(long long i, int z) const { return bgT[z] + widen_f32(U.p[S_TT][i]); }
     // stored floats are their own estimate input (exact; subnormals kept)
-    __device__ float fe(int k, long long i) const { return U.p[k][i]; }
-    __device__ bool nz(int k, long long i) const { return (__float_as_uint(U.p[k][i]) & 0x7fffffffu) != 0u; }
+    using Val = float;
+    __device__ Val load(int k, long long i) const { return U.p[k][i]; }
+    static constexpr int kGroup = 4;
+    static __device__ float fe(Val v) { return v; }
+    static __device__ bool nz(Val v) { return (__float_as_uint(v) & 0x7fffffffu) != 0u; }
     // Estimate inputs of a filtered row, with no FP64 operation per cell:
     // ro = float(rho0) + dro and tt = float(T0) + dT in FP32.  Against the FP64
     // values their relative error is at most 5 * 2^-24 (the profile's rounding,
@@ -564,10 +572,10 @@ struct CflFields32 {
     };
     using Min = float;
     __device__ Row row(int z) const { return {narrow_f64(bgR[z]), narrow_f64(bgT[z])}; }
-    __device__ void est_in(const Row& r, long long i, float& ro, float& tt, bool& ok, float& m) const {
-        m = U.p[S_RO][i];
+    __device__ void est_in(const Row& r, Val vro, Val vtt, float& ro, float& tt, bool& ok, float& m) const {
+        m = vro;
         ro = __fadd_rn(r.Rf, m);
-        tt = __fadd_rn(r.Tf, U.p[S_TT][i]);
+        tt = __fadd_rn(r.Tf, vtt);
         ok = fabsf(r.Rf) <= 4.0f * fabsf(ro) && fabsf(r.Tf) <= 4.0f * fabsf(tt);
     }
     __device__ double ro_min(float m, int z) const { return bgR[z] + widen_f32(m); }
@@ -613,65 +621,129 @@ __device__ __forceinline__ void cfl_cell(const Grid& g, const Consts& c, const F
     }
 }
 
+// The five running extrema (um a maximum, the others minima) of the n values
+// v[k * ld + j], j < n, in out[0..4]: warp k reduces quantity k, as an FP64
+// comparison takes a warp 64 cycles and all lanes of the SM's one unit together.
+// min/max are exact, so no order changes the result.
+__device__ __forceinline__ void reduce_cfl(const double* v, int n, long long ld, double* out) {
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (k < 5) {
+        double r = k == 0 ? 0.0 : 1e99;
+        for (int j = lane; j < n; j += 32) {
+            const double a = v[k * ld + j];
+            if (k == 0) r = (r < a) ? a : r;
+            else r = (a < r) ? a : r;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double a = __shfl_xor_sync(0xffffffffu, r, o);
+            if (k == 0) r = (r < a) ? a : r;
+            else r = (a < r) ? a : r;
+        }
+        if (lane == 0) out[k] = r;
+    }
+}
+
+// What the last block does with the extrema of all blocks
+struct CflEnd {
+    double* out;   // out[0..4] = the extrema, or
+    double* rec;   // the device time-step record (when set)
+    double sff;
+    int mag;
+};
+
+// DT = SFF * min(candidates) as step() forms it (3dmhdsub.h:44,102-104), kept
+// in the device record; a DT below 1e-8 (or not a number) halts the run as
+// 3dmhd.cpp:292 does: the flag stays set, the record's DT becomes 0 and the
+// substage kernels then leave the state unchanged.  TIMC and TIMT advance as
+// 3dmhdsub.h:150-152 does once per completed step.
+__device__ void cfl_record(const double v[5], const CflEnd& e) {
+    double* rec = e.rec;
+    auto mn = [](double a, double b) { return (b < a) ? b : a; };
+    const double dt = e.mag ? e.sff * mn(mn(v[1], v[2]), mn(v[3], v[4])) : e.sff * mn(mn(v[1], v[2]), v[3]);
+    const bool stop = rec[3] != 0.0 || !(dt >= 1.0e-8f);
+    if (rec[3] == 0.0) {
+        rec[4] = dt;
+        rec[2] = sqrt(v[0]);
+    }
+    rec[3] = stop ? 1.0 : 0.0;
+    rec[0] = stop ? 0.0 : dt;
+    if (!stop) {
+        rec[7] += dt;
+        rec[1] = rec[6] + rec[7];
+        rec[5] += 1.0;
+    }
+}
+
 // Block reduction of the running extrema into partials [5][gridDim.x]
-// (blockDim.x = 256); min/max are exact, so no order changes the result.
-__device__ void write_cfl_partials(double um, double w0, double w1, double w2, double w3, double* part) {
+// (blockDim.x = 256); the block that finishes last (`done` counts them, 0 at
+// launch) reduces the partials of all.
+__device__ void finish_cfl(double um, double w0, double w1, double w2, double w3, double* part, unsigned* done,
+                           const CflEnd& end) {
     __shared__ double s[5][256];
+    __shared__ double r[5];
+    __shared__ bool last;
     s[0][threadIdx.x] = um;
     s[1][threadIdx.x] = w0;
     s[2][threadIdx.x] = w1;
     s[3][threadIdx.x] = w2;
     s[4][threadIdx.x] = w3;
     __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) {
-            const double a = s[0][threadIdx.x + h];
-            s[0][threadIdx.x] = (s[0][threadIdx.x] < a) ? a : s[0][threadIdx.x];
-            for (int k = 1; k < 5; k++) {
-                const double b = s[k][threadIdx.x + h];
-                s[k][threadIdx.x] = (b < s[k][threadIdx.x]) ? b : s[k][threadIdx.x];
-            }
-        }
-        __syncthreads();
+    reduce_cfl(&s[0][0], 256, 256, r);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 5; k++) part[(long long)k * gridDim.x + blockIdx.x] = r[k];
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 5; k++) part[(long long)k * gridDim.x + blockIdx.x] = s[k][0];
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    reduce_cfl(part, gridDim.x, gridDim.x, r);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (end.rec) cfl_record(r, end);
+    else
+        for (int k = 0; k < 5; k++) end.out[k] = r[k];
 }
 
-
-// FP32 estimates of cell i's fast-mode candidate a0 and of mc from the float
-// inputs ro, tt (certified by `okin`), and whether its momenta are not all
-// exactly zero.  When `ok`, both are certified to 1.4e-6: to first order in
+// FP32 estimates of a cell's fast-mode candidate a0 and of mc from its fields v
+// and the float inputs ro, tt (certified by `okin`), and whether its momenta are
+// not all exactly zero.  When `ok`, both are certified to 1.4e-6: to first order in
 // u = 2^-24, mc is within 18u (inputs truncated to 23 bits) or 23u (FP32
 // storage: exact momenta and fields, ro and tt within 5u), a0 within 16u.
 template <bool MAG, class FA>
-__device__ __forceinline__ void cfl_estimate(const FA& U, long long i, float ro, float tt, bool okin, float ddf,
+__device__ __forceinline__ void cfl_estimate(const typename FA::Val v[8], float ro, float tt, bool okin, float ddf,
                                              float gam_f, float obeta_f, float& a0, float& mc, bool& ok, bool& nz) {
-    const float ru = U.fe(S_RU, i), rv = U.fe(S_RV, i), rw = U.fe(S_RW, i);
-    nz = U.nz(S_RU, i) | U.nz(S_RV, i) | U.nz(S_RW, i);  // no short circuit: the loads stay unconditional
+    const float ru = FA::fe(v[S_RU]), rv = FA::fe(v[S_RV]), rw = FA::fe(v[S_RW]);
+    nz = FA::nz(v[S_RU]) | FA::nz(v[S_RV]) | FA::nz(v[S_RW]);
     const float ir = __frcp_rn(ro);
     const float sq = __fadd_rn(__fadd_rn(__fmul_rn(ru, ru), __fmul_rn(rv, rv)), __fmul_rn(rw, rw));
     const float uuk = __fmul_rn(__fmul_rn(sq, ir), ir);
     float G = __fmul_rn(gam_f, tt);
     if constexpr (MAG) {
-        const float bx = U.fe(S_BX, i), by = U.fe(S_BY, i), bz = U.fe(S_BZ, i);
+        const float bx = FA::fe(v[S_BX]), by = FA::fe(v[S_BY]), bz = FA::fe(v[S_BZ]);
         const float b2 = __fadd_rn(__fadd_rn(__fmul_rn(bx, bx), __fmul_rn(by, by)), __fmul_rn(bz, bz));
         G = __fadd_rn(G, __fmul_rn(__fmul_rn(obeta_f, b2), ir));
     }
     const float uuf = __fadd_rn(__fadd_rn(uuk, G), __fmul_rn(2.0f, __fsqrt_rn(__fmul_rn(uuk, G))));
     mc = __fdiv_rn(uuk, tt);
     a0 = __fmul_rn(ddf, rsqrtf(uuf));
-    ok = okin && (ro >= 0x1p-20f && ro <= 0x1p20f) && (tt >= 0x1p-20f && tt <= 0x1p20f) && isfinite(uuf) &&
-         isfinite(mc) && isfinite(a0);
+    ok = okin && (ro >= 0x1p-20f && ro <= 0x1p20f) && (tt >= 0x1p-20f && tt <= 0x1p20f) && fabsf(uuf) < INFINITY &&
+         fabsf(mc) < INFINITY && fabsf(a0) < INFINITY;
 }
 
-// Whether a row takes the filtered path (see k_cfl_rows), with its DD.
-__device__ __forceinline__ bool cfl_fast_row(const Grid& g, const Consts& c, int y, int z, double& DDyz) {
-    DDyz = cfl_dd_yz(c, y, z);
-    const double P1 = 0.5f * DDyz * DDyz * c.REPR * c.CV;  // prefix of cfl_a1
-    const double P2 = 0.375f * DDyz * DDyz * c.RE;         // prefix of cfl_a2
+// Whether a row takes the filtered path (see k_cfl_rows), with its DD: where
+// DDX never undercuts min(DDZ[z], DDY[y]), and where DDX is the same in every
+// column (a uniform x grid), DD is the same in every cell of the row.
+__device__ __forceinline__ bool cfl_fast_row(const Grid& g, const Consts& c, int y, int z, double& DD) {
+    DD = cfl_dd_yz(c, y, z);
+    const bool dx = g.nx > 3 && c.DDXmin < DD;
+    if (dx && !c.DDXsame) return false;
+    if (dx) DD = c.DDXmin;
+    const double P1 = 0.5f * DD * DD * c.REPR * c.CV;  // prefix of cfl_a1
+    const double P2 = 0.375f * DD * DD * c.RE;         // prefix of cfl_a2
     const bool consts_ok = (c.GAMMA >= 0x1p-10 && c.GAMMA <= 0x1p10) && (c.OBETA >= 0.0 && c.OBETA <= 0x1p30);
-    return consts_ok && (g.nx <= 3 || !(c.DDXmin < DDyz)) && P1 > 0.0 && P2 > 0.0 && cfl_kappa(c, z) > 0.0;
+    return consts_ok && P1 > 0.0 && P2 > 0.0 && cfl_kappa(c, z) > 0.0;
 }
 
 // A row's place, DD and filter test.  A warp works through its rows in batches
@@ -699,6 +771,18 @@ __device__ __forceinline__ CflRowInfo cfl_row_from(const CflRowInfo& a, int t) {
             __shfl_sync(0xffffffffu, (int)a.fast, t) != 0};
 }
 
+// The fields of cells x, x + 32, ... of a row (columns beyond nPx: the last one's).
+template <bool MAG, class FA>
+__device__ __forceinline__ void cfl_load(const FA& U, long long row, int x, int nPx,
+                                         typename FA::Val (&v)[FA::kGroup][8]) {
+#pragma unroll
+    for (int k = 0; k < FA::kGroup; k++) {
+        const long long i = row + min(x + 32 * k, nPx);
+#pragma unroll
+        for (int f = 0; f < (MAG ? 8 : 5); f++) v[k][f] = U.load(f, i);
+    }
+}
+
 // Seeds of the filter: the smallest a0 estimate and the largest mc estimate
 // (momenta not all zero) over every kCflSeedStride-th row, as ordered integer
 // keys (0 = nothing seen).  Any estimate that some certified cell attains is a
@@ -723,16 +807,20 @@ __global__ void k_cfl_seed(Grid g, Consts c, FA U, unsigned* seed) {
             const float ddf = narrow_f64(ri.DD);
             const long long row = (long long)z * g.sz + (long long)y * g.sy;
             const typename FA::Row rk = U.row(z);
-#pragma unroll 4
-            for (int x = 1 + lane; x <= nPx; x += 32) {  // unrolled: the cells' loads overlap
-                float ro, tt, a0, mc;
-                bool okin, ok, nz;
-                typename FA::Min m;
-                U.est_in(rk, row + x, ro, tt, okin, m);
-                cfl_estimate<MAG>(U, row + x, ro, tt, okin, ddf, gam_f, obeta_f, a0, mc, ok, nz);
-                if (ok) {
-                    best_a = fminf(best_a, a0);
-                    if (nz) best_m = fmaxf(best_m, mc);
+            for (int x0 = 1; x0 <= nPx; x0 += 32 * FA::kGroup) {
+                typename FA::Val v[FA::kGroup][8];
+                cfl_load<MAG>(U, row, x0 + lane, nPx, v);
+#pragma unroll
+                for (int k = 0; k < FA::kGroup; k++) {
+                    float ro, tt, a0, mc;
+                    bool okin, ok, nz;
+                    typename FA::Min m;
+                    U.est_in(rk, v[k][S_RO], v[k][S_TT], ro, tt, okin, m);
+                    cfl_estimate<MAG, FA>(v[k], ro, tt, okin, ddf, gam_f, obeta_f, a0, mc, ok, nz);
+                    if (ok && x0 + lane + 32 * k <= nPx) {
+                        best_a = fminf(best_a, a0);
+                        if (nz) best_m = fmaxf(best_m, mc);
+                    }
                 }
             }
         }
@@ -755,8 +843,8 @@ constexpr float kCflTau = 1.52587890625e-05f;    // 2^-16: filter margin, > 2x t
 
 // The CFL reduction, one warp per (y, z) row of cells.
 //
-// On a row whose DD is the same in every cell (DDX never below
-// min(DDZ[z], DDY[y]); always so on uniform x/y grids) the candidates need no
+// On a row whose DD is the same in every cell (cfl_fast_row; always so on
+// uniform x grids) the candidates need no
 // per-cell FP64 arithmetic except where they can decide the result:
 //   * a1, a2 are products/quotients of ro with positive row constants and a3
 //     depends on DD alone; rounding is monotone, so their row minima are the
@@ -772,14 +860,16 @@ constexpr float kCflTau = 1.52587890625e-05f;    // 2^-16: filter margin, > 2x t
 //     is never better than the best over all of the warp's cells, and the cell
 //     holding the warp's exact extremum has an estimate within the error
 //     bound of that, so it is always evaluated exactly.
+// Bound by the latency of its loads: a lane loads 4 cells (FP64: 2) before it
+// uses the first (256x256x128 with lMag, whole reduction: FP32 storage 162 -> 106
+// us, FP64 222 -> 157).
 // The exact maximum of mc and minimum of a0 are therefore among the cells
 // evaluated exactly, and the result equals the cell-by-cell reduction bit for
 // bit; after the first passes only new near-extremes are evaluated.  Rows with varying DD, and launches whose constants break the
 // monotonicity (non-positive factors), evaluate every cell exactly.
 template <bool MAG, class FA>
-__global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c, FA U, const unsigned* seed,
-                                                             double* part) {
-    __shared__ int list[kCflWarps][32 * kCflK];
+__global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c, FA U, unsigned* seed, double* part,
+                                                             CflEnd end) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nPx = g.nx - 2, nPy = g.ny - 2, nPz = g.nz - 2;
     const long long nrows = (long long)nPy * nPz;
@@ -803,36 +893,37 @@ __global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c
                 for (int x = 1 + lane; x <= nPx; x += 32) cfl_cell<MAG>(g, c, U, x, y, z, OGAMMA, um, w0, w1, w2, w3);
                 continue;
             }
-            const double DDyz = ri.DD;
+            const double DD = ri.DD;
             typename FA::Min mro = INFINITY;  // no cell yet
-            const float ddf = narrow_f64(DDyz);
+            const float ddf = narrow_f64(DD);
             const typename FA::Row rk = U.row(z);
             for (int x0 = 1; x0 <= nPx; x0 += 32 * kCflK) {
                 float aA[kCflK], mA[kCflK];
                 unsigned okm = 0u, nzm = 0u, valid = 0u;
                 float Ma = INFINITY, Mm = -INFINITY;
 #pragma unroll
-                for (int k = 0; k < kCflK; k++) {
-                    const int x = x0 + k * 32 + lane;
-                    aA[k] = 0.0f;
-                    mA[k] = 0.0f;
-                    if (x > nPx) continue;
-                    valid |= 1u << k;
-                    const long long i = row + x;
-                    float ro, tt, a0, mc;
-                    bool okin, ok, nz;
-                    typename FA::Min m;
-                    U.est_in(rk, i, ro, tt, okin, m);
-                    mro = (m < mro) ? m : mro;
-                    cfl_estimate<MAG>(U, i, ro, tt, okin, ddf, gam_f, obeta_f, a0, mc, ok, nz);
-                    aA[k] = a0;
-                    mA[k] = mc;
-                    if (ok) {
-                        okm |= 1u << k;
-                        Ma = fminf(Ma, a0);
-                        if (nz) Mm = fmaxf(Mm, mc);
+                for (int k0 = 0; k0 < kCflK; k0 += FA::kGroup) {
+                    if (k0 > 0 && x0 + 32 * k0 > nPx) break;  // (uniform)
+                    typename FA::Val v[FA::kGroup][8];
+                    cfl_load<MAG>(U, row, x0 + 32 * k0 + lane, nPx, v);
+#pragma unroll
+                    for (int j = 0; j < FA::kGroup; j++) {
+                        const int k = k0 + j;
+                        float ro, tt;
+                        bool okin, ok, nz;
+                        typename FA::Min m;
+                        U.est_in(rk, v[j][S_RO], v[j][S_TT], ro, tt, okin, m);
+                        cfl_estimate<MAG, FA>(v[j], ro, tt, okin, ddf, gam_f, obeta_f, aA[k], mA[k], ok, nz);
+                        if (x0 + k * 32 + lane > nPx) continue;
+                        valid |= 1u << k;
+                        mro = (m < mro) ? m : mro;
+                        if (ok) {
+                            okm |= 1u << k;
+                            Ma = fminf(Ma, aA[k]);
+                            if (nz) Mm = fmaxf(Mm, mA[k]);
+                        }
+                        if (nz) nzm |= 1u << k;
                     }
-                    if (nz) nzm |= 1u << k;
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
@@ -849,28 +940,19 @@ __global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c
                     const bool v = (valid >> k) & 1u, ok = (okm >> k) & 1u, nz = (nzm >> k) & 1u;
                     if (v && (!ok || aA[k] <= ta || (nz && mA[k] >= tm))) cm |= 1u << k;
                 }
-                // Most passes have no such cell; the compaction (ballots and
-                // population counts, the latter on GB300's FP64 pipe) runs
-                // only when one has.
-                if (__any_sync(0xffffffffu, cm != 0u)) {
-                    int n = 0;
-#pragma unroll
-                    for (int k = 0; k < kCflK; k++) {
-                        const bool cand = (cm >> k) & 1u;
-                        const unsigned bal = __ballot_sync(0xffffffffu, cand);
-                        if (cand) list[wid][n + __popc(bal & ((1u << lane) - 1u))] = x0 + k * 32 + lane;
-                        n += __popc(bal);
-                    }
-                    __syncwarp();
-                    for (int j = lane; j < n; j += 32) {
-                        const int x = list[wid][j];
+                // Most passes have no such cell; else each lane evaluates its own,
+                // one per turn (the FP64 unit takes a warp's instruction as long
+                // for one lane as for 32)
+                while (__any_sync(0xffffffffu, cm != 0u)) {
+                    if (cm) {
+                        const int x = x0 + (__ffs((int)cm) - 1) * 32 + lane;
+                        cm &= cm - 1u;
                         double mc, UU;
                         cfl_speeds<MAG>(c, U, row + x, z, OGAMMA, mc, UU);
                         um = (um < mc) ? mc : um;
-                        const double a0 = DDyz / sqrt(UU);
+                        const double a0 = DD / sqrt(UU);
                         w0 = (a0 < w0) ? a0 : w0;
                     }
-                    __syncwarp();
                 }
             }
 #pragma unroll
@@ -892,15 +974,14 @@ __global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c
             }
         }
     }
-    write_cfl_partials(um, w0, w1, w2, w3, part);
+    finish_cfl(um, w0, w1, w2, w3, part, seed + 2, end);
 }
 
 // Launch the row reduction with one wave of resident blocks (each warp then
-// sees many rows, so its running estimates filter most cells); returns the
-// number of partial blocks.
+// sees many rows, so its running estimates filter most cells).
 template <class FA>
 int launch_cfl_rows_t(bool mag, const Grid& g, const Consts& c, FA U, double* partials, int max_blocks,
-                    cudaStream_t st) {
+                      const CflEnd& end, cudaStream_t st) {
     static int wave[2] = {0, 0};  // per accessor type
     int& w = wave[mag ? 1 : 0];
     if (!w) {
@@ -916,89 +997,22 @@ int launch_cfl_rows_t(bool mag, const Grid& g, const Consts& c, FA U, double* pa
     if (nb < 1) nb = 1;
     if (nb > w) nb = w;
     if (nb > max_blocks) nb = max_blocks;
-    // two seed words after the largest partial block (5 x max_blocks doubles)
+    // two seed words and the count of finished blocks after the largest partial block (5 x max_blocks doubles)
     unsigned* seed = reinterpret_cast<unsigned*>(partials + 5 * (size_t)max_blocks);
-    cudaMemsetAsync(seed, 0, 2 * sizeof(unsigned), st);
+    cudaMemsetAsync(seed, 0, 3 * sizeof(unsigned), st);
     const long long srows = (nrows + kCflSeedStride - 1) / kCflSeedStride;
     long long sb = (srows * 32 + 255) / 256;
     if (sb > w) sb = w;
     if (sb < 1) sb = 1;
     if (mag) {
         k_cfl_seed<true, FA><<<(int)sb, 256, 0, st>>>(g, c, U, seed);
-        k_cfl_rows<true, FA><<<(int)nb, kCflWarps * 32, 0, st>>>(g, c, U, seed, partials);
+        k_cfl_rows<true, FA><<<(int)nb, kCflWarps * 32, 0, st>>>(g, c, U, seed, partials, end);
     } else {
         k_cfl_seed<false, FA><<<(int)sb, 256, 0, st>>>(g, c, U, seed);
-        k_cfl_rows<false, FA><<<(int)nb, kCflWarps * 32, 0, st>>>(g, c, U, seed, partials);
+        k_cfl_rows<false, FA><<<(int)nb, kCflWarps * 32, 0, st>>>(g, c, U, seed, partials, end);
     }
-    return (int)nb;
+    return (int)cudaGetLastError();
 }
-int launch_cfl_rows(bool mag, const Grid& g, const Consts& c, Fields8 U, double* partials, int max_blocks,
-                    cudaStream_t st) {
-    return launch_cfl_rows_t(mag, g, c, CflFields64{U}, partials, max_blocks, st);
-}
-
-// Reduce the per-block CFL partials (5 x nb) into v[0] = max UMACH^2
-// candidate, v[1..4] = min time-step candidates, in thread 0.
-__device__ void reduce_cfl_partials(const double* part, int nb, double v[5]) {
-    __shared__ double s[5][256];
-    v[0] = 0.0;
-    for (int k = 1; k < 5; k++) v[k] = 1e99;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        const double a = part[b];
-        v[0] = (v[0] < a) ? a : v[0];
-        for (int k = 1; k < 5; k++) {
-            const double q = part[(long long)k * nb + b];
-            v[k] = (q < v[k]) ? q : v[k];
-        }
-    }
-    for (int k = 0; k < 5; k++) s[k][threadIdx.x] = v[k];
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) {
-            const double a = s[0][threadIdx.x + h];
-            s[0][threadIdx.x] = (s[0][threadIdx.x] < a) ? a : s[0][threadIdx.x];
-            for (int k = 1; k < 5; k++) {
-                const double b = s[k][threadIdx.x + h];
-                s[k][threadIdx.x] = (b < s[k][threadIdx.x]) ? b : s[k][threadIdx.x];
-            }
-        }
-        __syncthreads();
-    }
-    for (int k = 0; k < 5; k++) v[k] = s[k][0];
-}
-
-__global__ void k_cfl_finish(const double* part, int nb, double* out) {
-    double v[5];
-    reduce_cfl_partials(part, nb, v);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 5; k++) out[k] = v[k];
-}
-
-// DT = SFF * min(candidates) as step() forms it (3dmhdsub.h:44,102-104), kept
-// in the device record; a DT below 1e-8 (or not a number) halts the run as
-// 3dmhd.cpp:292 does: the flag stays set, the record's DT becomes 0 and the
-// substage kernels then leave the state unchanged.  TIMC and TIMT advance as
-// 3dmhdsub.h:150-152 does once per completed step.
-__global__ void k_cfl_record(const double* part, int nb, double sff, int mag, double* rec) {
-    double v[5];
-    reduce_cfl_partials(part, nb, v);
-    if (threadIdx.x != 0) return;
-    auto mn = [](double a, double b) { return (b < a) ? b : a; };
-    const double dt = mag ? sff * mn(mn(v[1], v[2]), mn(v[3], v[4])) : sff * mn(mn(v[1], v[2]), v[3]);
-    const bool stop = rec[3] != 0.0 || !(dt >= 1.0e-8f);
-    if (rec[3] == 0.0) {
-        rec[4] = dt;
-        rec[2] = sqrt(v[0]);
-    }
-    rec[3] = stop ? 1.0 : 0.0;
-    rec[0] = stop ? 0.0 : dt;
-    if (!stop) {
-        rec[7] += dt;
-        rec[1] = rec[6] + rec[7];
-        rec[5] += 1.0;
-    }
-}
-
 int grid_for(long long n, int threads, int cap) {
     long long b = (n + threads - 1) / threads;
     if (b < 1) b = 1;
@@ -1107,16 +1121,12 @@ __global__ void k_lrem_hrad(Grid g, Consts c, const double* TTM, double* hrad, d
 
 int parity_cfl(bool mag, const Grid& g, const Consts& c, Fields8 U, double* partials, int max_blocks, double* out5,
                cudaStream_t st) {
-    const int nb = launch_cfl_rows(mag, g, c, U, partials, max_blocks, st);
-    k_cfl_finish<<<1, 256, 0, st>>>(partials, nb, out5);
-    return (int)cudaGetLastError();
+    return launch_cfl_rows_t(mag, g, c, CflFields64{U}, partials, max_blocks, CflEnd{out5, nullptr, c.SFF, mag ? 1 : 0}, st);
 }
 
 int cfl_dt_on_device(bool mag, const Grid& g, const Consts& c, Fields8 U, double* partials, int max_blocks,
                      double* rec, cudaStream_t st) {
-    const int nb = launch_cfl_rows(mag, g, c, U, partials, max_blocks, st);
-    k_cfl_record<<<1, 256, 0, st>>>(partials, nb, c.SFF, mag ? 1 : 0, rec);
-    return (int)cudaGetLastError();
+    return launch_cfl_rows_t(mag, g, c, CflFields64{U}, partials, max_blocks, CflEnd{nullptr, rec, c.SFF, mag ? 1 : 0}, st);
 }
 
 int lrem_hrad_from_means(const Grid& g, const Consts& c, double* buf, cudaStream_t st) {
@@ -1134,16 +1144,14 @@ int lrem_profiles(const Grid& g, const Consts& c, const double* TT, double* buf,
 
 int cfl32_rows(bool mag, const Grid& g, const Consts& c, Fields8f U, const double* bgR, const double* bgT,
                double* partials, int max_blocks, double* out5, cudaStream_t st) {
-    const int nb = launch_cfl_rows_t(mag, g, c, CflFields32{U, bgR, bgT}, partials, max_blocks, st);
-    k_cfl_finish<<<1, 256, 0, st>>>(partials, nb, out5);
-    return (int)cudaGetLastError();
+    return launch_cfl_rows_t(mag, g, c, CflFields32{U, bgR, bgT}, partials, max_blocks,
+                             CflEnd{out5, nullptr, c.SFF, mag ? 1 : 0}, st);
 }
 
 int cfl32_dt_on_device(bool mag, const Grid& g, const Consts& c, Fields8f U, const double* bgR, const double* bgT,
                        double* partials, int max_blocks, double* rec, cudaStream_t st) {
-    const int nb = launch_cfl_rows_t(mag, g, c, CflFields32{U, bgR, bgT}, partials, max_blocks, st);
-    k_cfl_record<<<1, 256, 0, st>>>(partials, nb, c.SFF, mag ? 1 : 0, rec);
-    return (int)cudaGetLastError();
+    return launch_cfl_rows_t(mag, g, c, CflFields32{U, bgR, bgT}, partials, max_blocks,
+                             CflEnd{nullptr, rec, c.SFF, mag ? 1 : 0}, st);
 }
 
 }  // namespace mhd
