@@ -39,7 +39,7 @@ struct mhd_batch {
     int tile = -1;  // chosen tile shape
     int zmax = 64;  // longest z range of a work item (planes)
     bool uxy = true;   // every instance has uniform x/y grids
-    bool fp32 = false; // FP32-storage instances (one tile shape, 32x8)
+    bool fp32 = false; // FP32-storage instances (one tile shape, 32x4)
     int* d_left = nullptr;       // [n] steps each instance still takes in the current call
     int* d_err = nullptr;        // [4] the kernels' item checks (BatchCtl::err)
     int* h_left = nullptr;       // pinned staging of d_left
@@ -594,7 +594,7 @@ int mhd_batch_destroy(mhd_batch* b) {
 
 int mhd_batch_set_tile(mhd_batch* b, int tile) {
     if (!b || tile < -1 || tile >= kBatchTiles) return MHD_ERR_INVALID;
-    if (b->fp32 && tile > 0) return MHD_ERR_INVALID;  // one tile shape (32x8) for FP32 storage
+    if (b->fp32 && tile > 0) return MHD_ERR_INVALID;  // one tile shape (32x4) for FP32 storage
     b->tile = tile;
     b->built = false;
     return MHD_OK;

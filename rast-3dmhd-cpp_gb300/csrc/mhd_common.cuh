@@ -299,9 +299,9 @@ int widen32(const Grid& g, const float* U, const double* bgR, const double* bgT,
 // lRem profiles (as lrem_profiles) of an FP32-storage temperature: the plane
 // means T0(z) + mean(dT) summed in FP64
 int lrem_profiles32(const Grid& g, const Consts& c, const float* dT, const double* bgT, double* buf, cudaStream_t st);
-// ragged batches of FP32-storage instances (tile 32x8; same item and counter
+// ragged batches of FP32-storage instances (tile 32x4; same item and counter
 // conventions as the FP64 batch)
-constexpr int kBatch32TX = 32, kBatch32TY = 8;
+constexpr int kBatch32TX = 32, kBatch32TY = 4;
 int fused32_batch_substage(unsigned sw, const Fused32Args* args, const int4* items, int nitems, int* counter,
                            BatchCtl ctl, int grid, cudaStream_t st);
 int fused32_batch_occupancy(unsigned sw, int* blocks_per_sm);

@@ -8,27 +8,38 @@ namespace {
 
 using namespace fp32;
 
-// CTAs per SM: two with 128 registers a thread, which hold the cell's register
-// values loaded at the start of the plane, against three with 80 (1453 and 1558 us
-// per step at 256x256x128 with lMag)
-constexpr int kResident = 2;
+// CTAs per SM: four, with 128 registers a thread in tiles of 4 rows (16 warps) and
+// 96 in tiles of 5 rows (20 warps), in both cases without spilling the cell's
+// register values loaded at the start of the plane.  Many small CTAs wait less at
+// the barrier of a plane than few large ones.  With lMag, us per step at 200x150x100
+// and at 256x256x128, us per step of a batch of 24 instances:
+//   two CTAs of 8 rows (128 registers)     680  1364  1983
+//   two of 10 rows (96)                    670  1335  2019
+//   four of 4 rows (128)                   651  1357  1867
+//   four of 5 rows (96)                    617  1275  2018
+//   five of 4 rows (96)                    687  1515  1980
+// Batches therefore run tiles of 4 rows, one instance the better of the two by
+// split32 below.
+constexpr int kResident = 4;
+using BatchTile = Tile<kBatch32TY>;
 
-// one instance: grid (x tiles, y tiles, z chunks)
-template <class SW, bool EXTRA>
-__global__ void __launch_bounds__(kThreads, kResident) k_substage32(Fused32Args a) {
+// one instance: grid (tiles, x fastest; 1; z chunks)
+template <class SW, class T, bool EXTRA>
+__global__ void __launch_bounds__(T::kThreads, kResident) k_substage32(Fused32Args a) {
     extern __shared__ float smem32[];
     const int nPz = a.g.nz - 2;
     const int zb = 1 + (int)((long long)nPz * blockIdx.z / gridDim.z);
     const int ze = 1 + (int)((long long)nPz * (blockIdx.z + 1) / gridDim.z);
-    substage32_tile<SW, EXTRA>(a, blockIdx.x, blockIdx.y, zb, ze, smem32);
+    const int nbx = (a.g.nx - 2 + kTX - 1) / kTX;
+    substage32_tile<SW, T, EXTRA>(a, blockIdx.x % nbx, blockIdx.x / nbx, zb, ze, smem32);
 }
 
 // ragged batch: persistent CTAs take (instance, tile x, tile y, z range) items
 // (w = first plane | end plane << 16) from a counter that is zero at launch
 template <class SW>
-__global__ void __launch_bounds__(kThreads, kResident) k_substage32_batch(const Fused32Args* __restrict__ args,
-                                                               const int4* __restrict__ items, int nitems,
-                                                               int* counter, BatchCtl ctl) {
+__global__ void __launch_bounds__(BatchTile::kThreads, kResident)
+    k_substage32_batch(const Fused32Args* __restrict__ args, const int4* __restrict__ items, int nitems, int* counter,
+                       BatchCtl ctl) {
     extern __shared__ float smem32[];
     constexpr int kArgWords = sizeof(Fused32Args) / sizeof(int);
     __shared__ __align__(16) int s_args[kArgWords];
@@ -44,10 +55,11 @@ __global__ void __launch_bounds__(kThreads, kResident) k_substage32_batch(const 
         if (!batch_item_ok(ctl, args, it, kBatch32TX, kBatch32TY, SW::lMag ? 8 : 5) || ctl.left[it.x] <= 0) continue;
         // the instance's arguments in shared memory: every access to a field reads
         // its pointer there
-        for (int k = threadIdx.x; k < kArgWords; k += kThreads)
+        for (int k = threadIdx.x; k < kArgWords; k += BatchTile::kThreads)
             s_args[k] = reinterpret_cast<const int*>(args + it.x)[k];
         __syncthreads();
-        substage32_tile<SW>(*reinterpret_cast<const Fused32Args*>(s_args), it.y, it.z, it.w & 0xffff, it.w >> 16, smem32);
+        substage32_tile<SW, BatchTile>(*reinterpret_cast<const Fused32Args*>(s_args), it.y, it.z, it.w & 0xffff,
+                                       it.w >> 16, smem32);
         __syncthreads();
     }
 }
@@ -114,25 +126,38 @@ int fused32_walls(int planes, int chunks) {
            (planes - chunk_begin(planes, chunks - 1, chunks) >= kWallPlanes ? 2 : 0);
 }
 
-// Number of z ranges per column.  Microseconds per launch of n CTAs with P planes
-// each, measured with lMag at 32^3 .. 256x256x128 for 1 .. 64 ranges:
-//   n <= 152 (one per SM)       13 + 2.8 P   one CTA alone leaves issue slots empty
-//   n <= 304 (all resident)     13 + 4.1 P
-//   more                        20 + W (2 + 4.1 P), W = 0.7 n / 304 + 0.3 ceil(n / 304)
-// (the planes around a range and its start-up are the constants), and 4 for a
-// separate BCON launch where a range at a wall is too short for it.
-int chunks32(long long tiles, int sms, int planes) {
-    int best = 1;
+// Microseconds per launch of n CTAs: tiles of ty rows, c z ranges.  While all are
+// resident, the planes of a CTA (0.8 more around a range) follow one another, L
+// each, and share their SM's issue slots with the other CTAs, q each; with more
+// CTAs than that, in waves that overlap in part, b per plane.  Last, a separate BCON
+// launch where a range at a wall is too short for it.  Fitted to launches with lMag
+// on 16 grids of 32^3 .. 512x384x96 cells, 1 .. 64 ranges and both tiles: what it
+// chooses is within 5 % of the fastest on each, 1 % on average.
+double cost32(int ty, long long n, int sms, int planes, int c) {
+    const double L = ty == 4 ? 1.6 : 2.0, q = ty == 4 ? 0.7 : 0.75, b = ty == 4 ? 4.3 : 4.7;
+    const double start = ty == 4 ? 15.0 : 19.0, f = ty == 4 ? 0.6 : 0.5;
+    const long long wave = (long long)kResident * sms, per_sm = (n + sms - 1) / sms;
+    const double most = (planes + c - 1) / c + 0.8, avg = (double)planes / c + 0.8;
+    const double waves = f * (double)n / wave + (1.0 - f) * (double)((n + wave - 1) / wave);
+    const double t = n <= wave ? 8.0 + L * most + q * per_sm * avg : start + b * waves * avg;
+    return fused32_walls(planes, c) == 3 ? t : t + 4.1;
+}
+
+// Rows per tile and number of z ranges for one instance of nx x ny interior columns.
+struct Split32 {
+    int ty, chunks;
+};
+Split32 split32(int nx, int ny, int planes, int sms) {
+    Split32 best{5, 1};
     double best_cost = 1e300;
-    for (int c = 1; c <= planes; c++) {
-        const long long n = tiles * c, wave = (long long)kResident * sms;
-        const double most = (planes + c - 1) / c, avg = (double)planes / c;
-        const double waves = 0.7 * (double)n / wave + 0.3 * (double)((n + wave - 1) / wave);
-        double cost = n <= sms ? 13.0 + 2.8 * most : n <= wave ? 13.0 + 4.1 * most : 20.0 + waves * (2.0 + 4.1 * avg);
-        if (fused32_walls(planes, c) != 3) cost += 4.0;
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = c;
+    for (int ty = 4; ty <= 5; ty++) {
+        const long long tiles = (long long)((nx + kTX - 1) / kTX) * ((ny + ty - 1) / ty);
+        for (int c = 1; c <= planes; c++) {
+            const double cost = cost32(ty, tiles * c, sms, planes, c);
+            if (cost < best_cost - 1e-9) {
+                best_cost = cost;
+                best = {ty, c};
+            }
         }
     }
     return best;
@@ -148,24 +173,30 @@ int sm_count() {
     return n;
 }
 
-template <class SW, bool EXTRA>
+template <class SW, class T, bool EXTRA>
 int launch32_t(const Fused32Args& a, dim3 grid, cudaStream_t st) {
-    const size_t smem = smem_bytes<SW>();
+    const size_t smem = smem_bytes<SW, T>();
     static const cudaError_t set =
-        cudaFuncSetAttribute(k_substage32<SW, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_substage32<SW, T, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (set != cudaSuccess) return (int)set;
-    k_substage32<SW, EXTRA><<<grid, kThreads, smem, st>>>(a);
+    k_substage32<SW, T, EXTRA><<<grid, T::kThreads, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
 
 template <class SW>
 void launch32(const Fused32Args& args, cudaStream_t st, int* rc) {
     Fused32Args a = args;
-    const int nbx = (a.g.nx - 2 + kBatch32TX - 1) / kBatch32TX, nby = (a.g.ny - 2 + kBatch32TY - 1) / kBatch32TY;
-    const int planes = a.g.nz - 2, chunks = chunks32((long long)nbx * nby, sm_count(), planes);
-    a.walls = fused32_walls(planes, chunks);
-    const dim3 grid(nbx, nby, chunks);
-    *rc = (a.c.pl_mode == 3 || a.c.lrem) ? launch32_t<SW, true>(a, grid, st) : launch32_t<SW, false>(a, grid, st);
+    const int planes = a.g.nz - 2;
+    const Split32 s = split32(a.g.nx - 2, a.g.ny - 2, planes, sm_count());
+    a.walls = fused32_walls(planes, s.chunks);
+    // (y tiles of few rows could exceed the y extent of a grid)
+    const dim3 grid((a.g.nx - 2 + kTX - 1) / kTX * ((a.g.ny - 2 + s.ty - 1) / s.ty), 1, s.chunks);
+    const bool extra = a.c.pl_mode == 3 || a.c.lrem;
+    if (s.ty == 4) {
+        *rc = extra ? launch32_t<SW, Tile<4>, true>(a, grid, st) : launch32_t<SW, Tile<4>, false>(a, grid, st);
+    } else {
+        *rc = extra ? launch32_t<SW, Tile<5>, true>(a, grid, st) : launch32_t<SW, Tile<5>, false>(a, grid, st);
+    }
     if (*rc || a.walls == 3) return;
     // the walls that the substage left
     const int first = a.walls & 1 ? 1 : 0, n = a.walls ? 1 : 2;
@@ -177,15 +208,16 @@ void launch32(const Fused32Args& args, cudaStream_t st, int* rc) {
 template <class SW>
 void batch32_launch(const Fused32Args* args, const int4* items, int nitems, int* counter, BatchCtl ctl, int grid,
                     cudaStream_t st, int* rc) {
-    k_substage32_batch<SW><<<grid, kThreads, smem_bytes<SW>(), st>>>(args, items, nitems, counter, ctl);
+    k_substage32_batch<SW><<<grid, BatchTile::kThreads, smem_bytes<SW, BatchTile>(), st>>>(args, items, nitems, counter, ctl);
     *rc = (int)cudaGetLastError();
 }
 
 template <class SW>
 void batch32_occupancy(int* blocks, int* rc) {
-    const size_t smem = smem_bytes<SW>();
+    const size_t smem = smem_bytes<SW, BatchTile>();
     cudaFuncSetAttribute(k_substage32_batch<SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    *rc = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_substage32_batch<SW>, kThreads, smem);
+    *rc = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_substage32_batch<SW>, BatchTile::kThreads,
+                                                             smem);
 }
 
 template <class SW>

@@ -26,10 +26,12 @@
 // in 3 and 11 instructions (mhd_convert.cuh): 1010 instructions per cell and
 // substage with lMag, against 1470 for the version before it, which read the z
 // neighbours' halos and had two barriers per plane.  Measured, with BCON inside:
-// a step at 256x256x128 1630 -> 1363 us, at 64x64x32 98 -> 72 us, a batch of 24
-// instances 2380 -> 1980 us.  Two cells per thread packed into f32x2 operations
-// need 730 instructions per cell but 168 registers, 12 warps per SM: 620 us per
-// substage against 455.
+// a step at 256x256x128 1630 -> 1290 us, at 64x64x32 98 -> 66 us, a batch of 24
+// instances 2380 -> 1870 us (see the CTA sizes in mhd_fp32.cu).  Two cells per
+// thread packed into f32x2 operations need 730 instructions per cell but 168
+// registers, 12 warps per SM: 620 us per substage against 425; updating the fields
+// of a plane in four groups, each where its right-hand sides are complete, was 2 %
+// slower than all at the plane's end.
 #pragma once
 
 #include "mhd_common.cuh"
@@ -41,12 +43,15 @@ namespace mhd {
 namespace fp32 {
 
 // 32 columns per row: a warp's shared-memory accesses touch every bank once
-constexpr int kTX = 32, kTY = 8;
-constexpr int kThreads = kTX * kTY;
-constexpr int kPX = kTX + 2, kPY = kTY + 2;
-constexpr int kPlane = kPX * kPY;
-constexpr int kHalo = kPlane - kThreads;
-static_assert(kHalo <= kThreads, "one halo point per thread at most");
+constexpr int kTX = 32, kPX = kTX + 2;
+template <int TY>
+struct Tile {
+    static constexpr int kTY = TY;
+    static constexpr int kThreads = kTX * kTY;
+    static constexpr int kPlane = kPX * (kTY + 2);
+    static constexpr int kHalo = kPlane - kThreads;
+    static_assert(kHalo <= kThreads, "one halo point per thread at most");
+};
 
 // quantities of a ring plane, with halo: P_X, P_Y are dp + RU u, dp + RV v
 enum QF { F_RU = 0, F_RV, F_DT, F_U, F_V, F_W, F_PX, F_PY, F_BX, F_BY, F_BZ, F_NQ };
@@ -73,8 +78,9 @@ constexpr int nraw() {
 // floats: ring [3][nq][plane], Q1 and Q2 [2][2][plane], raw staging [nraw][plane], own columns [3][G_N][threads],
 // coefficient rows, x and y second-derivative coefficients [kCoef][kTX], [kCoef][kTY], scalars; before them the RK
 // coefficients (doubles)
-template <class SW>
+template <class SW, class T>
 constexpr size_t smem_bytes() {
+    constexpr int kPlane = T::kPlane, kThreads = T::kThreads, kTY = T::kTY;
     return ((size_t)(3 * nqf<SW>() + 4 + nraw<SW>()) * kPlane + 3 * G_N * kThreads + kZRing * ZF_N +
             kCoef * (kTX + kTY) + K_N) * sizeof(float) + R_N * sizeof(double);
 }
@@ -205,8 +211,9 @@ __device__ __forceinline__ Point point_values(const float* row, float ru, float 
 
 // One tile (bx, by) of one instance, interior z planes [zb, ze).  EXTRA: the
 // instantiation with the iTCon 2 plume heat sink and lRem.
-template <class SW, bool EXTRA = false>
+template <class SW, class T, bool EXTRA = false>
 __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, int by, int zb, int ze, float* smem) {
+    constexpr int kTY = T::kTY, kThreads = T::kThreads, kPlane = T::kPlane;
     constexpr int NQ = nqf<SW>(), NRAW = nraw<SW>();
     constexpr int kOwn = NQ * kPlane;
     constexpr int kSlot = NQ * kPlane + G_N * kThreads;  // a plane's arrays, then its own-column ones
@@ -238,7 +245,7 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
         const int r = tid - 2 * kTX;
         hk = (1 + r % kTY) * kPX + (r < kTY ? 0 : kPX - 1);
         hkind = 1;
-    } else if (tid < kHalo) {
+    } else if (tid < T::kHalo) {
         const int r = tid - 2 * kTX - 2 * kTY;
         hk = ((r & 2) ? (kTY + 1) * kPX : 0) + ((r & 1) ? kPX - 1 : 0);
         hkind = 2;

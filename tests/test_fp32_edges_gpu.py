@@ -1,6 +1,6 @@
-"""The FP32-storage substage at the edges of its 32 x 8 tile and of its z
-ranges, on isotropic, unequal and stretched x / y spacings: one step against
-the oracle within 1e-5 of each field's max-norm (the bound of the FP32-storage
+"""The FP32-storage substage at the edges of its tiles (32 columns by 4
+or 5 rows) and of its z ranges, on isotropic, unequal and stretched x / y
+spacings: one step against the oracle within 1e-5 of each field's max-norm (the bound of the FP32-storage
 form: its stencils work on floats, 6e-8, amplified by at most the 1e2 of the
 differenced terms), and a non-finite state that stays non-finite where it is
 and finite elsewhere.
@@ -14,7 +14,9 @@ from mhd_gb300.sim import Simulation
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(31, 7, 4), (32, 8, 5), (33, 9, 6), (2, 2, 4), (64, 17, 7), (40, 25, 33)]
+SIZES = [(31, 7, 4), (32, 8, 5), (33, 9, 6), (2, 2, 4), (64, 17, 7), (40, 25, 33),
+         # large enough for tiles of 5 rows: remainders 1, 4, 0
+         (161, 101, 6), (97, 79, 6), (193, 50, 6)]
 
 
 @pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
