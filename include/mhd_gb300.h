@@ -329,7 +329,7 @@ typedef struct mhd_batch mhd_batch;
 int mhd_batch_create(mhd_ctx* const* ctxs, const double* dts, int n, void* stream, mhd_batch** out);
 int mhd_batch_destroy(mhd_batch* b);
 /* tile shape: -1 = autotune on the next step, 0 = 32x4, 1 = 32x8, 2 = 16x8
- * (FP32-storage batches: 32x8, accepted as 0) */
+ * (FP32-storage batches: 32 columns by 4 rows, accepted as 0) */
 int mhd_batch_set_tile(mhd_batch* b, int tile);
 int mhd_batch_tile(const mhd_batch* b, int* tile);
 /* longest z range of a work item, in planes (default 64): an instance with

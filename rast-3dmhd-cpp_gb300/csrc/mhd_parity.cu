@@ -21,42 +21,102 @@
 namespace mhd {
 namespace {
 
-struct Ix {
-    long long i, sy, sz;
-    int x, y, z;
+// Scalars of k_flux: factors with the reference's association, and the operands
+// that make sums and products of fused multiply-adds (below).
+struct FluxScalars {
+    double one, nzero, mtwo;  // 1, -0, -2
+    double hx, h2x, hy, h2y, hz, h2z;
+    double ORE, ore43, c13ore;               // ORE, ORE C43, C13 ORE
+    double OCV, ocv_repr, ocvore, ocvore43;  // OCV, OCV / REPR, OCV ORE, (OCV ORE) C43
+    double ocvore2, c43ocvore;               // 2 (OCV ORE), (C43 OCV) ORE
+    double OMX, OMZ, OBETA, ORM, c1, c2;     // ..., Ohmic heating
 };
 
-__device__ __forceinline__ double d1x(const double* F, long long i, int x, const Consts& c) {
-    return ((F[i + 1] - F[i - 1]) * c.dxxdx[x]) * c.hx;
+__shared__ FluxScalars s_flux;
+constexpr int kFluxThreads = 128;
+
+FluxScalars flux_scalars(const Consts& c) {
+    FluxScalars k;
+    k.one = 1.0;
+    k.nzero = -0.0;
+    k.mtwo = -2.0;
+    k.hx = c.hx;
+    k.h2x = c.h2x;
+    k.hy = c.hy;
+    k.h2y = c.h2y;
+    k.hz = c.hz;
+    k.h2z = c.h2z;
+    k.ORE = c.ORE;
+    k.ore43 = c.ORE * c.C43;
+    k.c13ore = c.C13 * c.ORE;
+    k.OCV = c.OCV;
+    k.ocv_repr = c.OCV / c.REPR;
+    k.ocvore = c.OCV * c.ORE;
+    k.ocvore43 = k.ocvore * c.C43;
+    k.ocvore2 = k.ocvore * 2;
+    k.c43ocvore = c.C43 * c.OCV * c.ORE;
+    k.OMX = c.OMX;
+    k.OMZ = c.OMZ;
+    k.OBETA = c.OBETA;
+    k.ORM = c.ORM;
+    k.c1 = c.OBETA * c.ORM * c.OCV;
+    k.c2 = -2.0f * c.OBETA * c.ORM * c.OCV;
+    return k;
 }
-__device__ __forceinline__ double d1y(const double* F, long long i, long long sy, int y, const Consts& c) {
-    return ((F[i + sy] - F[i - sy]) * c.dyydy[y]) * c.hy;
+
+// A double whose sums, differences and products are single fused multiply-adds
+// with 1 or -0: the same bits as DADD and DMUL, but the FP64 unit takes 16 cycles
+// per warp for a fused multiply-add of three registers and 19 for DADD, DMUL or an
+// operand from the constant bank (one unit per SM).  1 and -0 come from shared
+// memory, so that the compiler does not know them.
+struct D {
+    double v;
+    __device__ __forceinline__ D(double d) : v(d) {}
+};
+__device__ __forceinline__ D operator+(D a, D b) { return fma(a.v, s_flux.one, b.v); }
+__device__ __forceinline__ D operator-(D a, D b) { return fma(-b.v, s_flux.one, a.v); }
+__device__ __forceinline__ D operator*(D a, D b) { return fma(a.v, b.v, s_flux.nzero); }
+__device__ __forceinline__ D operator-(D a) { return -a.v; }
+__device__ __forceinline__ D& operator+=(D& a, D b) { return a = a + b; }
+__device__ __forceinline__ D& operator-=(D& a, D b) { return a = a - b; }
+
+struct Field {
+    const double* p;
+    __device__ __forceinline__ D operator[](long long i) const { return p[i]; }
+};
+
+// (p - 2 c) + m; 2 c is exact
+__device__ __forceinline__ D second(D p, D c, D m) { return D(fma(s_flux.mtwo, c.v, p.v)) + m; }
+
+__device__ __forceinline__ D d1x(Field F, long long i, int x, const Consts& c) {
+    return ((F[i + 1] - F[i - 1]) * c.dxxdx[x]) * s_flux.hx;
 }
-__device__ __forceinline__ double d1z(const double* F, long long i, long long sz, int z, const Consts& c) {
-    return ((F[i + sz] - F[i - sz]) * c.dzzdz[z]) * c.hz;
+__device__ __forceinline__ D d1y(Field F, long long i, long long sy, int y, const Consts& c) {
+    return ((F[i + sy] - F[i - sy]) * c.dyydy[y]) * s_flux.hy;
 }
-__device__ __forceinline__ double d2x(const double* F, long long i, int x, const Consts& c) {
-    const double du = c.dxxdx[x];
-    return ((F[i + 1] - F[i - 1]) * c.d2xxdx2[x]) * c.hx + (((F[i + 1] - 2 * F[i]) + F[i - 1]) * (du * du)) * c.h2x;
+__device__ __forceinline__ D d1z(Field F, long long i, long long sz, int z, const Consts& c) {
+    return ((F[i + sz] - F[i - sz]) * c.dzzdz[z]) * s_flux.hz;
 }
-__device__ __forceinline__ double d2y(const double* F, long long i, long long sy, int y, const Consts& c) {
-    const double du = c.dyydy[y];
-    return ((F[i + sy] - F[i - sy]) * c.d2yydy2[y]) * c.hy + (((F[i + sy] - 2 * F[i]) + F[i - sy]) * (du * du)) * c.h2y;
+__device__ __forceinline__ D d2(D p, D f, D m, D a, D du, D h, D h2) {
+    return ((p - m) * a) * h + (second(p, f, m) * (du * du)) * h2;
 }
-__device__ __forceinline__ double d2z(const double* F, long long i, long long sz, int z, const Consts& c) {
-    const double du = c.dzzdz[z];
-    return ((F[i + sz] - F[i - sz]) * c.d2zzdz2[z]) * c.hz + (((F[i + sz] - 2 * F[i]) + F[i - sz]) * (du * du)) * c.h2z;
+__device__ __forceinline__ D d2x(Field F, long long i, int x, const Consts& c) {
+    return d2(F[i + 1], F[i], F[i - 1], c.d2xxdx2[x], c.dxxdx[x], s_flux.hx, s_flux.h2x);
 }
-__device__ __forceinline__ double mdx(const double* F, const double* G, long long i, int x, const Consts& c) {
-    return ((F[i + 1] * G[i + 1] - F[i - 1] * G[i - 1]) * c.dxxdx[x]) * c.hx;
+__device__ __forceinline__ D d2y(Field F, long long i, long long sy, int y, const Consts& c) {
+    return d2(F[i + sy], F[i], F[i - sy], c.d2yydy2[y], c.dyydy[y], s_flux.hy, s_flux.h2y);
 }
-__device__ __forceinline__ double mdy(const double* F, const double* G, long long i, long long sy, int y,
-                                      const Consts& c) {
-    return ((F[i + sy] * G[i + sy] - F[i - sy] * G[i - sy]) * c.dyydy[y]) * c.hy;
+__device__ __forceinline__ D d2z(Field F, long long i, long long sz, int z, const Consts& c) {
+    return d2(F[i + sz], F[i], F[i - sz], c.d2zzdz2[z], c.dzzdz[z], s_flux.hz, s_flux.h2z);
 }
-__device__ __forceinline__ double mdz(const double* F, const double* G, long long i, long long sz, int z,
-                                      const Consts& c) {
-    return ((F[i + sz] * G[i + sz] - F[i - sz] * G[i - sz]) * c.dzzdz[z]) * c.hz;
+__device__ __forceinline__ D mdx(Field F, Field G, long long i, int x, const Consts& c) {
+    return ((F[i + 1] * G[i + 1] - F[i - 1] * G[i - 1]) * c.dxxdx[x]) * s_flux.hx;
+}
+__device__ __forceinline__ D mdy(Field F, Field G, long long i, long long sy, int y, const Consts& c) {
+    return ((F[i + sy] * G[i + sy] - F[i - sy] * G[i - sy]) * c.dyydy[y]) * s_flux.hy;
+}
+__device__ __forceinline__ D mdz(Field F, Field G, long long i, long long sz, int z, const Consts& c) {
+    return ((F[i + sz] * G[i + sz] - F[i - sz] * G[i - sz]) * c.dzzdz[z]) * s_flux.hz;
 }
 
 // Pressure, gravity, 1/rho in place and the velocities over the extended
@@ -99,15 +159,27 @@ __global__ void k_prep_ext(Grid g, Consts c, Fields8 U, double* RI, double* FW, 
     }
 }
 
+// Bound by the FP64 unit: 603 instructions per cell with lMag, none of which the
+// reference's rounding lets go (the neighbours' derivatives of the cross terms are
+// 36 of them; exchanging them through shared memory needs 2-D tiles, whose waste on
+// rows that 32 does not divide is larger).  Constant products and OCV / REPR come
+// from the host.  64x64x32 with lMag: 172 us with DADD and DMUL, 151 now (the unit
+// is 88 % busy between launch and drain); blocks of 32, 64 and 128 threads are equal.
 template <class SW>
-__global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __restrict__ P,
-                       const double* __restrict__ UU, const double* __restrict__ VV, const double* __restrict__ WW) {
+__global__ void __launch_bounds__(kFluxThreads) k_flux(Grid g, Consts c, FluxScalars scalars, Fields8 U, Fields8 F, const double* __restrict__ P_,
+                       const double* __restrict__ U_, const double* __restrict__ V_, const double* __restrict__ W_) {
+    static_assert(sizeof(FluxScalars) / sizeof(double) <= kFluxThreads);
+    if (threadIdx.x < sizeof(FluxScalars) / sizeof(double))
+        reinterpret_cast<double*>(&s_flux)[threadIdx.x] = reinterpret_cast<const double*>(&scalars)[threadIdx.x];
+    __syncthreads();
+    const FluxScalars& k = s_flux;
+    const Field P{P_}, UU{U_}, VV{V_}, WW{W_};
     const int nPx = g.nx - 2, nPy = g.ny - 2, nPz = g.nz - 2;
     const long long ncell = (long long)nPx * nPy * nPz;
     const long long sy = g.sy, sz = g.sz;
     const int zl = 1, zr = g.nz - 1;
-    const double *RU = U.p[S_RU], *RV = U.p[S_RV], *RW = U.p[S_RW], *TT = U.p[S_TT], *RI = U.p[S_RO];
-    const double *BX = U.p[S_BX], *BY = U.p[S_BY], *BZ = U.p[S_BZ];
+    const Field RU{U.p[S_RU]}, RV{U.p[S_RV]}, RW{U.p[S_RW]}, TT{U.p[S_TT]}, RI{U.p[S_RO]};
+    const Field BX{U.p[S_BX]}, BY{U.p[S_BY]}, BZ{U.p[S_BZ]};
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ncell;
          t += (long long)gridDim.x * blockDim.x) {
         const int x = 1 + (int)(t % nPx);
@@ -116,18 +188,18 @@ __global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __r
         const long long i = z * sz + y * sy + x;
 
         // continuity, 3dmhdsub.h:204-227
-        double fr = -d1x(RU, i, x, c);
+        D fr = -d1x(RU, i, x, c);
         fr -= d1y(RV, i, sy, y, c);
-        double w1 = d1z(RW, i, sz, z, c);
-        if (z == zl) w1 = (4.0f * RW[i + sz] - RW[i + 2 * sz]) * (c.hz * c.dzzdz[zl]);
-        if (z == zr - 1) w1 = (RW[i - 2 * sz] - 4.0f * RW[i - sz]) * (c.hz * c.dzzdz[zr - 1]);
+        D w1 = d1z(RW, i, sz, z, c);
+        if (z == zl) w1 = (4.0f * RW[i + sz] - RW[i + 2 * sz]) * (k.hz * c.dzzdz[zl]);
+        if (z == zr - 1) w1 = (RW[i - 2 * sz] - 4.0f * RW[i - sz]) * (k.hz * c.dzzdz[zr - 1]);
         fr -= w1;
 
         // pressure and gravity, 3dmhdsub.h:266-272 (F.FW holds RO*GRAV from k_prep)
-        double fw = F.p[F_FW][i];
+        D fw = F.p[F_FW][i];
         fw -= d1z(P, i, sz, z, c);
-        double fv = -d1y(P, i, sy, y, c);
-        double fu = -d1x(P, i, x, c);
+        D fv = -d1y(P, i, sy, y, c);
+        D fu = -d1x(P, i, x, c);
 
         // momentum advection, 3dmhdsub.h:279-289
         fu -= mdx(RU, UU, i, x, c);
@@ -140,10 +212,10 @@ __global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __r
         fw -= mdy(RW, VV, i, sy, y, c);
         fw -= mdz(RW, WW, i, sz, z, c);
 
-        const double ri = RI[i], tt = TT[i];
+        const D ri = RI[i], tt = TT[i];
         // temperature advection, 3dmhdsub.h:293-296.  With lShr the reference
         // never re-initialises FT, so it keeps accumulating across calls.
-        double ft;
+        D ft = 0.0;
         if constexpr (!SW::lShr) {
             ft = -(d1x(TT, i, x, c) * UU[i]);
             ft -= d1y(TT, i, sy, y, c) * VV[i];
@@ -151,19 +223,18 @@ __global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __r
         } else {
             ft = F.p[F_FT][i];
         }
-        double tmp = c.OCV / c.REPR;
+        D tmp = k.ocv_repr;
         if (c.lrem && !SW::lShr) {
             // lRem: conduction of W = T - TTM(z) plus the mean profile's HRAD,
             // 3dmhdsub.h:297-313 (W at the stencil points as the reference stores it)
-            const double* M = c.lrem_ttm;
-            const double wc = tt - M[z];
-            const double wxp = TT[i + 1] - M[z], wxm = TT[i - 1] - M[z];
-            const double wyp = TT[i + sy] - M[z], wym = TT[i - sy] - M[z];
-            const double wzp = TT[i + sz] - M[z + 1], wzm = TT[i - sz] - M[z - 1];
-            const double dx = c.dxxdx[x], dy = c.dyydy[y], dz = c.dzzdz[z];
-            const double d2wx = ((wxp - wxm) * c.d2xxdx2[x]) * c.hx + (((wxp - 2 * wc) + wxm) * (dx * dx)) * c.h2x;
-            const double d2wy = ((wyp - wym) * c.d2yydy2[y]) * c.hy + (((wyp - 2 * wc) + wym) * (dy * dy)) * c.h2y;
-            const double d2wz = ((wzp - wzm) * c.d2zzdz2[z]) * c.hz + (((wzp - 2 * wc) + wzm) * (dz * dz)) * c.h2z;
+            const Field M{c.lrem_ttm};
+            const D wc = tt - M[z];
+            const D wxp = TT[i + 1] - M[z], wxm = TT[i - 1] - M[z];
+            const D wyp = TT[i + sy] - M[z], wym = TT[i - sy] - M[z];
+            const D wzp = TT[i + sz] - M[z + 1], wzm = TT[i - sz] - M[z - 1];
+            const D d2wx = d2(wxp, wc, wxm, c.d2xxdx2[x], c.dxxdx[x], k.hx, k.h2x);
+            const D d2wy = d2(wyp, wc, wym, c.d2yydy2[y], c.dyydy[y], k.hy, k.h2y);
+            const D d2wz = d2(wzp, wc, wzm, c.d2zzdz2[z], c.dzzdz[z], k.hz, k.h2z);
             ft += (d2wx * ri) * tmp;
             ft += (d2wy * ri) * tmp;
             ft += (d2wz * ri) * tmp;
@@ -179,102 +250,99 @@ __global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __r
         if (c.pl_mode == 3) ft -= (((c.pl_s * ri) * c.plx[x]) * c.ply[y]) * c.plz[z];
 
         // viscous Laplacians, 3dmhdsub.h:462-472
-        fu += d2x(UU, i, x, c) * (c.ORE * c.C43);
-        fu += d2y(UU, i, sy, y, c) * c.ORE;
-        fu += d2z(UU, i, sz, z, c) * c.ORE;
-        fv += d2x(VV, i, x, c) * c.ORE;
-        fv += d2y(VV, i, sy, y, c) * (c.ORE * c.C43);
-        fv += d2z(VV, i, sz, z, c) * c.ORE;
-        fw += d2x(WW, i, x, c) * c.ORE;
-        fw += d2y(WW, i, sy, y, c) * c.ORE;
-        fw += d2z(WW, i, sz, z, c) * (c.ORE * c.C43);
+        fu += d2x(UU, i, x, c) * k.ore43;
+        fu += d2y(UU, i, sy, y, c) * k.ORE;
+        fu += d2z(UU, i, sz, z, c) * k.ORE;
+        fv += d2x(VV, i, x, c) * k.ORE;
+        fv += d2y(VV, i, sy, y, c) * k.ore43;
+        fv += d2z(VV, i, sz, z, c) * k.ORE;
+        fw += d2x(WW, i, x, c) * k.ORE;
+        fw += d2y(WW, i, sy, y, c) * k.ORE;
+        fw += d2z(WW, i, sz, z, c) * k.ore43;
 
         // viscous cross terms, heating and pdV work, 3dmhdsub.h:475-538
-        const double c13ore = c.C13 * c.ORE;
-        const double ux = d1x(UU, i, x, c);  // WW1 of do 650
-        const double vx = d1x(VV, i, x, c);  // WW2 of do 670
-        double vy = 0.0;
+        const D ux = d1x(UU, i, x, c);  // WW1 of do 650
+        const D vx = d1x(VV, i, x, c);  // WW2 of do 670
+        D vy = 0.0;
         if constexpr (!SW::lShr) {
-            const double wx = d1x(WW, i, x, c);  // do 690
-            tmp = c.OCV * c.ORE;
-            ft += ((ri * ux) * ux) * (tmp * c.C43);
+            const D wx = d1x(WW, i, x, c);  // do 690
+            tmp = k.ocvore;
+            ft += ((ri * ux) * ux) * k.ocvore43;
             ft += ((ri * vx) * vx) * tmp;
             ft += ((ri * wx) * wx) * tmp;
-            ft -= (ux * tt) * c.OCV;
+            ft -= (ux * tt) * k.OCV;
         }
-        fu += (((d1x(VV, i + sy, x, c) - d1x(VV, i - sy, x, c)) * c.dyydy[y]) * c.hy) * c13ore;  // do 720
-        fv += (((d1x(UU, i + sy, x, c) - d1x(UU, i - sy, x, c)) * c.dyydy[y]) * c.hy) * c13ore;  // do 730
+        fu += (((d1x(VV, i + sy, x, c) - d1x(VV, i - sy, x, c)) * c.dyydy[y]) * k.hy) * k.c13ore;  // do 720
+        fv += (((d1x(UU, i + sy, x, c) - d1x(UU, i - sy, x, c)) * c.dyydy[y]) * k.hy) * k.c13ore;  // do 730
         if constexpr (!SW::lShr) {
-            const double uy = d1y(UU, i, sy, y, c);  // do 740
-            tmp = c.OCV * c.ORE;
+            const D uy = d1y(UU, i, sy, y, c);  // do 740
+            tmp = k.ocvore;
             ft += ((ri * uy) * uy) * tmp;
-            ft += ((ri * uy) * vx) * (tmp * 2);
+            ft += ((ri * uy) * vx) * k.ocvore2;
             vy = d1y(VV, i, sy, y, c);  // do 755
-            tmp = c.C43 * c.OCV * c.ORE;
+            tmp = k.c43ocvore;
             ft += ((ri * vy) * vy) * tmp;
-            ft -= (vy * tt) * c.OCV;
+            ft -= (vy * tt) * k.OCV;
         }
-        const double wz = d1z(WW, i, sz, z, c);  // do 790
+        const D wz = d1z(WW, i, sz, z, c);  // do 790
         if constexpr (!SW::lShr) {
-            tmp = c.C43 * c.OCV * c.ORE;
+            tmp = k.c43ocvore;
             ft += ((ri * wz) * wz) * tmp;
             ft += ((ri * ux) * wz) * (-tmp);
             ft += ((ri * ux) * vy) * (-tmp);
             ft += ((ri * vy) * wz) * (-tmp);
-            ft -= (wz * tt) * c.OCV;
+            ft -= (wz * tt) * k.OCV;
         }
-        fu += (((d1z(WW, i + 1, sz, z, c) - d1z(WW, i - 1, sz, z, c)) * c.dxxdx[x]) * c.hx) * c13ore;   // do 840
-        fv += (((d1z(WW, i + sy, sz, z, c) - d1z(WW, i - sy, sz, z, c)) * c.dyydy[y]) * c.hy) * c13ore; // do 850
-        const double uz = d1z(UU, i, sz, z, c);  // do 860
-        const double vz = d1z(VV, i, sz, z, c);  // do 880
+        fu += (((d1z(WW, i + 1, sz, z, c) - d1z(WW, i - 1, sz, z, c)) * c.dxxdx[x]) * k.hx) * k.c13ore;   // do 840
+        fv += (((d1z(WW, i + sy, sz, z, c) - d1z(WW, i - sy, sz, z, c)) * c.dyydy[y]) * k.hy) * k.c13ore; // do 850
+        const D uz = d1z(UU, i, sz, z, c);  // do 860
+        const D vz = d1z(VV, i, sz, z, c);  // do 880
         if constexpr (!SW::lShr) {
-            const double wy = d1y(WW, i, sy, y, c);  // do 900
-            tmp = c.OCV * c.ORE;
+            const D wy = d1y(WW, i, sy, y, c);  // do 900
+            tmp = k.ocvore;
             ft += ((ri * uz) * uz) * tmp;
             ft += ((ri * vz) * vz) * tmp;
             ft += ((ri * wy) * wy) * tmp;
-            ft += ((ri * vz) * wy) * (2.0f * tmp);
+            ft += ((ri * vz) * wy) * k.ocvore2;
         }
-        fw += (((d1z(UU, i + 1, sz, z, c) - d1z(UU, i - 1, sz, z, c)) * c.dxxdx[x]) * c.hx) * c13ore;   // do 920.1
-        fw += (((d1z(VV, i + sy, sz, z, c) - d1z(VV, i - sy, sz, z, c)) * c.dyydy[y]) * c.hy) * c13ore; // do 920.2
+        fw += (((d1z(UU, i + 1, sz, z, c) - d1z(UU, i - 1, sz, z, c)) * c.dxxdx[x]) * k.hx) * k.c13ore;   // do 920.1
+        fw += (((d1z(VV, i + sy, sz, z, c) - d1z(VV, i - sy, sz, z, c)) * c.dyydy[y]) * k.hy) * k.c13ore; // do 920.2
         if constexpr (!SW::lShr) {
-            const double wx = d1x(WW, i, x, c);  // do 930
-            tmp = c.OCV * c.ORE;
-            ft += ((ri * uz) * wx) * (2.0f * tmp);
+            const D wx = d1x(WW, i, x, c);  // do 930
+            tmp = k.ocvore;
+            ft += ((ri * uz) * wx) * k.ocvore2;
         }
 
         // Coriolis, 3dmhdsub.h:540-545
         if constexpr (SW::lRot) {
-            fu += RV[i] * c.OMZ;
-            fv -= RU[i] * c.OMZ;
-            fv += RW[i] * c.OMX;
-            fw -= RV[i] * c.OMX;
+            fu += RV[i] * k.OMZ;
+            fv -= RU[i] * k.OMZ;
+            fv += RW[i] * k.OMX;
+            fw -= RV[i] * k.OMX;
         }
 
         // induction, Lorentz force and Ohmic heating, 3dmhdsub.h:547-695.
         // sRU..sTT stand for the reference's reuse of RU, RV, RW, TT as scratch.
         if constexpr (SW::lMag) {
-            const double c1 = c.OBETA * c.ORM * c.OCV;
-            const double c2 = -2.0f * c.OBETA * c.ORM * c.OCV;
-            const double bx = BX[i], by = BY[i], bz = BZ[i];
-            const double u = UU[i], v = VV[i], w = WW[i];
-            double sRU = d1x(UU, i, x, c), sRV = d1x(VV, i, x, c), sRW = d1x(WW, i, x, c), sTT;
-            double ww2 = bx * sRV;
+            const D bx = BX[i], by = BY[i], bz = BZ[i];
+            const D u = UU[i], v = VV[i], w = WW[i];
+            D sRU = d1x(UU, i, x, c), sRV = d1x(VV, i, x, c), sRW = d1x(WW, i, x, c);
+            D ww2 = bx * sRV;
             ww2 -= by * sRU;
-            double ww3 = bx * sRW;
+            D ww3 = bx * sRW;
             ww3 -= bz * sRU;
             sRU = d1y(UU, i, sy, y, c);
             sRV = d1y(VV, i, sy, y, c);
             sRW = d1y(WW, i, sy, y, c);
-            double ww1 = by * sRU;
+            D ww1 = by * sRU;
             ww1 -= bx * sRV;
             ww3 += by * sRW;
             ww3 -= bz * sRV;
             sRU = d1z(UU, i, sz, z, c);
             sRV = d1z(VV, i, sz, z, c);
             sRW = d1z(WW, i, sz, z, c);
-            if (z == zl) sRW = (4.0f * WW[i + sz] - WW[i + 2 * sz]) * c.hz * c.dzzdz[zl];
-            if (z == zr - 1) sRW = (-4.0f * WW[i - sz] + WW[i - 2 * sz]) * c.hz * c.dzzdz[zr - 1];
+            if (z == zl) sRW = (4.0f * WW[i + sz] - WW[i + 2 * sz]) * k.hz * c.dzzdz[zl];
+            if (z == zr - 1) sRW = (-4.0f * WW[i - sz] + WW[i - 2 * sz]) * k.hz * c.dzzdz[zr - 1];
             ww1 += bz * sRU;
             ww1 -= bx * sRW;
             ww2 += bz * sRV;
@@ -282,17 +350,17 @@ __global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __r
             sRU = d1x(BX, i, x, c);
             sRV = d1x(BY, i, x, c);
             sRW = d1x(BZ, i, x, c);
-            sTT = d1y(BX, i, sy, y, c);
-            fu += (by * sTT) * c.OBETA;
-            fu -= (by * sRV) * c.OBETA;
-            fu -= (bz * sRW) * c.OBETA;
-            fv += (bx * sRV) * c.OBETA;
-            fv -= (bx * sTT) * c.OBETA;
-            fw += (bx * sRW) * c.OBETA;
-            ft += ((ri * sTT) * sTT) * c1;
-            ft += ((ri * sRV) * sRV) * c1;
-            ft += ((ri * sRW) * sRW) * c1;
-            ft += ((ri * sRV) * sTT) * c2;
+            D sTT = d1y(BX, i, sy, y, c);
+            fu += (by * sTT) * k.OBETA;
+            fu -= (by * sRV) * k.OBETA;
+            fu -= (bz * sRW) * k.OBETA;
+            fv += (bx * sRV) * k.OBETA;
+            fv -= (bx * sTT) * k.OBETA;
+            fw += (bx * sRW) * k.OBETA;
+            ft += ((ri * sTT) * sTT) * k.c1;
+            ft += ((ri * sRV) * sRV) * k.c1;
+            ft += ((ri * sRW) * sRW) * k.c1;
+            ft += ((ri * sRV) * sTT) * k.c2;
             ww1 -= u * sRU;
             ww1 -= v * sTT;
             ww2 -= u * sRV;
@@ -300,67 +368,67 @@ __global__ void k_flux(Grid g, Consts c, Fields8 U, Fields8 F, const double* __r
             sRU = d2x(BX, i, x, c);
             sRV = d2x(BY, i, x, c);
             sTT = d2y(BX, i, sy, y, c);
-            ww1 += sRU * c.ORM;
-            ww1 += sTT * c.ORM;
-            ww2 += sRV * c.ORM;
+            ww1 += sRU * k.ORM;
+            ww1 += sTT * k.ORM;
+            ww2 += sRV * k.ORM;
             sTT = d2x(BZ, i, x, c);
-            ww3 += sTT * c.ORM;
+            ww3 += sTT * k.ORM;
             sRU = d1z(BX, i, sz, z, c);
             sRV = d1y(BY, i, sy, y, c);
-            fu += (bz * sRU) * c.OBETA;
-            fw -= (bx * sRU) * c.OBETA;
-            ft += ((ri * sRU) * sRU) * c1;
-            ft += ((ri * sRU) * sRW) * c2;
+            fu += (bz * sRU) * k.OBETA;
+            fw -= (bx * sRU) * k.OBETA;
+            ft += ((ri * sRU) * sRU) * k.c1;
+            ft += ((ri * sRU) * sRW) * k.c2;
             ww1 -= w * sRU;
             ww2 -= v * sRV;
             sRU = d2z(BX, i, sz, z, c);
             if (z == zl)
-                sRU = (-3.0f * BX[i] + 4.0f * BX[i + sz] - BX[i + 2 * sz]) * c.hz * c.d2zzdz2[zl] +
-                      (2.0f * BX[i] - 5.0f * BX[i + sz] + 4.0f * BX[i + 2 * sz] - BX[i + 3 * sz]) * c.h2z * c.dzzdz[zl] *
+                sRU = (-3.0f * BX[i] + 4.0f * BX[i + sz] - BX[i + 2 * sz]) * k.hz * c.d2zzdz2[zl] +
+                      (2.0f * BX[i] - 5.0f * BX[i + sz] + 4.0f * BX[i + 2 * sz] - BX[i + 3 * sz]) * k.h2z * c.dzzdz[zl] *
                           c.dzzdz[zl];
             if (z == zr - 1)
-                sRU = (3.0f * BX[i] - 4.0f * BX[i - sz] + BX[i - 2 * sz]) * c.hz * c.d2zzdz2[zr - 1] +
-                      (2.0f * BX[i] - 5.0f * BX[i - sz] + 4.0f * BX[i - 2 * sz] - BX[i - 3 * sz]) * c.h2z *
+                sRU = (3.0f * BX[i] - 4.0f * BX[i - sz] + BX[i - 2 * sz]) * k.hz * c.d2zzdz2[zr - 1] +
+                      (2.0f * BX[i] - 5.0f * BX[i - sz] + 4.0f * BX[i - 2 * sz] - BX[i - 3 * sz]) * k.h2z *
                           c.dzzdz[zr - 1] * c.dzzdz[zr - 1];
             sRV = d2y(BY, i, sy, y, c);
-            ww1 += sRU * c.ORM;
-            ww2 += sRV * c.ORM;
+            ww1 += sRU * k.ORM;
+            ww2 += sRV * k.ORM;
             sRV = d1z(BY, i, sz, z, c);
             sRW = d1y(BZ, i, sy, y, c);
             sRU = sRV;
             sRU -= sRW;
-            fv += (bz * sRU) * c.OBETA;
-            fw -= (by * sRU) * c.OBETA;
-            ft += ((ri * sRV) * sRV) * c1;
-            ft += ((ri * sRW) * sRW) * c1;
-            ft += ((ri * sRV) * sRW) * c2;
+            fv += (bz * sRU) * k.OBETA;
+            fw -= (by * sRU) * k.OBETA;
+            ft += ((ri * sRV) * sRV) * k.c1;
+            ft += ((ri * sRW) * sRW) * k.c1;
+            ft += ((ri * sRV) * sRW) * k.c2;
             ww2 -= w * sRV;
             ww3 -= v * sRW;
             sRV = d2z(BY, i, sz, z, c);
             if (z == zl)
-                sRV = (-3.0f * BY[i] + 4.0f * BY[i + sz] - BY[i + 2 * sz]) * c.hz * c.d2zzdz2[zl] +
-                      (2.0f * BY[i] - 5.0f * BY[i + sz] + 4.0f * BY[i + 2 * sz] - BY[i + 3 * sz]) * c.h2z * c.dzzdz[zl] *
+                sRV = (-3.0f * BY[i] + 4.0f * BY[i + sz] - BY[i + 2 * sz]) * k.hz * c.d2zzdz2[zl] +
+                      (2.0f * BY[i] - 5.0f * BY[i + sz] + 4.0f * BY[i + 2 * sz] - BY[i + 3 * sz]) * k.h2z * c.dzzdz[zl] *
                           c.dzzdz[zl];
             if (z == zr - 1)
-                sRV = (3.0f * BY[i] - 4.0f * BY[i - sz] + BY[i - 2 * sz]) * c.hz * c.d2zzdz2[zr - 1] +
-                      (2.0f * BY[i] - 5.0f * BY[i - sz] + 4.0f * BY[i - 2 * sz] - BY[i - 3 * sz]) * c.h2z *
+                sRV = (3.0f * BY[i] - 4.0f * BY[i - sz] + BY[i - 2 * sz]) * k.hz * c.d2zzdz2[zr - 1] +
+                      (2.0f * BY[i] - 5.0f * BY[i - sz] + 4.0f * BY[i - 2 * sz] - BY[i - 3 * sz]) * k.h2z *
                           c.dzzdz[zr - 1] * c.dzzdz[zr - 1];
             sRW = d2y(BZ, i, sy, y, c);
-            ww2 += sRV * c.ORM;
-            ww3 += sRW * c.ORM;
+            ww2 += sRV * k.ORM;
+            ww3 += sRW * k.ORM;
             sRW = d1z(BZ, i, sz, z, c);
             ww3 -= w * sRW;
             sRW = d2z(BZ, i, sz, z, c);
-            ww3 += sRW * c.ORM;
-            F.p[F_WW1][i] = ww1;
-            F.p[F_WW2][i] = ww2;
-            F.p[F_WW3][i] = ww3;
+            ww3 += sRW * k.ORM;
+            F.p[F_WW1][i] = ww1.v;
+            F.p[F_WW2][i] = ww2.v;
+            F.p[F_WW3][i] = ww3.v;
         }
-        F.p[F_FU][i] = fu;
-        F.p[F_FV][i] = fv;
-        F.p[F_FW][i] = fw;
-        F.p[F_FR][i] = fr;
-        F.p[F_FT][i] = ft;
+        F.p[F_FU][i] = fu.v;
+        F.p[F_FV][i] = fv.v;
+        F.p[F_FW][i] = fw.v;
+        F.p[F_FR][i] = fr.v;
+        F.p[F_FT][i] = ft.v;
     }
 }
 
@@ -1024,7 +1092,7 @@ template <class SW>
 void launch_flux(const Grid& g, const Consts& c, Fields8 U, Fields8 F, double* P, double* UU, double* VV, double* WW,
                  cudaStream_t st) {
     const long long ncell = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-    k_flux<SW><<<grid_for(ncell, 128, 152 * 64), 128, 0, st>>>(g, c, U, F, P, UU, VV, WW);
+    k_flux<SW><<<grid_for(ncell, kFluxThreads, 152 * 64), kFluxThreads, 0, st>>>(g, c, flux_scalars(c), U, F, P, UU, VV, WW);
 }
 
 template <class SW>
