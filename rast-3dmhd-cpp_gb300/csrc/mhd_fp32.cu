@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(T::kThreads, kResident) k_substage32(Fused32Ar
     const int ze = 1 + (int)((long long)nPz * (blockIdx.z + 1) / gridDim.z);
     const int nbx = (a.g.nx - 2 + kTX - 1) / kTX;
     substage32_tile<SW, T, EXTRA>(a, blockIdx.x % nbx, blockIdx.x / nbx, zb, ze, smem32);
+    launch_next();
 }
 
 // ragged batch: persistent CTAs take (instance, tile x, tile y, z range) items
@@ -66,6 +67,8 @@ __global__ void __launch_bounds__(BatchTile::kThreads, kResident)
 
 template <class SW>
 __global__ void k_bcon_ghost32(Fused32Args a, int wall0, int nwalls) {
+    wait_previous();
+    launch_next();
     const int nPx = a.g.nx - 2, nPy = a.g.ny - 2;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nwalls * nPx * nPy) return;
@@ -126,21 +129,21 @@ int fused32_walls(int planes, int chunks) {
            (planes - chunk_begin(planes, chunks - 1, chunks) >= kWallPlanes ? 2 : 0);
 }
 
-// Microseconds per launch of n CTAs: tiles of ty rows, c z ranges.  While all are
-// resident, the planes of a CTA (0.8 more around a range) follow one another, L
-// each, and share their SM's issue slots with the other CTAs, q each; with more
-// CTAs than that, in waves that overlap in part, b per plane.  Last, a separate BCON
-// launch where a range at a wall is too short for it.  Fitted to launches with lMag
-// on 16 grids of 32^3 .. 512x384x96 cells, 1 .. 64 ranges and both tiles: what it
-// chooses is within 5 % of the fastest on each, 1 % on average.
+// Microseconds (less a constant) per launch of n CTAs: tiles of ty rows, c z ranges.
+// While all are resident, the planes of a CTA (0.4 more around a range) follow one
+// another, L each, and share their SM's issue slots with the other CTAs, q each;
+// with more CTAs than that, in waves that overlap in part, b per plane.  Last, a
+// separate BCON launch where a range at a wall is too short for it.  Fitted to
+// launches with lMag on 16 grids of 32^3 .. 512x384x96 cells, 1 .. 64 ranges and
+// both tiles: on those grids the split that it chooses is within 1 % of the fastest.
 double cost32(int ty, long long n, int sms, int planes, int c) {
-    const double L = ty == 4 ? 1.6 : 2.0, q = ty == 4 ? 0.7 : 0.75, b = ty == 4 ? 4.3 : 4.7;
-    const double start = ty == 4 ? 15.0 : 19.0, f = ty == 4 ? 0.6 : 0.5;
+    const double L = 2.1, q = ty == 4 ? 0.47 : 0.65, b = ty == 4 ? 4.27 : 4.73;
+    const double start = ty == 4 ? 0.0 : 1.7, more = ty == 4 ? 6.4 : 7.0, f = ty == 4 ? 0.85 : 0.63;
     const long long wave = (long long)kResident * sms, per_sm = (n + sms - 1) / sms;
-    const double most = (planes + c - 1) / c + 0.8, avg = (double)planes / c + 0.8;
+    const double most = (planes + c - 1) / c + 0.4, avg = (double)planes / c + 0.4;
     const double waves = f * (double)n / wave + (1.0 - f) * (double)((n + wave - 1) / wave);
-    const double t = n <= wave ? 8.0 + L * most + q * per_sm * avg : start + b * waves * avg;
-    return fused32_walls(planes, c) == 3 ? t : t + 4.1;
+    const double t = start + (n <= wave ? L * most + q * per_sm * avg : more + b * waves * avg);
+    return fused32_walls(planes, c) == 3 ? t : t + 3.1;
 }
 
 // Rows per tile and number of z ranges for one instance of nx x ny interior columns.
@@ -179,8 +182,7 @@ int launch32_t(const Fused32Args& a, dim3 grid, cudaStream_t st) {
     static const cudaError_t set =
         cudaFuncSetAttribute(k_substage32<SW, T, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (set != cudaSuccess) return (int)set;
-    k_substage32<SW, T, EXTRA><<<grid, T::kThreads, smem, st>>>(a);
-    return (int)cudaGetLastError();
+    return launch_overlapped(k_substage32<SW, T, EXTRA>, grid, T::kThreads, smem, st, a);
 }
 
 template <class SW>
@@ -201,8 +203,7 @@ void launch32(const Fused32Args& args, cudaStream_t st, int* rc) {
     // the walls that the substage left
     const int first = a.walls & 1 ? 1 : 0, n = a.walls ? 1 : 2;
     const int cells = n * (a.g.nx - 2) * (a.g.ny - 2);
-    k_bcon_ghost32<SW><<<(cells + 127) / 128, 128, 0, st>>>(a, first, n);
-    *rc = (int)cudaGetLastError();
+    *rc = launch_overlapped(k_bcon_ghost32<SW>, (cells + 127) / 128, 128, 0, st, a, first, n);
 }
 
 template <class SW>

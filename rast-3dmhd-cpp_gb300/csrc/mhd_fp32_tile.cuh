@@ -294,13 +294,9 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
     };
     auto row = [&](int z) { return zrow + (z & (kZRing - 1)) * ZF_N; };
 
-    // the first three planes, each into its own slot, where it is derived
     float *Pm = ring + (size_t)((zb - 1) % 3) * kSlot, *P0 = ring + (size_t)(zb % 3) * kSlot,
           *Pp = ring + (size_t)((zb + 1) % 3) * kSlot;
-    copy_plane(Pm, zb - 1);
-    copy_plane(P0, zb);
-    copy_plane(Pp, zb + 1);
-    // coefficients: rows zb - 1 .. zb + 2, columns, scalars
+    // coefficients: rows zb - 1 .. zb + 2, columns, scalars (no kernel writes them)
     for (int z = zb - 1; z <= zb + 2 && z <= ze; z++) put_row(z);
     for (int k = tid; k < kCoef * kTX; k += kThreads) xtab[k] = a.k.xf[k / kTX][min(x0 + k % kTX, g.nx - 1)];
     for (int k = tid; k < kCoef * kTY; k += kThreads) ytab[k] = a.k.yf[k / kTY][min(y0 + k % kTY, g.ny - 1)];
@@ -322,6 +318,11 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
         }
         sc[tid] = (float)v;
     }
+    // the first three planes, each into its own slot, where it is derived
+    wait_previous();
+    copy_plane(Pm, zb - 1);
+    copy_plane(P0, zb);
+    copy_plane(Pp, zb + 1);
     const int ym = g.ny - 1;
     const float cx = (float)a.k.cx1[min(x, g.nx - 1)], cy = (float)a.k.cy1[min(y, ym)];
     const float ncx = -cx, ncy = -cy;

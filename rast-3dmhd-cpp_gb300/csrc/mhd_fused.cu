@@ -40,10 +40,13 @@ __global__ void __launch_bounds__(DefaultTile::kThreads, kMinBlocks) k_substage(
     const int zb = lo + (int)((long long)nz * blockIdx.z / gridDim.z);
     const int ze = lo + (int)((long long)nz * (blockIdx.z + 1) / gridDim.z);
     substage_tile<SW, DefaultTile, UXY, kExtra, ISO>(a, blockIdx.x, blockIdx.y, zb, ze, ring);
+    launch_next();
 }
 
 template <class SW>
 __global__ void k_bcon_ghost(Grid g, Consts c, Fields8 U, double timt, int wall0, int nwalls) {
+    wait_previous();
+    launch_next();
     const int nPx = g.nx - 2, nPy = g.ny - 2;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nwalls * nPx * nPy) return;
@@ -64,17 +67,18 @@ int fused_walls(const FusedArgs& a, int lo, int planes, int chunks) {
 
 // Number of z ranges per column.  In units of the time the SM's one FP64 unit
 // takes for a plane of a tile (6.2 us with lMag), a launch of n CTAs with P
-// planes each lasts, measured at 32^3 .. 256x256x128 for 1 .. 64 ranges:
-//   n <= 152 (one per SM)          1.7 + 1.24 P   one CTA alone does not keep the unit busy
-//   n <= 304                       1.7 + 2.13 P
-//   n <= 456 (all resident)        1.7 + 3.05 P
-//   more                           5.0 + ceil(n / 456) (0.55 + 2.83 P)
+// planes each lasts, measured at 16^3 .. 300x256x40 for 1 .. 64 ranges:
+//   n <= 152 (one per SM)          1.5 + 1.24 P   one CTA alone does not keep the unit busy
+//   n <= 304                       1.5 + 2.1 P
+//   n <= 456 (all resident)        1.5 + 2.95 P
+//   more                           1.0 + ceil(n / 456) (1.4 + 2.95 P)
 // with the constants for the planes around a range and its start-up; the last
 // wave counts in full because its CTAs are not spread evenly over the SMs.  A
-// range too short for BCON at the walls adds a launch (0.8).  Against at most
-// eight ranges of four planes: a step at 32x32x32 138 -> 87 us (32 ranges of
-// one plane), 97x45x61 (no field) 344 -> 272 us, 128x128x64 1146 -> 1094 us
-// (BCON inside the launch included).
+// range too short for BCON at the walls adds a launch (0.6).  The choice is within
+// 2 % of the fastest on those 19 grids.  Against at most eight ranges of four
+// planes, us per step, launches not overlapped: 32x32x32 138 -> 87 (32 ranges of
+// one plane), 97x45x61 (no field) 344 -> 272, 128x128x64 1146 -> 1094 (BCON inside
+// the launch included).
 int choose_chunks(const FusedArgs& a, long long tiles, int sms, int lo, int planes) {
     int best = 1;
     double best_cost = 1e300;
@@ -88,11 +92,11 @@ int choose_chunks(const FusedArgs& a, long long tiles, int sms, int lo, int plan
     for (int c = 1; c <= planes; c++) {
         const long long n = tiles * c;
         const double most = (planes + c - 1) / c, avg = (double)planes / c;
-        double cost = n <= sms       ? 1.7 + 1.24 * most
-                      : n <= 2 * sms ? 1.7 + 2.13 * most
-                      : n <= wave    ? 1.7 + 3.05 * most
-                                     : 5.0 + (double)((n + wave - 1) / wave) * (0.55 + 2.83 * avg);
-        if (fused_walls(a, lo, planes, c) != need) cost += 0.8;
+        double cost = n <= sms       ? 1.5 + 1.24 * most
+                      : n <= 2 * sms ? 1.5 + 2.1 * most
+                      : n <= wave    ? 1.5 + 2.95 * most
+                                     : 1.0 + (double)((n + wave - 1) / wave) * (1.4 + 2.95 * avg);
+        if (fused_walls(a, lo, planes, c) != need) cost += 0.6;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = c;
@@ -119,8 +123,7 @@ int launch_t(const FusedArgs& a, int chunks, cudaStream_t st) {
         cudaFuncSetAttribute(k_substage<SW, UXY, ISO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (set != cudaSuccess) return (int)set;
     const int nbx = (a.g.nx - 2 + T::kTX - 1) / T::kTX, nby = (a.g.ny - 2 + T::kTY - 1) / T::kTY;
-    k_substage<SW, UXY, ISO><<<dim3(nbx, nby, chunks), T::kThreads, smem, st>>>(a);
-    return (int)cudaGetLastError();
+    return launch_overlapped(k_substage<SW, UXY, ISO>, dim3(nbx, nby, chunks), T::kThreads, smem, st, a);
 }
 
 template <class SW>
@@ -131,9 +134,9 @@ void launch_substage(const FusedArgs& a, int chunks, cudaStream_t st, int* rc) {
 }
 
 template <class SW>
-void launch_bcon_ghost(const FusedArgs& a, int wall0, int nwalls, cudaStream_t st) {
+void launch_bcon_ghost(const FusedArgs& a, int wall0, int nwalls, cudaStream_t st, int* rc) {
     const int n = nwalls * (a.g.nx - 2) * (a.g.ny - 2);
-    k_bcon_ghost<SW><<<(n + 127) / 128, 128, 0, st>>>(a.g, a.c, a.Uo, a.timt, wall0, nwalls);
+    *rc = launch_overlapped(k_bcon_ghost<SW>, (n + 127) / 128, 128, 0, st, a.g, a.c, a.Uo, a.timt, wall0, nwalls);
 }
 
 }  // namespace
@@ -158,8 +161,8 @@ int fused_substage(unsigned sw, const FusedArgs& args, cudaStream_t st) {
     if (rc) return rc;
     // the walls that the substage left
     const bool first = lo == 1 && !(a.walls & 1), last = lo + planes == a.g.nz - 1 && !(a.walls & 2);
-    if (first || last) MHD_DISPATCH_SW(sw, launch_bcon_ghost, a, first ? 0 : 1, (first ? 1 : 0) + (last ? 1 : 0), st);
-    return (int)cudaGetLastError();
+    if (first || last) MHD_DISPATCH_SW(sw, launch_bcon_ghost, a, first ? 0 : 1, (first ? 1 : 0) + (last ? 1 : 0), st, &rc);
+    return rc;
 }
 #endif
 

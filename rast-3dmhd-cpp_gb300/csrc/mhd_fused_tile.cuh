@@ -251,14 +251,15 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
            *Pp = ring + (size_t)((zb + 1) % 3) * kRing;
     double *Om = own + (size_t)((zb - 1) % 3) * kOwn, *O0 = own + (size_t)(zb % 3) * kOwn,
            *Op = own + (size_t)((zb + 1) % 3) * kOwn;
-    // the first three planes, each into its own slot, where it is derived; then
-    // the scalars and the first two coefficient rows
-    copy_plane(Pm, zb - 1);
-    copy_plane(P0, zb);
-    copy_plane(Pp, zb + 1);
+    // the scalars and the first two coefficient rows (no kernel writes them); then
+    // the first three planes, each into its own slot, where it is derived
     if (tid < SC_N) sc[tid] = K.sc[UXY ? 1 : 0][tid];
     for (int k = tid; k < 2 * ZR_N; k += kThreads)
         zrow[((zb + k / ZR_N) & (kZRing - 1)) * ZR_N + k % ZR_N] = zt[(size_t)(zb + k / ZR_N) * ZR_N + k % ZR_N];
+    wait_previous();
+    copy_plane(Pm, zb - 1);
+    copy_plane(P0, zb);
+    copy_plane(Pp, zb + 1);
 
     __syncthreads();
     const double one = sc[SC_ONE], nzero = sc[SC_NZ];

@@ -137,6 +137,7 @@ __global__ void k_prep(Grid g, Consts c, Fields8 U, double* FW, double* P, doubl
         VV[i] = U.p[S_RV][i] * ri;
         WW[i] = U.p[S_RW][i] * ri;
     }
+    launch_next();
 }
 
 // As k_prep, but 1/rho goes to separate scratch and RO is left as it was.
@@ -157,6 +158,7 @@ __global__ void k_prep_ext(Grid g, Consts c, Fields8 U, double* RI, double* FW, 
         VV[i] = U.p[S_RV][i] * ri;
         WW[i] = U.p[S_RW][i] * ri;
     }
+    launch_next();
 }
 
 // Bound by the FP64 unit: 603 instructions per cell with lMag, none of which the
@@ -172,6 +174,7 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux(Grid g, Consts c, FluxSca
     if (threadIdx.x < sizeof(FluxScalars) / sizeof(double))
         reinterpret_cast<double*>(&s_flux)[threadIdx.x] = reinterpret_cast<const double*>(&scalars)[threadIdx.x];
     __syncthreads();
+    wait_previous();
     const FluxScalars& k = s_flux;
     const Field P{P_}, UU{U_}, VV{V_}, WW{W_};
     const int nPx = g.nx - 2, nPy = g.ny - 2, nPz = g.nz - 2;
@@ -852,12 +855,14 @@ __device__ __forceinline__ void cfl_load(const FA& U, long long row, int x, int 
 }
 
 // Seeds of the filter: the smallest a0 estimate and the largest mc estimate
-// (momenta not all zero) over every kCflSeedStride-th row, as ordered integer
-// keys (0 = nothing seen).  Any estimate that some certified cell attains is a
-// valid filter base, so the row kernel may start from these.
+// (momenta not all zero) over every kCflSeedStride-th row, per block in
+// seeds[block] (infinity, 0: nothing seen).  Any estimate that some certified cell
+// attains is a valid filter base, so the row kernel may start from these.  Also
+// resets the row kernel's count of finished blocks.
 constexpr int kCflSeedStride = 16;
 template <bool MAG, class FA>
-__global__ void k_cfl_seed(Grid g, Consts c, FA U, unsigned* seed) {
+__global__ void k_cfl_seed(Grid g, Consts c, FA U, float2* seeds, unsigned* done) {
+    wait_previous();
     const int nPx = g.nx - 2, nPy = g.ny - 2, nPz = g.nz - 2;
     const long long nall = (long long)nPy * nPz;
     const long long nrows = (nall + kCflSeedStride - 1) / kCflSeedStride;
@@ -898,11 +903,18 @@ __global__ void k_cfl_seed(Grid g, Consts c, FA U, unsigned* seed) {
         best_a = fminf(best_a, __shfl_xor_sync(0xffffffffu, best_a, o));
         best_m = fmaxf(best_m, __shfl_xor_sync(0xffffffffu, best_m, o));
     }
-    if (lane == 0) {
-        // positive floats order like their bit patterns
-        if (best_a < INFINITY) atomicMax(&seed[0], 0x7f800000u - __float_as_uint(best_a));
-        if (best_m > 0.0f) atomicMax(&seed[1], __float_as_uint(best_m));
+    __shared__ float2 s[8];
+    if (lane == 0) s[threadIdx.x / 32] = make_float2(best_a, best_m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; k++) {
+            best_a = fminf(best_a, s[k].x);
+            best_m = fmaxf(best_m, s[k].y);
+        }
+        seeds[blockIdx.x] = make_float2(best_a, best_m);
+        if (blockIdx.x == 0) *done = 0u;
     }
+    launch_next();
 }
 
 constexpr int kCflK = 8;                         // cells per lane in one pass over a row
@@ -936,8 +948,8 @@ constexpr float kCflTau = 1.52587890625e-05f;    // 2^-16: filter margin, > 2x t
 // bit; after the first passes only new near-extremes are evaluated.  Rows with varying DD, and launches whose constants break the
 // monotonicity (non-positive factors), evaluate every cell exactly.
 template <bool MAG, class FA>
-__global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c, FA U, unsigned* seed, double* part,
-                                                             CflEnd end) {
+__global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c, FA U, const float2* seeds, int nseeds,
+                                                             unsigned* done, double* part, CflEnd end) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nPx = g.nx - 2, nPy = g.ny - 2, nPz = g.nz - 2;
     const long long nrows = (long long)nPy * nPz;
@@ -945,8 +957,19 @@ __global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c
     const float gam_f = (float)c.GAMMA, obeta_f = (float)c.OBETA;
     double um = 0.0f, w0 = 1e99, w1 = 1e99, w2 = 1e99, w3 = 1e99;
     // the best estimates so far (warp-uniform), starting from the seeds
-    float run_a = seed[0] ? __uint_as_float(0x7f800000u - seed[0]) : INFINITY;
-    float run_m = seed[1] ? __uint_as_float(seed[1]) : -INFINITY;
+    wait_previous();
+    float run_a = INFINITY, run_m = 0.0f;
+    for (int k = lane; k < nseeds; k += 32) {
+        const float2 q = seeds[k];
+        run_a = fminf(run_a, q.x);
+        run_m = fmaxf(run_m, q.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        run_a = fminf(run_a, __shfl_xor_sync(0xffffffffu, run_a, o));
+        run_m = fmaxf(run_m, __shfl_xor_sync(0xffffffffu, run_m, o));
+    }
+    if (!(run_m > 0.0f)) run_m = -INFINITY;
     const long long stride = (long long)gridDim.x * kCflWarps;
     for (long long rb = (long long)blockIdx.x * kCflWarps + wid; rb < nrows; rb += 32 * stride) {
         // lane j holds the j-th row of this batch of 32 and, once that row is
@@ -1042,7 +1065,8 @@ __global__ void __launch_bounds__(kCflWarps * 32, 3) k_cfl_rows(Grid g, Consts c
             }
         }
     }
-    finish_cfl(um, w0, w1, w2, w3, part, seed + 2, end);
+    finish_cfl(um, w0, w1, w2, w3, part, done, end);
+    launch_next();
 }
 
 // Launch the row reduction with one wave of resident blocks (each warp then
@@ -1065,21 +1089,20 @@ int launch_cfl_rows_t(bool mag, const Grid& g, const Consts& c, FA U, double* pa
     if (nb < 1) nb = 1;
     if (nb > w) nb = w;
     if (nb > max_blocks) nb = max_blocks;
-    // two seed words and the count of finished blocks after the largest partial block (5 x max_blocks doubles)
-    unsigned* seed = reinterpret_cast<unsigned*>(partials + 5 * (size_t)max_blocks);
-    cudaMemsetAsync(seed, 0, 3 * sizeof(unsigned), st);
     const long long srows = (nrows + kCflSeedStride - 1) / kCflSeedStride;
     long long sb = (srows * 32 + 255) / 256;
     if (sb > w) sb = w;
+    if (sb > max_blocks) sb = max_blocks;
     if (sb < 1) sb = 1;
-    if (mag) {
-        k_cfl_seed<true, FA><<<(int)sb, 256, 0, st>>>(g, c, U, seed);
-        k_cfl_rows<true, FA><<<(int)nb, kCflWarps * 32, 0, st>>>(g, c, U, seed, partials, end);
-    } else {
-        k_cfl_seed<false, FA><<<(int)sb, 256, 0, st>>>(g, c, U, seed);
-        k_cfl_rows<false, FA><<<(int)nb, kCflWarps * 32, 0, st>>>(g, c, U, seed, partials, end);
-    }
-    return (int)cudaGetLastError();
+    // the seeds and the count of finished blocks after the largest partial block (the
+    // scratch holds 8 x max_blocks doubles, the partials 5 x max_blocks)
+    float2* seeds = reinterpret_cast<float2*>(partials + 5 * (size_t)max_blocks);
+    unsigned* done = reinterpret_cast<unsigned*>(seeds + max_blocks);
+    const auto seed = mag ? k_cfl_seed<true, FA> : k_cfl_seed<false, FA>;
+    const auto rows = mag ? k_cfl_rows<true, FA> : k_cfl_rows<false, FA>;
+    const int e = launch_overlapped(seed, (int)sb, 256, 0, st, g, c, U, seeds, done);
+    return e ? e : launch_overlapped(rows, (int)nb, kCflWarps * 32, 0, st, g, c, U, (const float2*)seeds, (int)sb, done,
+                                     partials, end);
 }
 int grid_for(long long n, int threads, int cap) {
     long long b = (n + threads - 1) / threads;
@@ -1090,9 +1113,10 @@ int grid_for(long long n, int threads, int cap) {
 
 template <class SW>
 void launch_flux(const Grid& g, const Consts& c, Fields8 U, Fields8 F, double* P, double* UU, double* VV, double* WW,
-                 cudaStream_t st) {
+                 cudaStream_t st, int* rc) {
     const long long ncell = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-    k_flux<SW><<<grid_for(ncell, kFluxThreads, 152 * 64), kFluxThreads, 0, st>>>(g, c, flux_scalars(c), U, F, P, UU, VV, WW);
+    *rc = launch_overlapped(k_flux<SW>, grid_for(ncell, kFluxThreads, 152 * 64), kFluxThreads, 0, st, g, c, flux_scalars(c), U,
+                            F, (const double*)P, (const double*)UU, (const double*)VV, (const double*)WW);
 }
 
 template <class SW>
@@ -1107,8 +1131,9 @@ int parity_fluxes(unsigned sw, const Grid& g, const Consts& c, Fields8 U, Fields
                   double* VV, double* WW, cudaStream_t st) {
     const long long n = (long long)g.nx * g.ny * g.nz;
     k_prep<<<grid_for(n, 256, 152 * 32), 256, 0, st>>>(g, c, U, F.p[F_FW], P, UU, VV, WW);
-    MHD_DISPATCH_SW(sw, launch_flux, g, c, U, F, P, UU, VV, WW, st);
-    return (int)cudaGetLastError();
+    int rc = (int)cudaGetLastError();
+    if (!rc) MHD_DISPATCH_SW(sw, launch_flux, g, c, U, F, P, UU, VV, WW, st, &rc);
+    return rc;
 }
 
 int parity_fluxes_ext(unsigned sw, const Grid& g, const Consts& c, Fields8 U, Fields8 F, double* RI, double* P,
@@ -1117,8 +1142,9 @@ int parity_fluxes_ext(unsigned sw, const Grid& g, const Consts& c, Fields8 U, Fi
     k_prep_ext<<<grid_for(n, 256, 152 * 32), 256, 0, st>>>(g, c, U, RI, F.p[F_FW], P, UU, VV, WW);
     Fields8 V = U;
     V.p[S_RO] = RI;  // k_flux reads 1/rho through the RO slot
-    MHD_DISPATCH_SW(sw, launch_flux, g, c, V, F, P, UU, VV, WW, st);
-    return (int)cudaGetLastError();
+    int rc = (int)cudaGetLastError();
+    if (!rc) MHD_DISPATCH_SW(sw, launch_flux, g, c, V, F, P, UU, VV, WW, st, &rc);
+    return rc;
 }
 
 int parity_rk(int kind, int nf, const Grid& g, Fields8 U, Fields8 Z, Fields8 F, double coef, cudaStream_t st) {

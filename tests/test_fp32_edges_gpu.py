@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 SIZES = [(31, 7, 4), (32, 8, 5), (33, 9, 6), (2, 2, 4), (64, 17, 7), (40, 25, 33),
          # large enough for tiles of 5 rows: remainders 1, 4, 0
-         (161, 101, 6), (97, 79, 6), (193, 50, 6)]
+         (97, 201, 9), (97, 224, 9), (161, 25, 20)]
 
 
 @pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
