@@ -15,7 +15,9 @@ from mhd_gb300.sim import Batch, Simulation
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(15, 7, 4), (16, 8, 5), (17, 9, 6), (31, 8, 7), (33, 17, 4), (2, 2, 4), (16, 2, 9), (18, 25, 33)]
+SIZES = [(15, 7, 4), (16, 8, 5), (17, 9, 6), (31, 8, 7), (33, 17, 4), (2, 2, 4), (16, 2, 9), (18, 25, 33),
+         # tiles of different numbers of z ranges (25 and 26, 30 and 31, 22 and 23)
+         (33, 41, 83), (65, 17, 104), (49, 33, 76)]
 
 
 @pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
