@@ -388,7 +388,8 @@ def run_ours(args, dist: Dist) -> None:
                 "serial_transfers": {"value": dist.world * case.cells / serial_s if e2e_steps else None,
                                      "ms_per_step": 1e3 * serial_s if e2e_steps else None,
                                      "path": "mhd_upload_state + mhd_step + mhd_download_state"}},
-        "gpu_launches": 6 * args.steps,
+        # one substage kernel each, BCON inside it (its z ranges at the walls hold 3 planes)
+        "gpu_launches": 3 * args.steps,
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                      "frac": achieved_gbs / hbm_peak, "traffic": traffic,
                      "traffic_note": "ncu dram read+write of one launch at 256x256x128, scaled per cell",
@@ -412,13 +413,13 @@ def run_ours(args, dist: Dist) -> None:
 
 
 # FP64-pipe instructions per interior cell per substage of the fused kernel,
-# keyed by (lMag, lRot, lShr): ncu's sm__inst_executed_pipe_fp64 share x the
-# 2/clk/SM pipe rate x elapsed cycles / cells, from the 256x256x128 capture in
+# keyed by (lMag, lRot, lShr): ncu's sm__inst_executed_pipe_fp64 (16 cycles each for
+# a warp) x 32 / cells, from the 256x256x128 capture in
 # profiles/k_substage_fp64_config1physics_256x256x128.md.
-FP64_INST_PER_CELL_SUBSTAGE: dict = {(True, True, True): 200.5}
+FP64_INST_PER_CELL_SUBSTAGE: dict = {(True, True, True): 167.4}
 # DRAM traffic over algorithmic bytes of one k_substage launch, measured by ncu
-# at 256x256x128 (2.274 GB / 2.282 GB); applied to the full-size average launch.
-TRAFFIC_OVER_ALGORITHMIC = {(True, True, True): 2.274 / 2.282}
+# at 256x256x128 (2.285 GB / 2.282 GB); applied to the full-size average launch.
+TRAFFIC_OVER_ALGORITHMIC = {(True, True, True): 2.285 / 2.282}
 
 
 # ---------------------------------------------------------------------------

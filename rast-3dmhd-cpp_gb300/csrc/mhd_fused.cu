@@ -1,9 +1,8 @@
 // mhd_fused.cu -- launches of the fused FP64 RK3 substage for one instance
 // (the per-tile work is in mhd_fused_tile.cuh) and of the wall kernel.
 //
-// The grid is (x tiles, y tiles, z chunks): splitting every column into z
-// ranges spreads a small grid over the SMs and turns the tail wave of a large
-// one into many short work units (choose_chunks).
+// Splitting every column into z ranges spreads a small grid over the SMs and turns
+// the tail wave of a large one into many short work units (choose_blocks).
 #include "mhd_fused_tile.cuh"
 
 #include <algorithm>

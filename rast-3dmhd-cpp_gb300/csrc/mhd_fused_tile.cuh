@@ -45,8 +45,9 @@
 // neighbour's products formed anew, plain sums and products, about 200 FP64
 // instructions per cell): a step at 512x512x256 (lMag, lRot, lShr) 68.9 ->
 // 55.4 ms, a batch of 24 instances 10.3 -> 8.3 ms per step, at 32x32x32 181 ->
-// 138 us; the FP64 unit is 90 % busy (184 instructions per cell and substage
-// at 256x256x128 with lMag).
+// 138 us (with the split and the overlapped launches of mhd_fused.cu 53.8 ms and
+// 72 us).  At 256x256x128 the FP64 unit is 94 % busy with lMag, lRot and lShr (167
+// instructions per cell and substage), 90 % with lMag alone (184).
 // Results agree with the reference to rounding (1e-12 of each field's
 // max-norm after a step, checked against the oracle).
 //

@@ -168,8 +168,9 @@ __global__ void k_prep_ext(Grid g, Consts c, Fields8 U, double* RI, double* FW, 
 // from the host.  64x64x32 with lMag: 172 us with DADD and DMUL, 151 now (the unit
 // is 88 % busy between launch and drain); blocks of 32, 64 and 128 threads are equal.
 template <class SW>
-__global__ void __launch_bounds__(kFluxThreads) k_flux(Grid g, Consts c, FluxScalars scalars, Fields8 U, Fields8 F, const double* __restrict__ P_,
-                       const double* __restrict__ U_, const double* __restrict__ V_, const double* __restrict__ W_) {
+__global__ void __launch_bounds__(kFluxThreads)
+    k_flux(Grid g, Consts c, FluxScalars scalars, Fields8 U, Fields8 F, const double* __restrict__ P_,
+           const double* __restrict__ U_, const double* __restrict__ V_, const double* __restrict__ W_) {
     static_assert(sizeof(FluxScalars) / sizeof(double) <= kFluxThreads);
     if (threadIdx.x < sizeof(FluxScalars) / sizeof(double))
         reinterpret_cast<double*>(&s_flux)[threadIdx.x] = reinterpret_cast<const double*>(&scalars)[threadIdx.x];
@@ -942,7 +943,7 @@ constexpr float kCflTau = 1.52587890625e-05f;    // 2^-16: filter margin, > 2x t
 //     bound of that, so it is always evaluated exactly.
 // Bound by the latency of its loads: a lane loads 4 cells (FP64: 2) before it
 // uses the first (256x256x128 with lMag, whole reduction: FP32 storage 162 -> 106
-// us, FP64 222 -> 157).
+// us, FP64 222 -> 157; with overlapped launches and seeds per block 103 and 146).
 // The exact maximum of mc and minimum of a0 are therefore among the cells
 // evaluated exactly, and the result equals the cell-by-cell reduction bit for
 // bit; after the first passes only new near-extremes are evaluated.  Rows with varying DD, and launches whose constants break the

@@ -135,8 +135,8 @@ class Server:
         self.zrange = {"fp64": None, "fp32": None}
         self.balance = balance
         # nominal cell-RK3-updates/s of a batch per precision (the 64-instance batch, measured:
-        # 7.97e8 and 4.29e9)
-        self.rates = dict(rates or {"fp64": 8.0e8, "fp32": 4.3e9})
+        # 1.03e9 and 5.48e9)
+        self.rates = dict(rates or {"fp64": 1.03e9, "fp32": 5.5e9})
         self.progress = progress
         self.progress_s = float(progress_s)
         self.completed = 0
