@@ -26,7 +26,7 @@ using BatchTile = Tile<kBatch32TY>;
 // one instance: grid (tiles, x fastest; 1; z chunks)
 template <class SW, class T, bool EXTRA>
 __global__ void __launch_bounds__(T::kThreads, kResident) k_substage32(Fused32Args a) {
-    extern __shared__ float smem32[];
+    extern __shared__ double smem32[];
     const int nPz = a.g.nz - 2;
     const int zb = 1 + (int)((long long)nPz * blockIdx.z / gridDim.z);
     const int ze = 1 + (int)((long long)nPz * (blockIdx.z + 1) / gridDim.z);
@@ -41,7 +41,7 @@ template <class SW>
 __global__ void __launch_bounds__(BatchTile::kThreads, kResident)
     k_substage32_batch(const Fused32Args* __restrict__ args, const int4* __restrict__ items, int nitems, int* counter,
                        BatchCtl ctl) {
-    extern __shared__ float smem32[];
+    extern __shared__ double smem32[];
     constexpr int kArgWords = sizeof(Fused32Args) / sizeof(int);
     __shared__ __align__(16) int s_args[kArgWords];
     __shared__ int s_item;

@@ -210,17 +210,18 @@ __device__ __forceinline__ Point point_values(const float* row, float ru, float 
 }
 
 // One tile (bx, by) of one instance, interior z planes [zb, ze).  EXTRA: the
-// instantiation with the iTCon 2 plume heat sink and lRem.
+// instantiation with the iTCon 2 plume heat sink and lRem.  `smem` begins with
+// the RK coefficients, so the kernels declare it as doubles (8-byte aligned).
 template <class SW, class T, bool EXTRA = false>
-__device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, int by, int zb, int ze, float* smem) {
+__device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, int by, int zb, int ze, double* smem) {
     constexpr int kTY = T::kTY, kThreads = T::kThreads, kPlane = T::kPlane;
     constexpr int NQ = nqf<SW>(), NRAW = nraw<SW>();
     constexpr int kOwn = NQ * kPlane;
     constexpr int kSlot = NQ * kPlane + G_N * kThreads;  // a plane's arrays, then its own-column ones
     const Grid& g = a.g;
     const Consts& c = a.c;
-    double* rk = reinterpret_cast<double*>(smem);  // [R_N]
-    float* ring = smem + 2 * R_N;
+    double* rk = smem;                         // [R_N]
+    float* ring = reinterpret_cast<float*>(smem + R_N);
     float* qbuf = ring + 3 * kSlot;            // [parity][Q1, Q2][plane]
     float* stage = qbuf + 4 * kPlane;          // [nraw][plane]
     float* zrow = stage + NRAW * kPlane;       // [kZRing][ZF_N]
