@@ -167,10 +167,11 @@ __global__ void k_prep_ext(Grid g, Consts c, Fields8 U, double* RI, double* FW, 
 // rows that 32 does not divide is larger).  Constant products and OCV / REPR come
 // from the host.  64x64x32 with lMag: 172 us with DADD and DMUL, 151 now (the unit
 // is 88 % busy between launch and drain); blocks of 32, 64 and 128 threads are equal.
+// P_ .. W_ are not __restrict__: k_prep may still write them when this kernel starts.
 template <class SW>
 __global__ void __launch_bounds__(kFluxThreads)
-    k_flux(Grid g, Consts c, FluxScalars scalars, Fields8 U, Fields8 F, const double* __restrict__ P_,
-           const double* __restrict__ U_, const double* __restrict__ V_, const double* __restrict__ W_) {
+    k_flux(Grid g, Consts c, FluxScalars scalars, Fields8 U, Fields8 F, const double* P_, const double* U_,
+           const double* V_, const double* W_) {
     static_assert(sizeof(FluxScalars) / sizeof(double) <= kFluxThreads);
     if (threadIdx.x < sizeof(FluxScalars) / sizeof(double))
         reinterpret_cast<double*>(&s_flux)[threadIdx.x] = reinterpret_cast<const double*>(&scalars)[threadIdx.x];
