@@ -247,40 +247,6 @@ struct BatchCtl {
     int n;
 };
 
-// Check of a work item and of its instance's arguments before a kernel uses
-// them: an item that fails records its code in ctl.err and is skipped, so a
-// malformed work list shows up as an error status instead of a stray access.
-// Codes: 1 instance index, 2 grid sizes, 3 tile position, 4 z range, 5 a
-// field pointer is null.
-template <class A>
-__device__ __forceinline__ bool batch_item_ok(const BatchCtl& ctl, const A* args, int4 it, int tx, int ty, int nf) {
-    int code = 0;
-    if (it.x < 0 || it.x >= ctl.n) {
-        code = 1;
-    } else {
-        const A& a = args[it.x];
-        const int zb = it.w & 0xffff, ze = it.w >> 16;
-        if (a.g.nx < 3 || a.g.ny < 3 || a.g.nz < 6 || a.g.sy != a.g.nx || a.g.sz != (long long)a.g.nx * a.g.ny)
-            code = 2;
-        else if (it.y < 0 || it.z < 0 || 1 + it.y * tx > a.g.nx - 2 || 1 + it.z * ty > a.g.ny - 2)
-            code = 3;
-        else if (zb < 1 || ze > a.g.nz - 1 || zb >= ze)
-            code = 4;
-        else
-            for (int f = 0; f < nf; f++)
-                if (!a.U.p[f] || !a.Uo.p[f] || !a.Z.p[f]) code = 5;
-    }
-    if (code) {
-        if (atomicCAS(ctl.err, 0, code) == 0) {
-            ctl.err[1] = it.x;
-            ctl.err[2] = it.y | (it.z << 16);
-            ctl.err[3] = it.w;
-        }
-        return false;
-    }
-    return true;
-}
-
 // _uxy: uniform x/y grids (d2xxdx2 = d2yydy2 = 0); _gen: any grid.
 // Item w = first z plane | (end plane << 16).
 int fused_batch_substage_uxy(unsigned sw, int tile, const FusedArgs* args, const int4* items, int nitems, int* counter,
@@ -328,6 +294,46 @@ struct Fused32Args {
     double gam, zet;
     int walls;  // as FusedArgs
 };
+// Whether the arguments hold nf fields where the kernels look for them: the FP64
+// substage addresses field f at p[0] + f * fs.
+__host__ __device__ __forceinline__ bool fields_ok(const FusedArgs& a, int nf) {
+    bool ok = a.fs >= a.g.sz * a.g.nz;
+    auto placed = [&](const Fields8& q, int f) { return q.p[f] && q.p[f] == q.p[0] + f * a.fs; };
+    for (int f = 0; f < nf; f++) ok = ok && placed(a.U, f) && placed(a.Uo, f) && placed(a.Z, f);
+    return ok;
+}
+__host__ __device__ __forceinline__ bool fields_ok(const Fused32Args& a, int nf) {
+    bool ok = true;
+    for (int f = 0; f < nf; f++) ok = ok && a.U.p[f] && a.Uo.p[f] && a.Z.p[f];
+    return ok;
+}
+
+// Check of a work item and of its instance's arguments before a kernel uses
+// them: an item that fails records its code in ctl.err and is skipped, so a
+// malformed work list shows up as an error status instead of a stray access.
+// Codes: 0 valid, 1 instance index, 2 grid sizes, 3 tile position, 4 z range, 5 a
+// field is missing or not where the kernel looks for it.
+template <class A>
+__host__ __device__ __forceinline__ int batch_item_code(int n, const A* args, int4 it, int tx, int ty, int nf) {
+    if (it.x < 0 || it.x >= n) return 1;
+    const A& a = args[it.x];
+    const int zb = it.w & 0xffff, ze = it.w >> 16;
+    if (a.g.nx < 3 || a.g.ny < 3 || a.g.nz < 6 || a.g.sy != a.g.nx || a.g.sz != (long long)a.g.nx * a.g.ny) return 2;
+    if (it.y < 0 || it.z < 0 || 1 + it.y * tx > a.g.nx - 2 || 1 + it.z * ty > a.g.ny - 2) return 3;
+    if (zb < 1 || ze > a.g.nz - 1 || zb >= ze) return 4;
+    return fields_ok(a, nf) ? 0 : 5;
+}
+template <class A>
+__device__ __forceinline__ bool batch_item_ok(const BatchCtl& ctl, const A* args, int4 it, int tx, int ty, int nf) {
+    const int code = batch_item_code(ctl.n, args, it, tx, ty, nf);
+    if (code && atomicCAS(ctl.err, 0, code) == 0) {
+        ctl.err[1] = it.x;
+        ctl.err[2] = it.y | (it.z << 16);
+        ctl.err[3] = it.w;
+    }
+    return code == 0;
+}
+
 // One substage and BCON (a.walls is set here).
 int fused32_substage(unsigned sw, const Fused32Args& a, cudaStream_t st);
 int communicate32(int nf, const Grid& g, Fields8f U, cudaStream_t st);
