@@ -129,7 +129,7 @@ const char* mhd_status_string(int status);
 
 /* ---- state transfer (dump / restart, 3dmhdio.h:20-72) ----------------- */
 /* Copy one whole field (ghosts included) host <-> device.  A download
- * synchronises the context's stream. */
+ * synchronises the context's stream; one of the state keeps no device memory. */
 int mhd_upload(mhd_ctx* ctx, int field, const double* host);
 int mhd_download(mhd_ctx* ctx, int field, double* host);
 /* All nfields state fields (5 without lMag, else 8) from / to one

@@ -311,50 +311,61 @@ int upload32(mhd_ctx* ctx, int field, const double* host) {
     return MHD_OK;
 }
 
+// The z ghost planes of U32[1-cur], which no step writes, from U32[cur].
+int copy_zghosts32(mhd_ctx* ctx) {
+    const int e = zghosts32(ctx->g, ctx->U32[ctx->cur], ctx->U32[1 - ctx->cur], ctx->stream);
+    return e ? cuda_fail(ctx, (cudaError_t)e, "ghost plane copy") : MHD_OK;
+}
+
+int sync_zghosts32(mhd_ctx* ctx) {
+    if (ctx->ghosts_synced) return MHD_OK;
+    const int rc = copy_zghosts32(ctx);
+    if (!rc) ctx->ghosts_synced = true;
+    return rc;
+}
+
 // Fields [field, field + nf) of the state to the host, widened on the device in
 // pieces of kStage elements.  Widening on the host (a copy of each field into a
 // fresh buffer, then one thread's loop) took 67 ms for the eight fields of
-// 256x256x128; the copy alone takes 3.
+// 256x256x128; this takes 3.5.  The pieces stand in U32[1-cur], whose values no
+// step reads but for the z ghost planes, put back afterwards, so a download keeps
+// no device memory (a buffer for it was half as much again as a 32^3 instance
+// holds).  Before the first step there is no U32[1-cur]: then in a buffer that is
+// freed again, or without memory for one in the reduction scratch.
 constexpr size_t kStage = 2u << 20;  // 16 MB: a piece's copy takes far longer than its kernel
 
-int download32(mhd_ctx* ctx, int field, int nf, double* host) {
-    if (!ctx->d_stage) {
-        const size_t len = std::min(kStage, ctx->ncell * (size_t)ctx->nf);
-        if (cudaMalloc(&ctx->d_stage, len * sizeof(double)) == cudaSuccess) {
-            ctx->stage_len = len;
-            ctx->bytes += len * sizeof(double);
-        } else {
-            ctx->d_stage = nullptr;
-            cudaGetLastError();
-        }
-    }
-    // without memory for it: the reduction scratch, which this stream's work does not hold
-    double* const buf = ctx->d_stage ? ctx->d_stage : ctx->red;
-    const long long len = ctx->d_stage ? (long long)ctx->stage_len : 8LL * ctx->red_blocks;
-    const long long first = (long long)field * (long long)ctx->ncell, total = (long long)nf * (long long)ctx->ncell;
+int widen_to_host(mhd_ctx* ctx, double* buf, long long len, long long first, long long total, double* host) {
     for (long long at = 0; at < total; at += len) {
         const int n = (int)std::min(len, total - at);
         const int e = widen32(ctx->g, ctx->U32[ctx->cur], ctx->d_bg, ctx->d_bg + ctx->g.nz, first + at, n, buf, ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "widening launch");
         CK(cudaMemcpyAsync(host + at, buf, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     }
-    CK(cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
 }
 
-int sync_zghosts32(mhd_ctx* ctx) {
-    if (ctx->ghosts_synced) return MHD_OK;
-    const size_t plane = (size_t)ctx->g.sz * sizeof(float);
-    float* a = ctx->U32[ctx->cur];
-    float* b = ctx->U32[1 - ctx->cur];
-    const size_t last = (size_t)(ctx->g.nz - 1) * ctx->g.sz;
-    for (int f = 0; f < 8; f++) {
-        float* fa = a + (size_t)f * ctx->ncell;
-        float* fb = b + (size_t)f * ctx->ncell;
-        CK(cudaMemcpyAsync(fb, fa, plane, cudaMemcpyDeviceToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(fb + last, fa + last, plane, cudaMemcpyDeviceToDevice, ctx->stream));
+int download32(mhd_ctx* ctx, int field, int nf, double* host) {
+    const long long first = (long long)field * (long long)ctx->ncell, total = (long long)nf * (long long)ctx->ncell;
+    int rc;
+    if (float* other = ctx->U32[1 - ctx->cur]) {
+        rc = widen_to_host(ctx, reinterpret_cast<double*>(other), (long long)std::min(kStage, 4 * ctx->ncell), first, total, host);
+        if (!rc && ctx->ghosts_synced) rc = copy_zghosts32(ctx);
+    } else {
+        double* own = nullptr;
+        const long long len = std::min((long long)kStage, total);
+        if (cudaMalloc(&own, (size_t)len * sizeof(double)) != cudaSuccess) {
+            own = nullptr;
+            cudaGetLastError();
+        }
+        rc = own ? widen_to_host(ctx, own, len, first, total, host)
+                 : widen_to_host(ctx, ctx->red, 8LL * ctx->red_blocks, first, total, host);
+        if (own) {
+            cudaStreamSynchronize(ctx->stream);
+            cudaFree(own);
+        }
     }
-    ctx->ghosts_synced = true;
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
 }
 
@@ -809,7 +820,6 @@ int mhd_destroy(mhd_ctx* ctx) {
     cudaFree(ctx->U32[0]);
     cudaFree(ctx->U32[1]);
     cudaFree(ctx->FT64);
-    cudaFree(ctx->d_stage);
     cudaFree(ctx->d_bg);
     cudaFree(ctx->d_plume);
     cudaFree(ctx->d_lrem);

@@ -337,6 +337,8 @@ __device__ __forceinline__ bool batch_item_ok(const BatchCtl& ctl, const A* args
 // One substage and BCON (a.walls is set here).
 int fused32_substage(unsigned sw, const Fused32Args& a, cudaStream_t st);
 int communicate32(int nf, const Grid& g, Fields8f U, cudaStream_t st);
+// the z ghost planes of all eight fields of `from` into those of `to`
+int zghosts32(const Grid& g, const float* from, float* to, cudaStream_t st);
 // elements [first, first + n) of an FP32-storage state (fields one after another) as FP64 values in out
 int widen32(const Grid& g, const float* U, const double* bgR, const double* bgT, long long first, int n, double* out,
             cudaStream_t st);

@@ -42,8 +42,6 @@ struct mhd_ctx {
     bool fp32 = false;
     float* U32[2] = {nullptr, nullptr};
     double* FT64 = nullptr;     // persistent FT (lShr)
-    double* d_stage = nullptr;  // FP64 values on their way to the host (first download on)
-    size_t stage_len = 0;       // its length in elements
     double* d_bg = nullptr;     // rho0, T0, dzT0, d2zT0 (4 x nz), then the float table
     std::vector<double> h_bg;   // host copy of the four profiles
     std::vector<double> h_cz;   // cz1, cz2a, cz2b (3 x nz)

@@ -292,12 +292,28 @@ __global__ void k_widen32(Grid g, const float* U, const double* bgR, const doubl
     }
 }
 
+// planes 0 and nz - 1 of eight fields
+__global__ void k_zghosts32(Grid g, const float* from, float* to) {
+    const long long n = 16 * g.sz, stride = (long long)gridDim.x * blockDim.x;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += stride) {
+        const int k = (int)(t / g.sz);  // field and side
+        const long long i = ((long long)(k >> 1) * g.nz + (k & 1 ? g.nz - 1 : 0)) * g.sz + t % g.sz;
+        to[i] = from[i];
+    }
+}
+
 }  // namespace
 
 int widen32(const Grid& g, const float* U, const double* bgR, const double* bgT, long long first, int n, double* out,
             cudaStream_t st) {
     const int b = (n + 255) / 256;
     k_widen32<<<b < 152 * 16 ? b : 152 * 16, 256, 0, st>>>(g, U, bgR, bgT, first, n, out);
+    return (int)cudaGetLastError();
+}
+
+int zghosts32(const Grid& g, const float* from, float* to, cudaStream_t st) {
+    const long long b = (16 * g.sz + 255) / 256;
+    k_zghosts32<<<(int)(b < 152 * 8 ? b : 152 * 8), 256, 0, st>>>(g, from, to);
     return (int)cudaGetLastError();
 }
 
