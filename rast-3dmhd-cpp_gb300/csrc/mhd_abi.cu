@@ -599,9 +599,10 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     const double scales[4] = {ctx->k.ORE, ctx->k.ORE * ctx->k.C43, ctx->k.ORM, 1.0};
     for (int ax = 0; ax < 2; ax++) {
         side_off[ax] = h.size();
-        for (int k = 0; k < 4; k++)
-            for (int sg = 1; sg >= -1; sg -= 2)
-                for (int i = 0; i < ns[ax]; i++) h.push_back(scales[k] * (c2b(ax, i) + sg * c2a(ax, i)));
+        for (int k = 0; k < 4; k++) {
+            for (int i = 0; i < ns[ax]; i++) h.push_back(scales[k] * c2b(ax, i));
+            for (int i = 0; i < ns[ax]; i++) h.push_back(scales[k] * c2a(ax, i));
+        }
     }
     // the FP32 kernels' column coefficients, two floats per double
     size_t sidef_off[2];
@@ -642,8 +643,8 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
             };
             r[ZR_CZ] = cz / kap;
             for (int k = 0; k < 3; k++) {
-                r[ZR_SZ0 + 2 * k] = scales[k] * (zb + za) / kap;
-                r[ZR_SZ0 + 2 * k + 1] = scales[k] * (zb - za) / kap;
+                r[ZR_SZ0 + 2 * k] = u ? scales[k] * (zb + za) / kap : scales[k] * zb;
+                r[ZR_SZ0 + 2 * k + 1] = u ? scales[k] * (zb - za) / kap : scales[k] * za;
             }
             r[ZR_KZP] = u ? sT * (kz * (zb + za) + dkz * cz) : kz;
             r[ZR_KZM] = u ? sT * (kz * (zb - za) - dkz * cz) : dkz * cz;
@@ -657,8 +658,8 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
             r[ZR_SBW] = centre(2, 2, -1);
             r[ZR_KQZ] = c13ore * cz;
             r[ZR_OCZ] = ctx->k.OBETA * cz / kap;
-            r[ZR_TZP] = zb + za;
-            r[ZR_TZM] = zb - za;
+            r[ZR_TZP] = u ? zb + za : zb;
+            r[ZR_TZM] = u ? zb - za : za;
             r[ZR_STL] = 2.0 * (bx + by + zb);
             r[ZR_WD2] = ctx->k.ORM * za / kap;
             r[ZR_WD1] = ctx->k.ORM * zb / kap;

@@ -109,7 +109,8 @@ struct Fields8 {
 enum ZRow {
     ZR_CZ = 0,    // cz1 / kappa (cz1 = dzzdz*hz)
     ZR_SZ0,       // z second-derivative factors of the planes above and below, b + a and b - a
-                  // (a = d2zzdz2*hz, b = dzzdz^2*h2z), scaled by ORE, ORE*C43, ORM, over kappa: 6 entries
+                  // (a = d2zzdz2*hz, b = dzzdz^2*h2z), other grids b and a, scaled by ORE, ORE*C43, ORM,
+                  // over kappa: 6 entries
     ZR_KZP = ZR_SZ0 + 6,  // conduction: the factors of T(z+1) and T(z-1), kapz (b +- a) +- dkapz cz1, with
     ZR_KZM,               // kapz, dkapz = OCV/REPR * (RKAPA, DKAPA), times sT; other grids: kapz and dkapz cz1
     ZR_KX, ZR_KY,         // kapz cx2b, kapz cy2b (cx2b = duudu^2*h2u), times sT
@@ -117,7 +118,7 @@ enum ZRow {
     ZR_ST, ZR_SB, ZR_SBW, // T (kapz and sT included) and B, and 2 (sx + sy) of B for the wall planes
     ZR_KQZ,               // C13*ORE*cz1
     ZR_OCZ,               // OBETA*cz1 / kappa
-    ZR_TZP, ZR_TZM, ZR_STL,  // the unscaled Laplacian's b + a, b - a and centre coefficient (lRem; other grids)
+    ZR_TZP, ZR_TZM, ZR_STL,  // the unscaled Laplacian's b + a, b - a and centre coefficient (lRem); other grids b, a
     ZR_WD2, ZR_WD1,          // ORM a and ORM b over kappa: the one-sided d2B/dz2 on the walls
     ZR_N
 };
@@ -148,7 +149,7 @@ struct Coefs {
     // c2a = d2uudu2*hu, c2b = duudu^2*h2u
     const double *cx1, *cx2a, *cx2b;
     const double *cy1, *cy2a, *cy2b;
-    // per column (any grid): c2b + c2a and c2b - c2a, scaled by ORE, ORE*C43, ORM and unscaled
+    // per column (any grid): c2b and c2a, scaled by ORE, ORE*C43, ORM and unscaled
     const double *xt[8], *yt[8];
     // for the FP32 kernels: c2b and c2a as floats, scaled alike
     const float *xf[8], *yf[8];

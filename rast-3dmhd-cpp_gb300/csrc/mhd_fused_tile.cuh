@@ -407,17 +407,20 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
                 }
                 if constexpr (SW::lShr) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.FT + inx));
             }
-            // second-derivative coefficients of the planes / columns above (p) and
-            // below (m): scale k = 0 ORE, 1 ORE*C43, 2 ORM, 3 unscaled (T)
-            auto pxs = [&](int k) { return UXY ? sc[SC_SX0 + k] : K.xt[2 * k][xc]; };
-            auto mxs = [&](int k) { return UXY ? sc[SC_SX0 + k] : K.xt[2 * k + 1][xc]; };
-            auto pys = [&](int k) { return UXY ? sc[SC_SY0 + k] : K.yt[2 * k][yc]; };
-            auto mys = [&](int k) { return UXY ? sc[SC_SY0 + k] : K.yt[2 * k + 1][yc]; };
-            // ... and their sum, the coefficient of the centre (kx, ky, kz: scale per axis)
-            auto centre = [&](int kx, int ky, int kz, int row) {
-                if constexpr (UXY) return R[row];
-                else return (pxs(kx) + mxs(kx)) + (pys(ky) + mys(ky)) + (kz < 0 ? 0.0 : R[ZR_SZ0 + 2 * kz] + R[ZR_SZ0 + 2 * kz + 1]);
+            // uniform grids: second-derivative coefficients of both neighbours in x and y, scale
+            // k = 0 ORE, 1 ORE*C43, 2 ORM
+            auto sx = [&](int k) { return sc[SC_SX0 + k]; };
+            auto sy = [&](int k) { return sc[SC_SY0 + k]; };
+            // other grids: acc + b (p - 2 c + m) + a (p - m) along an axis.  Merged into
+            // factors b + a and b - a the first-derivative part would carry an error of
+            // eps b (stretched x and y, RE = RM = 2, 100 steps at 24x21x20: 1.7 times the
+            // error of BX and BY against 80-bit arithmetic).
+            auto d2 = [&](double b, double a_, double p, double m, double c0, double acc) {
+                return fma(a_, sub(p, m), fma(b, fma(-2.0, c0, add(p, m)), acc));
             };
+            auto lapx = [&](int q, int k, double acc) { return d2(K.xt[2 * k][xc], K.xt[2 * k + 1][xc], XP(q), XM(q), C0(q), acc); };
+            auto lapy = [&](int q, int k, double acc) { return d2(K.yt[2 * k][yc], K.yt[2 * k + 1][yc], YP(q), YM(q), C0(q), acc); };
+            auto lapz = [&](int q, int k, double acc) { return d2(R[ZR_SZ0 + 2 * k], R[ZR_SZ0 + 2 * k + 1], ZP(q), ZM(q), C0(q), acc); };
 
             const double rwp = Op[O_RW * kThreads + tid], rwm = Om[O_RW * kThreads + tid];
             const double u = C0(Q_U), v = C0(Q_V), w = C0(Q_W), tt = C0(Q_TT);
@@ -434,29 +437,40 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
             double fu = SX(sub(XM(Q_PX), XP(Q_PX)));
             double fv = SY(sub(YM(Q_PY), YP(Q_PY)));
             double fw = fma(cz, sub(Om[O_PZ * kThreads + tid], Op[O_PZ * kThreads + tid]), mul(sc[SC_GRAV], ro0));
-            {
-                const double ap = UXY ? sub(pxs(0), rup) : fma(-gcx, rup, pxs(0));
-                const double am = UXY ? add(mxs(0), rum) : fma(gcx, rum, mxs(0));
-                fu = fma(pxs(1), XP(Q_U), fma(mxs(1), XM(Q_U), fu));
-                fv = fma(ap, XP(Q_V), fma(am, XM(Q_V), fv));
-                fw = fma(ap, XP(Q_W), fma(am, XM(Q_W), fw));
+            if constexpr (UXY) {
+                {
+                    const double ap = sub(sx(0), rup), am = add(sx(0), rum);
+                    fu = fma(sx(1), XP(Q_U), fma(sx(1), XM(Q_U), fu));
+                    fv = fma(ap, XP(Q_V), fma(am, XM(Q_V), fv));
+                    fw = fma(ap, XP(Q_W), fma(am, XM(Q_W), fw));
+                }
+                {
+                    const double ap = ISO ? sub(sy(0), rvp) : fma(-gcy, rvp, sy(0));
+                    const double am = ISO ? add(sy(0), rvm) : fma(gcy, rvm, sy(0));
+                    fu = fma(ap, YP(Q_U), fma(am, YM(Q_U), fu));
+                    fv = fma(sy(1), YP(Q_V), fma(sy(1), YM(Q_V), fv));
+                    fw = fma(ap, YP(Q_W), fma(am, YM(Q_W), fw));
+                }
+                {
+                    const double ap = fma(-cz, rwp, R[ZR_SZ0]), am = fma(cz, rwm, R[ZR_SZ0 + 1]);
+                    fu = fma(ap, ZP(Q_U), fma(am, ZM(Q_U), fu));
+                    fv = fma(ap, ZP(Q_V), fma(am, ZM(Q_V), fv));
+                    fw = fma(R[ZR_SZ0 + 2], ZP(Q_W), fma(R[ZR_SZ0 + 3], ZM(Q_W), fw));
+                }
+                fu = fma(-R[ZR_SU], u, fu);
+                fv = fma(-R[ZR_SV], v, fv);
+                fw = fma(-R[ZR_SW], w, fw);
+            } else {
+                fu = fma(-gcy, fma(rvp, YP(Q_U), mul(-rvm, YM(Q_U))), fu);
+                fu = fma(-cz, fma(rwp, ZP(Q_U), mul(-rwm, ZM(Q_U))), fu);
+                fv = fma(-gcx, fma(rup, XP(Q_V), mul(-rum, XM(Q_V))), fv);
+                fv = fma(-cz, fma(rwp, ZP(Q_V), mul(-rwm, ZM(Q_V))), fv);
+                fw = fma(-gcx, fma(rup, XP(Q_W), mul(-rum, XM(Q_W))), fw);
+                fw = fma(-gcy, fma(rvp, YP(Q_W), mul(-rvm, YM(Q_W))), fw);
+                fu = lapz(Q_U, 0, lapy(Q_U, 0, lapx(Q_U, 1, fu)));
+                fv = lapz(Q_V, 0, lapy(Q_V, 1, lapx(Q_V, 0, fv)));
+                fw = lapz(Q_W, 1, lapy(Q_W, 0, lapx(Q_W, 0, fw)));
             }
-            {
-                const double ap = ISO ? sub(pys(0), rvp) : fma(-gcy, rvp, pys(0));
-                const double am = ISO ? add(mys(0), rvm) : fma(gcy, rvm, mys(0));
-                fu = fma(ap, YP(Q_U), fma(am, YM(Q_U), fu));
-                fv = fma(pys(1), YP(Q_V), fma(mys(1), YM(Q_V), fv));
-                fw = fma(ap, YP(Q_W), fma(am, YM(Q_W), fw));
-            }
-            {
-                const double ap = fma(-cz, rwp, R[ZR_SZ0]), am = fma(cz, rwm, R[ZR_SZ0 + 1]);
-                fu = fma(ap, ZP(Q_U), fma(am, ZM(Q_U), fu));
-                fv = fma(ap, ZP(Q_V), fma(am, ZM(Q_V), fv));
-                fw = fma(R[ZR_SZ0 + 2], ZP(Q_W), fma(R[ZR_SZ0 + 3], ZM(Q_W), fw));
-            }
-            fu = fma(-centre(1, 0, 0, ZR_SU), u, fu);
-            fv = fma(-centre(0, 1, 0, ZR_SV), v, fv);
-            fw = fma(-centre(0, 0, 1, ZR_SW), w, fw);
 
             // ---- viscous cross terms (3dmhdsub.h:486-487,517-518,531-532)
             {
@@ -484,16 +498,15 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
             }
             {
                 double lapT = 0.0;
-                if ((EXTRA && c.lrem && !SW::lShr) || !UXY) {
-                    lapT = mul(UXY ? sc[SC_TX] : pxs(3), XP(Q_TT));
-                    lapT = fma(UXY ? sc[SC_TX] : mxs(3), XM(Q_TT), lapT);
-                    lapT = fma(UXY ? sc[SC_TY] : pys(3), YP(Q_TT), lapT);
-                    lapT = fma(UXY ? sc[SC_TY] : mys(3), YM(Q_TT), lapT);
+                if constexpr (!UXY) {
+                    lapT = d2(R[ZR_TZP], R[ZR_TZM], ZP(Q_TT), ZM(Q_TT), tt, lapy(Q_TT, 3, lapx(Q_TT, 3, 0.0)));
+                } else if (EXTRA && c.lrem && !SW::lShr) {
+                    lapT = mul(sc[SC_TX], XP(Q_TT));
+                    lapT = fma(sc[SC_TX], XM(Q_TT), lapT);
+                    lapT = fma(sc[SC_TY], YP(Q_TT), lapT);
+                    lapT = fma(sc[SC_TY], YM(Q_TT), lapT);
                     lapT = fma(R[ZR_TZP], ZP(Q_TT), fma(R[ZR_TZM], ZM(Q_TT), lapT));
-                    double S;
-                    if constexpr (UXY) S = R[ZR_STL];
-                    else S = (pxs(3) + mxs(3)) + (pys(3) + mys(3)) + (R[ZR_TZP] + R[ZR_TZM]);
-                    lapT = fma(-S, tt, lapT);
+                    lapT = fma(-R[ZR_STL], tt, lapT);
                 }
                 if (EXTRA && c.lrem && !SW::lShr) {
                     // lRem: conduction of T - TTM(z) plus HRAD (3dmhdsub.h:297-313),
@@ -568,42 +581,58 @@ __device__ __forceinline__ void substage_tile(const FusedArgs& a, int bx, int by
                 w2 = fma(bx, vx, fma(bzc, dVz, mul(-by, add(ux, wzm))));
                 w3 = fma(bx, wx, fma(by, wy, mul(-bz, q3c)));
                 // advection and resistive Laplacians
-                {
-                    const double ap = UXY ? sub(pxs(2), u) : fma(-gcx, u, pxs(2));
-                    const double am = UXY ? add(mxs(2), u) : fma(gcx, u, mxs(2));
-                    w1 = fma(ap, XP(Q_BX), fma(am, XM(Q_BX), w1));
-                    w2 = fma(ap, XP(Q_BY), fma(am, XM(Q_BY), w2));
-                    w3 = fma(ap, XP(Q_BZ), fma(am, XM(Q_BZ), w3));
-                }
-                {
-                    const double ap = ISO ? sub(pys(2), v) : fma(-gcy, v, pys(2));
-                    const double am = ISO ? add(mys(2), v) : fma(gcy, v, mys(2));
-                    w1 = fma(ap, YP(Q_BX), fma(am, YM(Q_BX), w1));
-                    w2 = fma(ap, YP(Q_BY), fma(am, YM(Q_BY), w2));
-                    w3 = fma(ap, YP(Q_BZ), fma(am, YM(Q_BZ), w3));
-                }
-                {
+                if constexpr (UXY) {
+                    {
+                        const double ap = sub(sx(2), u);
+                        const double am = add(sx(2), u);
+                        w1 = fma(ap, XP(Q_BX), fma(am, XM(Q_BX), w1));
+                        w2 = fma(ap, XP(Q_BY), fma(am, XM(Q_BY), w2));
+                        w3 = fma(ap, XP(Q_BZ), fma(am, XM(Q_BZ), w3));
+                    }
+                    {
+                        const double ap = ISO ? sub(sy(2), v) : fma(-gcy, v, sy(2));
+                        const double am = ISO ? add(sy(2), v) : fma(gcy, v, sy(2));
+                        w1 = fma(ap, YP(Q_BX), fma(am, YM(Q_BX), w1));
+                        w2 = fma(ap, YP(Q_BY), fma(am, YM(Q_BY), w2));
+                        w3 = fma(ap, YP(Q_BZ), fma(am, YM(Q_BZ), w3));
+                    }
                     const double ap = sub(R[ZR_SZ0 + 4], czw), am = add(R[ZR_SZ0 + 5], czw);
                     w3 = fma(ap, ZP(Q_BZ), fma(am, ZM(Q_BZ), w3));
-                    w3 = fma(-centre(2, 2, 2, ZR_SB), bz, w3);
+                    w3 = fma(-R[ZR_SB], bz, w3);
                     if (!wall) {
-                        const double S = centre(2, 2, 2, ZR_SB);
+                        const double S = R[ZR_SB];
                         w1 = fma(ap, ZP(Q_BX), fma(am, ZM(Q_BX), fma(-S, bx, w1)));
                         w2 = fma(ap, ZP(Q_BY), fma(am, ZM(Q_BY), fma(-S, by, w2)));
-                    } else {
-                        // d2B/dz2 with the one-sided wall stencils (3dmhdsub.h:640-654,673-687)
-                        const double S = centre(2, 2, -1, ZR_SBW);
-                        const int s = (z == zl) ? 1 : -1;
-                        const long long j2 = i + 2 * s * g.sz, j3 = i + 3 * s * g.sz;
-                        const double d2 = R[ZR_WD2], d1 = R[ZR_WD1];
-                        const double X1 = (s > 0) ? ZP(Q_BX) : ZM(Q_BX), X2 = U0[S_BX * fs + j2], X3 = U0[S_BX * fs + j3];
-                        const double Y1 = (s > 0) ? ZP(Q_BY) : ZM(Q_BY), Y2 = U0[S_BY * fs + j2], Y3 = U0[S_BY * fs + j3];
-                        const double sg = (double)s;
+                    }
+                } else {
+                    const double cxu = mul(gcx, u), cyv = mul(gcy, v);
+                    auto advect = [&](int q, double acc) {
+                        acc = fma(-czw, sub(ZP(q), ZM(q)), acc);
+                        return fma(-cxu, sub(XP(q), XM(q)), fma(-cyv, sub(YP(q), YM(q)), acc));
+                    };
+                    w1 = lapy(Q_BX, 2, lapx(Q_BX, 2, advect(Q_BX, w1)));
+                    w2 = lapy(Q_BY, 2, lapx(Q_BY, 2, advect(Q_BY, w2)));
+                    w3 = lapz(Q_BZ, 2, lapy(Q_BZ, 2, lapx(Q_BZ, 2, advect(Q_BZ, w3))));
+                    if (!wall) {
+                        w1 = lapz(Q_BX, 2, w1);
+                        w2 = lapz(Q_BY, 2, w2);
+                    }
+                }
+                if (wall) {
+                    // d2B/dz2 with the one-sided wall stencils (3dmhdsub.h:640-654,673-687)
+                    const double S = R[ZR_SBW];
+                    const int s = (z == zl) ? 1 : -1;
+                    const long long j2 = i + 2 * s * g.sz, j3 = i + 3 * s * g.sz;
+                    const double a2 = R[ZR_WD2], b2 = R[ZR_WD1];
+                    const double X1 = (s > 0) ? ZP(Q_BX) : ZM(Q_BX), X2 = U0[S_BX * fs + j2], X3 = U0[S_BX * fs + j3];
+                    const double Y1 = (s > 0) ? ZP(Q_BY) : ZM(Q_BY), Y2 = U0[S_BY * fs + j2], Y3 = U0[S_BY * fs + j3];
+                    const double sg = (double)s;
+                    if constexpr (UXY) {
                         w1 = fma(-czw, ZP(Q_BX) - ZM(Q_BX), fma(-S, bx, w1));
                         w2 = fma(-czw, ZP(Q_BY) - ZM(Q_BY), fma(-S, by, w2));
-                        w1 += sg * (-3.0 * bx + 4.0 * X1 - X2) * d2 + (2.0 * bx - 5.0 * X1 + 4.0 * X2 - X3) * d1;
-                        w2 += sg * (-3.0 * by + 4.0 * Y1 - Y2) * d2 + (2.0 * by - 5.0 * Y1 + 4.0 * Y2 - Y3) * d1;
                     }
+                    w1 += sg * (-3.0 * bx + 4.0 * X1 - X2) * a2 + (2.0 * bx - 5.0 * X1 + 4.0 * X2 - X3) * b2;
+                    w2 += sg * (-3.0 * by + 4.0 * Y1 - Y2) * a2 + (2.0 * by - 5.0 * Y1 + 4.0 * Y2 - Y3) * b2;
                 }
                 // current density j' = OBETA j (in units of kappa): the Lorentz force is
                 // B x j' and the Ohmic heating proportional to |j'|^2
