@@ -85,8 +85,14 @@ struct Field {
     __device__ __forceinline__ D operator[](long long i) const { return p[i]; }
 };
 
-// (p - 2 c) + m; 2 c is exact
-__device__ __forceinline__ D second(D p, D c, D m) { return D(fma(s_flux.mtwo, c.v, p.v)) + m; }
+// (p - 2 c) + m.  2 c is exact unless it overflows; there c stands for it as an
+// infinity (integer operations, whose pipe idles here).
+__device__ __forceinline__ D second(D p, D c, D m) {
+    const unsigned hi = (unsigned)__double2hiint(c.v), sign = hi & 0x80000000u;
+    const bool overflows = (hi ^ sign) - 0x7fe00000u < 0x00100000u;  // 2^1023 <= |c| < infinity
+    const double cc = __hiloint2double((int)(overflows ? sign | 0x7ff00000u : hi), overflows ? 0 : __double2loint(c.v));
+    return D(fma(s_flux.mtwo, cc, p.v)) + m;
+}
 
 __device__ __forceinline__ D d1x(Field F, long long i, int x, const Consts& c) {
     return ((F[i + 1] - F[i - 1]) * c.dxxdx[x]) * s_flux.hx;
