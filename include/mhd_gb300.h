@@ -315,6 +315,10 @@ int mhd_static_lrem_profile(const mhd_params* p, const mhd_static_params* s, dou
  * kernels use against the hardware conversions, on n test patterns of seed;
  * *mismatches receives the number of differing results (0 expected). */
 int mhd_selftest_convert(long long n, unsigned long long seed, long long* mismatches);
+/* Self-check: the reciprocals of the fused substages against 1 / x, the FP32 one
+ * on every float and the FP64 one on n test patterns of seed; the number of
+ * results beyond their error bound (0 expected). */
+int mhd_selftest_recip(long long n, unsigned long long seed, long long* bad32, long long* bad64);
 
 /* ---- ragged batches ------------------------------------------------------ */
 /* n independent instances (fused-path contexts with one switch set and one

@@ -169,6 +169,20 @@ __device__ __forceinline__ void bcon32_cell(const Grid& g, const Consts& c, cons
     }
 }
 
+// 1/x: one Newton-Raphson step from the hardware estimate, which is good to one
+// unit in the last place: the error stays within 2^-24 + 2^-43 of the value (a
+// rounded quotient's is 2^-24).  Where x or the estimate is no normal number (|x|
+// below 2^-126 or above 2^126, infinity, NaN) the residual is 1 or no number: there
+// the estimate that knows subnormal numbers, alone (a division spills registers).
+__device__ __forceinline__ float recip32(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    const float e = fmaf(-x, r, 1.0f);
+    r = fmaf(r, e, r);
+    if (!(fabsf(e) < 0.5f)) asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // The derived quantities of a point: 1/rho, the velocities, and the
 // equation of state as the deviation dp = rho0 dT + drho T0 + drho dT of p from
 // the plane's rho0 T0.  rho0 and T0 come as float pairs hi + lo (about 48
@@ -176,7 +190,7 @@ __device__ __forceinline__ void bcon32_cell(const Grid& g, const Consts& c, cons
 // (two-sum), plus rl, and recover every product's rounding error by fma, so dp
 // keeps about one float rounding where its terms cancel (near pressure
 // balance; measured against 80-bit sums: <= 0.6 ulp up to a 1e6 cancellation
-// ratio).  1/rho is the hardware estimate after one Newton step.
+// ratio).
 struct Point {
     float ri, u, v, w, dp;
 };
@@ -191,10 +205,7 @@ __device__ __forceinline__ Point point_values(const float* row, float ru, float 
     Point p;
     float se;
     const float s = two_sum(rh, dro, se);
-    const float x = add(s, add(se, rl));
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    p.ri = fmaf(r, fmaf(-x, r, 1.0f), r);
+    p.ri = recip32(add(s, add(se, rl)));
     const float p1 = mul(rh, dt), e1 = fmaf(rh, dt, -p1);
     const float p2 = mul(th, dro), e2 = fmaf(th, dro, -p2);
     const float p3 = mul(dro, dt), e3 = fmaf(dro, dt, -p3);

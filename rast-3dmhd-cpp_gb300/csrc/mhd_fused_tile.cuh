@@ -103,7 +103,9 @@ constexpr size_t ring_bytes() {
     return ring_doubles<SW, T>() * sizeof(double);
 }
 
-// 1/x: r is the hardware estimate, e = 1 - x r, and 1/x = r / (1 - e) = r (1 + e + e^2) + O(e^3)
+// 1/x by Chebyshev's third-order iteration: r is the hardware estimate, e = 1 - x r, and
+// 1/x = r / (1 - e) = r (1 + e + e^2) + O(e^3); within 2^-53 + 2^-59 of the value (a rounded
+// quotient's error is 2^-53)
 __device__ __forceinline__ double recip(double x, double one) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));

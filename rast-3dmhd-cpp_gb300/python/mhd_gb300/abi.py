@@ -118,6 +118,7 @@ SIGNATURES = {
     "mhd_steps_host": [C.c_void_p, C.c_int, _DP, _DP, C.c_double],
     "mhd_set_plume": [C.c_void_p, C.POINTER(MhdPlume)],
     "mhd_selftest_convert": [C.c_longlong, C.c_ulonglong, C.POINTER(C.c_longlong)],
+    "mhd_selftest_recip": [C.c_longlong, C.c_ulonglong, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)],
     "mhd_static_state": [C.POINTER(MhdParams), C.POINTER(MhdStaticParams), _DP],
     "mhd_static_lrem_profile": [C.POINTER(MhdParams), C.POINTER(MhdStaticParams), _DP, _DP, _DP],
     "mhd_diagnostics": [C.c_void_p, C.POINTER(MhdDiag)],
