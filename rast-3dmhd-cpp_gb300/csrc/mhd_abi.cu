@@ -708,12 +708,8 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     {
         const double* b0 = ctx->d_metric;
         const double** c1s[2] = {&ctx->coef.cx1, &ctx->coef.cy1};
-        const double** c2as[2] = {&ctx->coef.cx2a, &ctx->coef.cy2a};
-        const double** c2bs[2] = {&ctx->coef.cx2b, &ctx->coef.cy2b};
         for (int ax = 0; ax < 2; ax++) {
             *c1s[ax] = b0 + base_off[ax];
-            *c2as[ax] = b0 + base_off[ax] + ns[ax];
-            *c2bs[ax] = b0 + base_off[ax] + 2 * ns[ax];
             for (int k = 0; k < 8; k++)
                 (ax ? ctx->coef.yf : ctx->coef.xf)[k] =
                     reinterpret_cast<const float*>(b0 + sidef_off[ax]) + (size_t)k * ns[ax];

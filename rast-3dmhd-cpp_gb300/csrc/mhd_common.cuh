@@ -145,11 +145,10 @@ enum Scalar {
 struct Coefs {
     const double* zt[2];  // [nz][ZR_N]: any grid, uniform x / y
     const double* sc[2];  // [SC_N]
-    // per column (any grid): first-derivative factors duudu*hu, second-derivative coefficients
-    // c2a = d2uudu2*hu, c2b = duudu^2*h2u
-    const double *cx1, *cx2a, *cx2b;
-    const double *cy1, *cy2a, *cy2b;
-    // per column (any grid): c2b and c2a, scaled by ORE, ORE*C43, ORM and unscaled
+    // per column (any grid): first-derivative factors duudu*hu
+    const double *cx1, *cy1;
+    // per column (any grid): second-derivative coefficients c2b = duudu^2*h2u and
+    // c2a = d2uudu2*hu, scaled by ORE, ORE*C43, ORM and unscaled
     const double *xt[8], *yt[8];
     // for the FP32 kernels: c2b and c2a as floats, scaled alike
     const float *xf[8], *yf[8];
