@@ -242,33 +242,26 @@ int set_profile(mhd_ctx* ctx, int field, const double* host) {
 }  // namespace
 
 namespace mhd::ctxops {
-// With rho0 and T0 in h_bg: T0's premultiplied z derivatives, the float
-// coefficient table, and both uploaded.
+// With rho0 and T0 in h_bg: what the float coefficient table takes from them, and
+// both uploaded.
 int profiles_from_means(mhd_ctx* ctx) {
     const int nz = ctx->g.nz;
-    const double* bg = ctx->h_bg.data() + nz;
-    {
-        double* d1 = ctx->h_bg.data() + 2 * nz;
-        double* d2 = ctx->h_bg.data() + 3 * nz;
-        const double *cz1 = ctx->h_cz.data(), *cz2a = cz1 + nz, *cz2b = cz1 + 2 * nz;
-        for (int z = 0; z < nz; z++) {
-            d1[z] = d2[z] = 0.0;
-            if (z == 0 || z == nz - 1) continue;
-            const double p = bg[z + 1], m = bg[z - 1];
-            d1[z] = (p - m) * cz1[z];
-            d2[z] = (p - m) * cz2a[z] + (p + m - 2.0 * bg[z]) * cz2b[z];
-        }
-    }
-    // the profiles' hydrostatic residual rho0 GRAV - D_z(rho0 T0) per interior z, in
-    // FP64 (the two terms nearly cancel); the FP32 kernels add the deviations to it
-    const double* r0 = ctx->h_bg.data();
-    const double* cz1 = ctx->h_cz.data();
+    const double *r0 = ctx->h_bg.data(), *bg = r0 + nz;
+    const double *cz1 = ctx->h_cz.data(), *cz2a = cz1 + nz, *cz2b = cz1 + 2 * nz;
     for (int z = 0; z < nz; z++) {
         float* row = ctx->h_zf.data() + (size_t)z * ZF_N;
-        row[ZF_DZT] = (float)ctx->h_bg[2 * (size_t)nz + z];
-        row[ZF_D2T] = (float)ctx->h_bg[3 * (size_t)nz + z];
-        double hz = 0.0;
-        if (z > 0 && z < nz - 1) hz = r0[z] * ctx->prm.GRAV - (r0[z + 1] * bg[z + 1] - r0[z - 1] * bg[z - 1]) * cz1[z];
+        // per interior z, in FP64: T0's first and second z derivatives, and the profiles'
+        // hydrostatic residual rho0 GRAV - D_z(rho0 T0) (the two terms nearly cancel), to
+        // which the FP32 kernels add the deviations
+        double d1 = 0.0, d2 = 0.0, hz = 0.0;
+        if (z > 0 && z < nz - 1) {
+            const double p = bg[z + 1], m = bg[z - 1];
+            d1 = (p - m) * cz1[z];
+            d2 = (p - m) * cz2a[z] + (p + m - 2.0 * bg[z]) * cz2b[z];
+            hz = r0[z] * ctx->prm.GRAV - (r0[z + 1] * p - r0[z - 1] * m) * cz1[z];
+        }
+        row[ZF_DZT] = (float)d1;
+        row[ZF_D2T] = (float)d2;
         row[ZF_HZ] = (float)hz;
         // rho0 and T0 as float pairs hi + lo (hi the nearest float, lo the
         // nearest float to the exact remainder): about 48 significant bits,
@@ -282,8 +275,8 @@ int profiles_from_means(mhd_ctx* ctx) {
     // on the context's stream: its kernels read the profiles (a plain cudaMemcpy
     // runs on the legacy stream, which the non-blocking context stream does not
     // wait for); the sync keeps h_bg / h_zf stable until the copies are done
-    CK(cudaMemcpyAsync(ctx->d_bg, ctx->h_bg.data(), sizeof(double) * 4 * nz, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_bg + 4 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz, cudaMemcpyHostToDevice,
+    CK(cudaMemcpyAsync(ctx->d_bg, ctx->h_bg.data(), sizeof(double) * 2 * nz, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_bg + 2 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz, cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
@@ -393,7 +386,7 @@ int fused32_step(mhd_ctx* ctx, double dt, const double* dtp = nullptr) {
         a.FT = ctx->FT64;
         a.bgR = ctx->d_bg;
         a.bgT = ctx->d_bg + nz;
-        a.zf = reinterpret_cast<const float*>(ctx->d_bg + 4 * nz);
+        a.zf = reinterpret_cast<const float*>(ctx->d_bg + 2 * nz);
         a.gdt = gam[s] * dt;
         a.zdt = zet[s] * dt;
         a.dtp = dtp;
@@ -740,12 +733,12 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     ctx->red_blocks = 152 * 8;
     ctx->fp32 = p.precision == MHD_PREC_FP32;
     ctx->h_cz.assign(h.begin() + base_off[2], h.begin() + base_off[2] + 3 * nz);
-    ctx->h_bg.assign(4 * (size_t)nz, 0.0);
+    ctx->h_bg.assign(2 * (size_t)nz, 0.0);
     int arc = MHD_OK;
     if (ctx->fp32) {
         arc = alloc_f32(ctx, &ctx->U32[0]);
-        // 4 x nz double profiles, then the [nz][ZF_N] float coefficient table
-        const size_t bg_bytes = sizeof(double) * 4 * nz + sizeof(float) * ZF_N * nz;
+        // 2 x nz double profiles, then the [nz][ZF_N] float coefficient table
+        const size_t bg_bytes = sizeof(double) * 2 * nz + sizeof(float) * ZF_N * nz;
         if (!arc && cudaMalloc(&ctx->d_bg, bg_bytes) != cudaSuccess) arc = MHD_ERR_NOMEM;
         if (!arc && cudaMemsetAsync(ctx->d_bg, 0, bg_bytes, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
         ctx->h_zf.assign(ZF_N * (size_t)nz, 0.0f);
@@ -762,7 +755,7 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
             row[ZF_KAP] = (float)(tmpc * p.RKAPA[z]);
             row[ZF_DKAP] = (float)(tmpc * p.DKAPA[z]);
         }
-        if (!arc && cudaMemcpyAsync(ctx->d_bg + 4 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz,
+        if (!arc && cudaMemcpyAsync(ctx->d_bg + 2 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz,
                                     cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
     } else {
         arc = alloc_block(ctx, &ctx->U[0], 8);

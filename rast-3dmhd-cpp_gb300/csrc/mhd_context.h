@@ -42,11 +42,11 @@ struct mhd_ctx {
     bool fp32 = false;
     float* U32[2] = {nullptr, nullptr};
     double* FT64 = nullptr;     // persistent FT (lShr)
-    double* d_bg = nullptr;     // rho0, T0, dzT0, d2zT0 (4 x nz), then the float table
-    std::vector<double> h_bg;   // host copy of the four profiles
+    double* d_bg = nullptr;     // rho0, T0 (2 x nz), then the float table
+    std::vector<double> h_bg;   // host copy of the two profiles
     std::vector<double> h_cz;   // cz1, cz2a, cz2b (3 x nz)
     // float per-z coefficients of the FP32 kernels, [nz][ZF_N] (device copy
-    // after d_bg's 4 x nz doubles)
+    // after d_bg's 2 x nz doubles)
     std::vector<float> h_zf;
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     bool profiling = false;
