@@ -71,6 +71,9 @@ std::map<std::string, std::pair<int, int>> g_tune_cache;  // signature -> (tile,
 // reload two halo planes each.
 constexpr int kZChoices = 3;
 constexpr int kZMax[kZChoices] = {64, 32, 16};
+// every range then holds the planes of BCON, so that the candidates have no separate
+// BCON launch (a grid is cut into ranges of at least half of the limit)
+static_assert(kZMax[kZChoices - 1] >= 2 * kWallPlanes);
 constexpr int kNoLimit = 1 << 30;
 
 int bfail(mhd_batch* b, int code, const std::string& msg) {
@@ -424,19 +427,12 @@ int autotune(mhd_batch* b, double* ms_out) {
     }
     FusedArgs* d_args = nullptr;
     Fused32Args* d_args32 = nullptr;
-    int2* d_bitems = nullptr;
-    std::vector<int2> bitems;
-    make_bcon_items(b, kZMax[kZChoices - 1], bitems);
     int* d_cnt = nullptr;
     int best = 0;
     double best_ms = 1e300;
     if (!rc && cudaMalloc(&d_args, sizeof(FusedArgs) * 6 * n) != cudaSuccess) rc = MHD_ERR_NOMEM;
     if (!rc && cudaMalloc(&d_args32, sizeof(Fused32Args) * 6 * n) != cudaSuccess) rc = MHD_ERR_NOMEM;
     if (!rc && cudaMalloc(&d_cnt, sizeof(int) * 6) != cudaSuccess) rc = MHD_ERR_NOMEM;
-    if (!rc && !bitems.empty()) {
-        if (cudaMalloc(&d_bitems, sizeof(int2) * bitems.size()) != cudaSuccess) rc = MHD_ERR_NOMEM;
-        else cudaMemcpyAsync(d_bitems, bitems.data(), sizeof(int2) * bitems.size(), cudaMemcpyHostToDevice, b->stream);
-    }
     if (!rc) {
         if (b->fp32) {
             std::vector<Fused32Args> a32;
@@ -474,7 +470,7 @@ int autotune(mhd_batch* b, double* ms_out) {
             cudaMemcpyAsync(d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, b->stream);
             cudaStreamSynchronize(b->stream);
             cudaGraphExec_t ex[2] = {nullptr, nullptr};
-            rc = capture(b, t, d_args, d_args32, d_items, (int)items.size(), d_bitems, (int)bitems.size(), d_cnt, ex);
+            rc = capture(b, t, d_args, d_args32, d_items, (int)items.size(), nullptr, 0, d_cnt, ex);
             if (!rc) {
                 for (int w = 0; w < 2; w++) cudaGraphLaunch(ex[w], b->stream);
                 cudaEventRecord(e0, b->stream);
@@ -500,7 +496,6 @@ int autotune(mhd_batch* b, double* ms_out) {
     cudaStreamSynchronize(b->stream);
     cudaFree(d_args);
     cudaFree(d_args32);
-    cudaFree(d_bitems);
     cudaFree(d_cnt);
     for (void* p : owned) cudaFree(p);
     if (rc) return rc;
