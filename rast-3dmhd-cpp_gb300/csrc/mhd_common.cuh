@@ -9,6 +9,8 @@
 
 #include <cstdint>
 
+#include "mhd_split.h"
+
 namespace mhd {
 
 // Compile-time physics switches, the reference's 3dmhdparam.h:8-17 and
@@ -211,7 +213,6 @@ struct FusedArgs {
     // kWallPlanes planes that BCON involves
     int walls;
 };
-constexpr int kWallPlanes = 3;
 // Device time-step record of mhd_steps_cfl: [0] DT in use (0 once halted),
 // [1] TIMT, [2] UMACH, [3] halt flag (DT < 1e-8), [4] the CFL DT computed
 // last, [5] completed steps, [6] TIMI, [7] TIMC.
@@ -221,17 +222,6 @@ int cfl_dt_on_device(bool mag, const Grid& g, const Consts& c, Fields8 U, double
 // One substage over planes [zlo, zhi) and BCON of the walls they touch (a.walls is set here).
 int fused_substage(unsigned sw, const FusedArgs& a, cudaStream_t st);
 // the instantiation with the optional temperature terms (fused_substage calls it)
-// Blocks of a substage launch, (tile, z range) each, of planes [lo, lo + planes).
-// Every tile in `ranges` ranges, the tiles of a range one after another; or
-// (ranges = 0) up to four classes of equal length, numbered in order: block j of a
-// class is tile tile0 + j % tiles, planes [lo + z0 + len * (j / tiles), + len).
-struct ZSplit {
-    int lo, planes, nbx, tiles, ranges;
-    int first, last;  // planes of the shortest range that begins at lo, and that ends the planes
-    struct Class {
-        int blocks, tile0, tiles, z0, len;
-    } cls[4];
-};
 int fused_substage_xp(unsigned sw, const FusedArgs& a, const ZSplit& s, int blocks, cudaStream_t st);
 // Ragged batches: persistent CTAs take (instance, tile x, tile y) items from a
 // counter that must be zero at launch.  Tile shapes: 0 = 32x4, 1 = 32x8, 2 = 16x8.

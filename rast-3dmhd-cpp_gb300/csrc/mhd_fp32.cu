@@ -19,8 +19,8 @@ using namespace fp32;
 //   four of 5 rows (96)                    617  1275  2018
 //   five of 4 rows (96)                    687  1515  1980
 // Batches therefore run tiles of 4 rows, one instance the better of the two by
-// split32 below.
-constexpr int kResident = 4;
+// split32 (mhd_split.h).
+constexpr int kResident = kResident32;
 using BatchTile = Tile<kBatch32TY>;
 
 // one instance: grid (tiles, x fastest; 1; z chunks)
@@ -121,51 +121,6 @@ __global__ void k_comm32(int nf, Grid g, Fields8f U) {
     }
 }
 
-// First plane of z range k of n over `planes` planes (the kernel's split).
-int chunk_begin(int planes, int k, int n) { return (int)((long long)planes * k / n); }
-
-int fused32_walls(int planes, int chunks) {
-    return (chunk_begin(planes, 1, chunks) >= kWallPlanes ? 1 : 0) |
-           (planes - chunk_begin(planes, chunks - 1, chunks) >= kWallPlanes ? 2 : 0);
-}
-
-// Microseconds (less a constant) per launch of n CTAs: tiles of ty rows, c z ranges.
-// While all are resident, the planes of a CTA (0.4 more around a range) follow one
-// another, L each, and share their SM's issue slots with the other CTAs, q each;
-// with more CTAs than that, in waves that overlap in part, b per plane.  Last, a
-// separate BCON launch where a range at a wall is too short for it.  Fitted to
-// launches with lMag on 16 grids of 32^3 .. 512x384x96 cells, 1 .. 64 ranges and
-// both tiles: on those grids the split that it chooses is within 1 % of the fastest.
-double cost32(int ty, long long n, int sms, int planes, int c) {
-    const double L = 2.1, q = ty == 4 ? 0.47 : 0.65, b = ty == 4 ? 4.27 : 4.73;
-    const double start = ty == 4 ? 0.0 : 1.7, more = ty == 4 ? 6.4 : 7.0, f = ty == 4 ? 0.85 : 0.63;
-    const long long wave = (long long)kResident * sms, per_sm = (n + sms - 1) / sms;
-    const double most = (planes + c - 1) / c + 0.4, avg = (double)planes / c + 0.4;
-    const double waves = f * (double)n / wave + (1.0 - f) * (double)((n + wave - 1) / wave);
-    const double t = start + (n <= wave ? L * most + q * per_sm * avg : more + b * waves * avg);
-    return fused32_walls(planes, c) == 3 ? t : t + 3.1;
-}
-
-// Rows per tile and number of z ranges for one instance of nx x ny interior columns.
-struct Split32 {
-    int ty, chunks;
-};
-Split32 split32(int nx, int ny, int planes, int sms) {
-    Split32 best{5, 1};
-    double best_cost = 1e300;
-    for (int ty = 4; ty <= 5; ty++) {
-        const long long tiles = (long long)((nx + kTX - 1) / kTX) * ((ny + ty - 1) / ty);
-        for (int c = 1; c <= planes; c++) {
-            const double cost = cost32(ty, tiles * c, sms, planes, c);
-            if (cost < best_cost - 1e-9) {
-                best_cost = cost;
-                best = {ty, c};
-            }
-        }
-    }
-    return best;
-}
-
 int sm_count() {
     static const int n = [] {
         int dev = 0, sms = 0;
@@ -190,7 +145,7 @@ void launch32(const Fused32Args& args, cudaStream_t st, int* rc) {
     Fused32Args a = args;
     const int planes = a.g.nz - 2;
     const Split32 s = split32(a.g.nx - 2, a.g.ny - 2, planes, sm_count());
-    a.walls = fused32_walls(planes, s.chunks);
+    a.walls = split32_walls(planes, s.chunks);
     // (y tiles of few rows could exceed the y extent of a grid)
     const dim3 grid((a.g.nx - 2 + kTX - 1) / kTX * ((a.g.ny - 2 + s.ty - 1) / s.ty), 1, s.chunks);
     const bool extra = a.c.pl_mode == 3 || a.c.lrem;

@@ -43,7 +43,7 @@ namespace mhd {
 namespace fp32 {
 
 // 32 columns per row: a warp's shared-memory accesses touch every bank once
-constexpr int kTX = 32, kPX = kTX + 2;
+constexpr int kTX = kTX32, kPX = kTX + 2;
 template <int TY>
 struct Tile {
     static constexpr int kTY = TY;
