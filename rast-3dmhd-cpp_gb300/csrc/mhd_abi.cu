@@ -616,8 +616,9 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     // ... and the same first-derivative and 'b' coefficients in every interior column
     for (int ax = 0; ax < 2; ax++)
         for (int i = 2; i <= ns[ax] - 2; i++) uxy = uxy && c1(ax, i) == c1(ax, 1) && c2b(ax, i) == c2b(ax, 1);
-    // the unit of the uniform-grid kernels has to be an ordinary number
-    uxy = uxy && std::isnormal(c1(0, 1)) && std::isnormal(1.0 / c1(0, 1));
+    // the unit of the uniform-grid kernels: squares of y and z derivatives in that unit
+    // (heating) have to stay in range as those in true units do
+    uxy = uxy && std::fabs(c1(0, 1)) > 0x1p-200 && std::fabs(c1(0, 1)) < 0x1p200;
     // The coefficient rows and scalars of the fused kernels (mhd_common.cuh), for
     // any grid (kappa = 1) and, where it applies, for uniform x / y.
     const double tmpc = ctx->k.OCV / ctx->k.REPR, c13ore = ctx->k.C13 * ctx->k.ORE;
