@@ -26,7 +26,7 @@
 // in 3 and 11 instructions (mhd_convert.cuh): 1010 instructions per cell and
 // substage with lMag, against 1470 for the version before it, which read the z
 // neighbours' halos and had two barriers per plane.  Measured, with BCON inside:
-// a step at 256x256x128 1630 -> 1290 us, at 64x64x32 98 -> 56 us, a batch of 24
+// a step at 256x256x128 1630 -> 1262 us, at 64x64x32 98 -> 56 us, a batch of 24
 // instances 2380 -> 1870 us (see the CTA sizes in mhd_fp32.cu).  Two cells per
 // thread packed into f32x2 operations need 730 instructions per cell but 168
 // registers, 12 warps per SM: 620 us per substage against 425; updating the fields
@@ -53,10 +53,10 @@ struct Tile {
     static_assert(kHalo <= kThreads, "one halo point per thread at most");
 };
 
-// quantities of a ring plane, with halo: P_X, P_Y are dp + RU u, dp + RV v
-enum QF { F_RU = 0, F_RV, F_DT, F_U, F_V, F_W, F_PX, F_PY, F_BX, F_BY, F_BZ, F_NQ };
-// quantities of the own column only: RW, dp + RW w
-enum OF { G_RW = 0, G_PZ, G_N };
+// quantities of a ring plane, with halo
+enum QF { F_RU = 0, F_RV, F_DT, F_U, F_V, F_W, F_DP, F_BX, F_BY, F_BZ, F_NQ };
+// quantities of the own column only
+enum OF { G_RW = 0, G_N };
 // scalars
 enum SF { K_GRAV = 0, K_OMZ, K_NOMZ, K_OMX, K_NOMX, K_HQ, K_C43, K_OCV, K_OB, K_OHM, K_TMPC, K_C13ORE, K_N };
 
@@ -365,12 +365,8 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
         P[F_U * kPlane + k] = p.u;
         P[F_V * kPlane + k] = p.v;
         P[F_W * kPlane + k] = p.w;
-        P[F_PX * kPlane + k] = fmaf(r[S_RU], p.u, p.dp);
-        P[F_PY * kPlane + k] = fmaf(r[S_RV], p.v, p.dp);
-        if (own) {
-            P[kOwn + G_RW * kThreads + tid] = r[S_RW];
-            P[kOwn + G_PZ * kThreads + tid] = fmaf(r[S_RW], p.w, p.dp);
-        }
+        P[F_DP * kPlane + k] = p.dp;
+        if (own) P[kOwn + G_RW * kThreads + tid] = r[S_RW];
         if constexpr (SW::lMag) {
             P[F_BX * kPlane + k] = r[S_BX];
             P[F_BY * kPlane + k] = r[S_BY];
@@ -430,11 +426,16 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
         q3p = own_q3(Pp, ux1, vy1);
         if (active) {
             const float* R = row(z);
-            // the register: its loads (L2 hits, prefetched) are under way meanwhile
+            // the register: its loads (L2 hits, prefetched) are under way meanwhile; without
+            // lMag from after the momentum terms on (before them the 5-row tile spills, a
+            // step at 256x256x128 1101 us instead of 894)
             const int i = z * sz + oc;
             double zf[NRAW];
+            auto load_register = [&] {
 #pragma unroll
-            for (int f = 0; f < NRAW; f++) zf[f] = a.Z.p[f][i];
+                for (int f = 0; f < NRAW; f++) zf[f] = a.Z.p[f][i];
+            };
+            if constexpr (SW::lMag) load_register();
             const double t0z = a.bgT[z], r0z = a.bgR[z];
             // (constant offsets from one pointer per plane)
             const float *c0 = P0 + pc, *cp = Pp + pc, *cm = Pm + pc;
@@ -488,15 +489,20 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
             // advection (3dmhdsub.h:279-289), viscous Laplacians (3dmhdsub.h:462-472)
             const float up = XP(F_U), um = XM(F_U), vp = YP(F_V), vm = YM(F_V), wp = ZP(F_W), wm = ZM(F_W);
             const float dUz = sub(ZP(F_U), ZM(F_U)), dVz = sub(ZP(F_V), ZM(F_V)), dWz = sub(wp, wm);
-            float fu = mul(cx, sub(XM(F_PX), XP(F_PX)));
-            float fv = mul(cy, sub(YM(F_PY), YP(F_PY)));
-            float fw = fmaf(dro0, sc[K_GRAV], fmaf(cz, sub(wm_[G_PZ * kThreads], wp_[G_PZ * kThreads]), R[ZF_HZ]));
-            fu = fmaf(ncy, sub(mul(rvp, YP(F_U)), mul(rvm, YM(F_U))), fu);
-            fu = fmaf(ncz, sub(mul(rwp, ZP(F_U)), mul(rwm, ZM(F_U))), fu);
-            fv = fmaf(ncx, sub(mul(rup, XP(F_V)), mul(rum, XM(F_V))), fv);
-            fv = fmaf(ncz, sub(mul(rwp, ZP(F_V)), mul(rwm, ZM(F_V))), fv);
-            fw = fmaf(ncx, sub(mul(rup, XP(F_W)), mul(rum, XM(F_W))), fw);
-            fw = fmaf(ncy, sub(mul(rvp, YP(F_W)), mul(rvm, YM(F_W))), fw);
+            float fu = mul(cx, sub(XM(F_DP), XP(F_DP)));
+            float fv = mul(cy, sub(YM(F_DP), YP(F_DP)));
+            float fw = fmaf(dro0, sc[K_GRAV], fmaf(cz, sub(ZM(F_DP), ZP(F_DP)), R[ZF_HZ]));
+            // (each momentum flux by itself: added to dp at the points first, it would carry
+            // dp's rounding; a difference rounds one of its two products)
+            fu = fmaf(ncx, fmaf(rup, up, -mul(rum, um)), fu);
+            fv = fmaf(ncy, fmaf(rvp, vp, -mul(rvm, vm)), fv);
+            fw = fmaf(ncz, fmaf(rwp, wp, -mul(rwm, wm)), fw);
+            fu = fmaf(ncy, fmaf(rvp, YP(F_U), -mul(rvm, YM(F_U))), fu);
+            fu = fmaf(ncz, fmaf(rwp, ZP(F_U), -mul(rwm, ZM(F_U))), fu);
+            fv = fmaf(ncx, fmaf(rup, XP(F_V), -mul(rum, XM(F_V))), fv);
+            fv = fmaf(ncz, fmaf(rwp, ZP(F_V), -mul(rwm, ZM(F_V))), fv);
+            fw = fmaf(ncx, fmaf(rup, XP(F_W), -mul(rum, XM(F_W))), fw);
+            fw = fmaf(ncy, fmaf(rvp, YP(F_W), -mul(rvm, YM(F_W))), fw);
             fu = lapx(F_U, 1, lapy(F_U, 0, lapz(F_U, 0, dUz, fu)));
             fv = lapx(F_V, 0, lapy(F_V, 1, lapz(F_V, 0, dVz, fv)));
             fw = lapx(F_W, 0, lapy(F_W, 0, lapz(F_W, 1, dWz, fw)));
@@ -516,6 +522,7 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
                 fw = fmaf(R[ZF_KQZ], sub(q3p, q3m), fw);
             }
 
+            if constexpr (!SW::lMag) load_register();
             // ---- temperature (deviation stencils plus the profile's derivatives):
             // nadv collects what is subtracted, qr the terms proportional to 1/rho
             const float dTz = sub(ZP(F_DT), ZM(F_DT)), Tz = fmaf(cz, dTz, R[ZF_DZT]);
