@@ -73,10 +73,12 @@ struct Consts {
 // while the one before it on its stream drains; it reaches the memory of earlier
 // work only after wait_previous(), which returns when that work is complete and
 // visible.  launch_next() lets the next such kernel start as soon as every block of
-// this one has; without it that happens when this one ends.  The kernels call it
-// last: called first, the next kernel's blocks crowd onto the SMs that are free then
-// (a step at 64x64x32: 187 us without overlap, 253 so, 178 called last; 32x32x32 87,
-// 99, 72; FP32 storage at 64x64x32 67, 84, 59).
+// this one has called it; without it (k_flux, and the kernels launched plainly before
+// one of these) that happens when this one ends.  The substage, CFL and k_prep kernels
+// call it last: called first, the next kernel's blocks crowd onto the SMs that are free
+// then (a step at 64x64x32: 187 us without overlap, 253 so, 178 called last; 32x32x32
+// 87, 99, 72; FP32 storage at 64x64x32 67, 84, 59).  The wall kernels, a few short
+// blocks, call it after their own wait.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>

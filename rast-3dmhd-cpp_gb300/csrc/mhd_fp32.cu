@@ -9,8 +9,8 @@ namespace {
 using namespace fp32;
 
 // CTAs per SM: four, with 128 registers a thread in tiles of 4 rows (16 warps) and
-// 96 in tiles of 5 rows (20 warps), in both cases without spilling the cell's
-// register values loaded at the start of the plane.  Many small CTAs wait less at
+// 96 in tiles of 5 rows (20 warps).  Neither spills, but for 4 and 16 bytes in two
+// kernels with the optional temperature terms.  Many small CTAs wait less at
 // the barrier of a plane than few large ones.  With lMag, us per step at 200x150x100
 // and at 256x256x128, us per step of a batch of 24 instances:
 //   two CTAs of 8 rows (128 registers)     680  1364  1983

@@ -10,9 +10,11 @@ namespace {
 
 using namespace fused;
 // tile of the single-instance kernel (MHD_FUSED_TILE_X x MHD_FUSED_TILE_Y threads):
-// 16 x 8 loads 18 x 10 ring points per 128 cells (32 x 4: 34 x 6), and each
-// warp still reads whole 128-byte rows (measured: 71.7 vs 72.9 ms per step at
-// 512 x 512 x 256; 32 x 6, 32 x 8 and 16 x 12 run fewer CTAs per SM and are slower)
+// 16 x 8 loads 18 x 10 ring points per 128 cells (32 x 4: 34 x 6), and each warp still
+// reads whole 128-byte rows.  ms per step at 512 x 512 x 256, with lMag, lRot and lShr
+// and with lMag alone: 16 x 8 53.9 and 59.1; 8 x 16 55.4, 60.1; 32 x 4 56.5, 62.0; with
+// more threads and so fewer CTAs per SM 32 x 6 61.5, 69.1; 16 x 12 62.3, 70.9; 32 x 8
+// 65.9, 71.4.
 #ifndef MHD_FUSED_TILE_X
 #define MHD_FUSED_TILE_X 16
 #endif
@@ -27,6 +29,7 @@ using namespace fused;
 #endif
 constexpr bool kExtra = MHD_FUSED_XP != 0;
 using DefaultTile = Tile<MHD_FUSED_TILE_X, MHD_FUSED_TILE_Y>;
+// three CTAs per SM: 168 registers, of which some kernels spill 4 to 56 bytes
 constexpr int kMinBlocks = DefaultTile::kThreads >= 256 ? 2 : 3;
 
 // grid (x tiles, y tiles, z ranges)

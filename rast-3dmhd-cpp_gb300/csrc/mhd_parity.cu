@@ -951,6 +951,8 @@ constexpr float kCflTau = 1.52587890625e-05f;    // 2^-16: filter margin, > 2x t
 // Bound by the latency of its loads: a lane loads 4 cells (FP64: 2) before it
 // uses the first (256x256x128 with lMag, whole reduction: FP32 storage 162 -> 106
 // us, FP64 222 -> 157; with overlapped launches and seeds per block 103 and 146).
+// The price is spilling: 128 bytes stored and 148 to 160 loaded by a thread with lMag
+// (40 to 48 and 56 to 64 without) at the 80 registers of three blocks per SM.
 // The exact maximum of mc and minimum of a0 are therefore among the cells
 // evaluated exactly, and the result equals the cell-by-cell reduction bit for
 // bit; after the first passes only new near-extremes are evaluated.  Rows with varying DD, and launches whose constants break the

@@ -97,7 +97,9 @@ inline int split_walls(int nz, const ZSplit& s) {
 // with the constants for the planes around a range and its start-up; the last
 // wave counts in full because its CTAs are not spread evenly over the SMs.  A
 // range too short for BCON at the walls adds a launch (0.6).  The choice is within
-// 2 % of the fastest on those 19 grids.  Against at most eight ranges of four
+// 2 % of the fastest on those 19 grids, and within 1.1 % without lMag, with lShr and
+// with all three switches, whose planes cost 0.6 to 0.95 of the unit (nine grids of
+// 32^3 to 200x150x100, 1 .. 32 ranges and the full wave).  Against at most eight ranges of four
 // planes, us per step, launches not overlapped: 32x32x32 138 -> 87 (32 ranges of
 // one plane), 97x45x61 (no field) 344 -> 272, 128x128x64 1146 -> 1094 (BCON inside
 // the launch included).
@@ -108,8 +110,10 @@ inline long long choose_blocks(int nz, bool mixed, int resident, int nbx, long l
     const long long wave = (long long)resident * sms;
     // A slab of a host-to-host step runs beside the slabs of other substages,
     // which fill its last wave: where a plane has a wave of tiles, about two waves
-    // of long ranges (256x256x128: 8.65 ms per step with 2 ranges, 9.24 with the 8
-    // of the model below; 512x512x256: 57.3 ms with 1)
+    // of long ranges.  ms per step with the model below and so: 256x256x128 (512
+    // tiles) 8.79, 8.40; 240x248x64, 256x240x64 and 512x256x64 equal; 320x200x100
+    // (500) 7.20, 7.35; 320x320x100 (800) 10.68, 10.78.  From half a wave on it would
+    // lose: 200x150x100 (247) 3.55, 3.79; 224x232x128 (406) 6.72, 6.97.
     if (planes < nz - 2 && tiles >= wave)
         return tiles * std::max(1LL, std::min<long long>(planes, (2 * wave + tiles / 2) / tiles));
     for (int c = 1; c <= planes; c++) {
