@@ -276,8 +276,7 @@ int profiles_from_means(mhd_ctx* ctx) {
     // runs on the legacy stream, which the non-blocking context stream does not
     // wait for); the sync keeps h_bg / h_zf stable until the copies are done
     CK(cudaMemcpyAsync(ctx->d_bg, ctx->h_bg.data(), sizeof(double) * 2 * nz, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_bg + 2 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz, cudaMemcpyHostToDevice,
-                       ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_zf, ctx->h_zf.data(), sizeof(float) * ZF_N * nz, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
 }
@@ -386,7 +385,7 @@ int fused32_step(mhd_ctx* ctx, double dt, const double* dtp = nullptr) {
         a.FT = ctx->FT64;
         a.bgR = ctx->d_bg;
         a.bgT = ctx->d_bg + nz;
-        a.zf = reinterpret_cast<const float*>(ctx->d_bg + 2 * nz);
+        a.zf = ctx->d_zf;
         a.gdt = gam[s] * dt;
         a.zdt = zet[s] * dt;
         a.dtp = dtp;
@@ -738,10 +737,12 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
     int arc = MHD_OK;
     if (ctx->fp32) {
         arc = alloc_f32(ctx, &ctx->U32[0]);
-        // 2 x nz double profiles, then the [nz][ZF_N] float coefficient table
+        // the [nz][ZF_N] float coefficient table, then 2 x nz double profiles
+        static_assert(ZF_N % 2 == 0, "the profiles follow at an even number of floats");
         const size_t bg_bytes = sizeof(double) * 2 * nz + sizeof(float) * ZF_N * nz;
-        if (!arc && cudaMalloc(&ctx->d_bg, bg_bytes) != cudaSuccess) arc = MHD_ERR_NOMEM;
-        if (!arc && cudaMemsetAsync(ctx->d_bg, 0, bg_bytes, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
+        if (!arc && cudaMalloc(&ctx->d_zf, bg_bytes) != cudaSuccess) arc = MHD_ERR_NOMEM;
+        ctx->d_bg = reinterpret_cast<double*>(ctx->d_zf + (size_t)ZF_N * nz);
+        if (!arc && cudaMemsetAsync(ctx->d_zf, 0, bg_bytes, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
         ctx->h_zf.assign(ZF_N * (size_t)nz, 0.0f);
         for (int z = 0; z < nz; z++) {
             float* row = ctx->h_zf.data() + (size_t)z * ZF_N;
@@ -756,8 +757,8 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
             row[ZF_KAP] = (float)(tmpc * p.RKAPA[z]);
             row[ZF_DKAP] = (float)(tmpc * p.DKAPA[z]);
         }
-        if (!arc && cudaMemcpyAsync(ctx->d_bg + 2 * nz, ctx->h_zf.data(), sizeof(float) * ZF_N * nz,
-                                    cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
+        if (!arc && cudaMemcpyAsync(ctx->d_zf, ctx->h_zf.data(), sizeof(float) * ZF_N * nz, cudaMemcpyHostToDevice,
+                                    ctx->stream) != cudaSuccess) arc = MHD_ERR_CUDA;
     } else {
         arc = alloc_block(ctx, &ctx->U[0], 8);
     }
@@ -811,7 +812,7 @@ int mhd_destroy(mhd_ctx* ctx) {
     cudaFree(ctx->U32[0]);
     cudaFree(ctx->U32[1]);
     cudaFree(ctx->FT64);
-    cudaFree(ctx->d_bg);
+    cudaFree(ctx->d_zf);
     cudaFree(ctx->d_plume);
     cudaFree(ctx->d_lrem);
     if (ctx->h_out) cudaFreeHost(ctx->h_out);

@@ -168,7 +168,7 @@ void fill_args32(const mhd_batch* b, int zmax, const std::vector<float*>& U0, co
                 a.FT = FT[i];
                 a.bgR = c->d_bg;
                 a.bgT = c->d_bg + nz;
-                a.zf = reinterpret_cast<const float*>(c->d_bg + 2 * nz);
+                a.zf = c->d_zf;
                 a.gdt = gam[s] * b->dt[i];
                 a.zdt = zet[s] * b->dt[i];
                 a.timt = c->timt;

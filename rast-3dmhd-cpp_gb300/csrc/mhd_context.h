@@ -42,12 +42,11 @@ struct mhd_ctx {
     bool fp32 = false;
     float* U32[2] = {nullptr, nullptr};
     double* FT64 = nullptr;     // persistent FT (lShr)
-    double* d_bg = nullptr;     // rho0, T0 (2 x nz), then the float table
+    float* d_zf = nullptr;      // per-z coefficients of the FP32 kernels, [nz][ZF_N], then
+    double* d_bg = nullptr;     // rho0, T0 (2 x nz), in the same allocation
     std::vector<double> h_bg;   // host copy of the two profiles
     std::vector<double> h_cz;   // cz1, cz2a, cz2b (3 x nz)
-    // float per-z coefficients of the FP32 kernels, [nz][ZF_N] (device copy
-    // after d_bg's 2 x nz doubles)
-    std::vector<float> h_zf;
+    std::vector<float> h_zf;    // host copy of d_zf
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     bool profiling = false;
     std::vector<cudaEvent_t> prof_events;  // pairs around each substage launch
