@@ -394,6 +394,7 @@ def run_ours(args, dist: Dist) -> None:
                      "frac": achieved_gbs / hbm_peak, "traffic": traffic,
                      "traffic_note": "ncu dram read+write of one launch at 256x256x128, scaled per cell",
                      "kernel": "k_substage (fused RK3 substage)", "peak_source": f"{peak_src} hbm_gbs",
+                     "note": "share of the HBM roof; what bounds the kernel is the FP64 pipe (key fp64)",
                      "algorithmic_bytes_per_cell_step": bytes_cell_step,
                      "avg_launch_ms": 1e3 * avg_launch_s, "launches": launches},
         "fp64": {"bound": "fp64 pipe", "unit": "G FP64 inst/s",

@@ -23,7 +23,7 @@
 // plane are those of the FP64 kernel (mhd_fused_tile.cuh).  Field addresses are
 // one multiply-add each (32-bit element indices on pointers in the constant
 // bank), and the conversions between float and double run on the integer pipe
-// in 3 and 11 instructions (mhd_convert.cuh): 1010 instructions per cell and
+// in 3 and 11 instructions (mhd_convert.cuh): 1040 instructions per cell and
 // substage with lMag, against 1470 for the version before it, which read the z
 // neighbours' halos and had two barriers per plane.  Measured, with BCON inside:
 // a step at 256x256x128 1630 -> 1262 us, at 64x64x32 98 -> 56 us, a batch of 24
