@@ -129,7 +129,9 @@ const char* mhd_status_string(int status);
 
 /* ---- state transfer (dump / restart, 3dmhdio.h:20-72) ----------------- */
 /* Copy one whole field (ghosts included) host <-> device.  A download
- * synchronises the context's stream; one of the state keeps no device memory. */
+ * synchronises the context's stream; one of the state keeps no device memory
+ * in the context (those of FP32-storage contexts share 16 MB in the process, freed
+ * with the last such context). */
 int mhd_upload(mhd_ctx* ctx, int field, const double* host);
 int mhd_download(mhd_ctx* ctx, int field, double* host);
 /* All nfields state fields (5 without lMag, else 8) from / to one

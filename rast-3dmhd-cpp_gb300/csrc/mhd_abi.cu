@@ -13,9 +13,11 @@
 #include "mhd_context.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -319,12 +321,43 @@ int sync_zghosts32(mhd_ctx* ctx) {
 // Fields [field, field + nf) of the state to the host, widened on the device in
 // pieces of kStage elements.  Widening on the host (a copy of each field into a
 // fresh buffer, then one thread's loop) took 67 ms for the eight fields of
-// 256x256x128; this takes 3.5.  The pieces stand in U32[1-cur], whose values no
-// step reads but for the z ghost planes, put back afterwards, so a download keeps
-// no device memory (a buffer for it was half as much again as a 32^3 instance
-// holds).  Before the first step there is no U32[1-cur]: then in a buffer that is
-// freed again, or without memory for one in the reduction scratch.
+// 256x256x128; this takes 3.5.  A buffer for the pieces in every context was half as
+// much again as a 32^3 instance holds, so the FP32-storage contexts of the process
+// share one, freed with the last of them.  A download holds it until its stream is
+// done.  One that finds it taken by another thread, on another device or without
+// memory does not wait: its pieces stand in U32[1-cur], whose values no step reads but
+// for the z ghost planes, put back afterwards (32^3: 43 us instead of 30, two pieces
+// and that kernel), or before the first step in the reduction scratch.
 constexpr size_t kStage = 2u << 20;  // 16 MB: a piece's copy takes far longer than its kernel
+
+struct {
+    std::atomic<int> contexts{0};  // FP32-storage contexts alive
+    std::mutex taken;              // held by the download that uses the buffer
+    int device = -1;
+    double* p = nullptr;
+} g_stage;
+
+void stage_release() {
+    if (--g_stage.contexts > 0) return;
+    // (taken: a context made meanwhile is downloading, and will free it)
+    std::unique_lock<std::mutex> lock(g_stage.taken, std::try_to_lock);
+    if (!lock.owns_lock() || g_stage.contexts > 0) return;
+    cudaFree(g_stage.p);
+    g_stage.p = nullptr;
+}
+// The buffer on the current device, or null (g_stage.taken is held).
+double* stage_here() {
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    if (!g_stage.p) {
+        if (cudaMalloc(&g_stage.p, kStage * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            g_stage.p = nullptr;
+        }
+        g_stage.device = device;
+    }
+    return g_stage.device == device ? g_stage.p : nullptr;
+}
 
 int widen_to_host(mhd_ctx* ctx, double* buf, long long len, long long first, long long total, double* host) {
     for (long long at = 0; at < total; at += len) {
@@ -338,27 +371,21 @@ int widen_to_host(mhd_ctx* ctx, double* buf, long long len, long long first, lon
 
 int download32(mhd_ctx* ctx, int field, int nf, double* host) {
     const long long first = (long long)field * (long long)ctx->ncell, total = (long long)nf * (long long)ctx->ncell;
+    float* const other = ctx->U32[1 - ctx->cur];
+    std::unique_lock<std::mutex> lock(g_stage.taken, std::try_to_lock);
     int rc;
-    if (float* other = ctx->U32[1 - ctx->cur]) {
+    if (double* shared = lock.owns_lock() ? stage_here() : nullptr) {
+        rc = widen_to_host(ctx, shared, kStage, first, total, host);
+    } else if (other) {
         rc = widen_to_host(ctx, reinterpret_cast<double*>(other), (long long)std::min(kStage, 4 * ctx->ncell), first, total, host);
         if (!rc && ctx->ghosts_synced) rc = copy_zghosts32(ctx);
     } else {
-        double* own = nullptr;
-        const long long len = std::min((long long)kStage, total);
-        if (cudaMalloc(&own, (size_t)len * sizeof(double)) != cudaSuccess) {
-            own = nullptr;
-            cudaGetLastError();
-        }
-        rc = own ? widen_to_host(ctx, own, len, first, total, host)
-                 : widen_to_host(ctx, ctx->red, 8LL * ctx->red_blocks, first, total, host);
-        if (own) {
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(own);
-        }
+        rc = widen_to_host(ctx, ctx->red, 8LL * ctx->red_blocks, first, total, host);
     }
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
-    return MHD_OK;
+    // (also after an error: the buffer is given up only when nothing uses it any more)
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "cudaStreamSynchronize");
+    return rc;
 }
 
 // One FP32-storage step; dtp as for fused_step.
@@ -732,6 +759,7 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
 
     ctx->red_blocks = 152 * 8;
     ctx->fp32 = p.precision == MHD_PREC_FP32;
+    if (ctx->fp32) g_stage.contexts++;
     ctx->h_cz.assign(h.begin() + base_off[2], h.begin() + base_off[2] + 3 * nz);
     ctx->h_bg.assign(2 * (size_t)nz, 0.0);
     int arc = MHD_OK;
@@ -801,6 +829,7 @@ int mhd_create(const mhd_params* params, void* stream, mhd_ctx** out) {
 int mhd_destroy(mhd_ctx* ctx) {
     if (!ctx) return MHD_ERR_INVALID;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->fp32) stage_release();
     cudaFree(ctx->d_metric);
     cudaFree(ctx->U[0]);
     cudaFree(ctx->U[1]);

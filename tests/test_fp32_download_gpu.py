@@ -76,3 +76,31 @@ def test_batch_goes_on_after_downloads():
 
     for got, ref in zip(run(True), run(False)):
         assert np.array_equal(got, ref)
+
+
+def test_downloads_of_several_threads():
+    """Downloads at the same time, of which one holds the shared buffer and the
+    others go through their own contexts: each gets its state, and stepping goes
+    on from it."""
+    from concurrent.futures import ThreadPoolExecutor
+    sizes = [(20, 12, 9), (33, 8, 6), (64, 48, 40), (70, 60, 50)]
+    sims = [started(s)[1] for s in sizes]
+    refs = [started(s)[1] for s in sizes]
+    for s in sims + refs:
+        s.steps(2)
+    want = [whole(s) for s in refs]
+
+    def often(sim):
+        return [whole(sim) for _ in range(20)]
+
+    with ThreadPoolExecutor(len(sims)) as ex:
+        got = list(ex.map(often, sims))
+    for g, w in zip(got, want):
+        for a in g:
+            assert np.array_equal(a, w)
+    for s, r in zip(sims, refs):
+        s.steps(3)
+        r.steps(3)
+        assert np.array_equal(whole(s), whole(r))
+        s.close()
+        r.close()
