@@ -9,10 +9,11 @@ namespace {
 using namespace fp32;
 
 // CTAs per SM: four, with 128 registers a thread in tiles of 4 rows (16 warps) and
-// 96 in tiles of 5 rows (20 warps).  Neither spills, but for 4 and 16 bytes in two
-// kernels with the optional temperature terms.  Many small CTAs wait less at
-// the barrier of a plane than few large ones.  With lMag, us per step at 200x150x100
-// and at 256x256x128, us per step of a batch of 24 instances:
+// 96 in tiles of 5 rows (20 warps).  Neither spills, but for 4 bytes in one kernel.
+// Many small CTAs wait less at the barrier of a plane than few large ones.  With lMag,
+// us per step at 200x150x100 and at 256x256x128, us per step of a batch of 24 instances
+// (all before points beyond the grid were left out, which takes 8 % off the first and
+// 5 % off the batches, and before the ring held the pressure deviation, 1 to 3 %):
 //   two CTAs of 8 rows (128 registers)     680  1364  1983
 //   two of 10 rows (96)                    670  1335  2019
 //   four of 4 rows (128)                   651  1357  1867

@@ -263,12 +263,15 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
         hkind = 2;
     }
     const int hx = x0 - 1 + hk % kPX, hy = y0 - 1 + hk / kPX;
-    // Element indices of the points in plane 0 (a field has fewer than 2^31
-    // elements); points beyond the grid read its last column or row instead (no
-    // active cell uses them).
+    // Points beyond the grid, which no active cell uses, are not read: those of the
+    // halo are left out and the columns filled with zeros (reading the last column in
+    // their stead, lanes with one address, made a step at 33x300x61 306 us instead of 197)
+    const bool own_in = x < g.nx && y < g.ny;
+    if (hx >= g.nx || hy >= g.ny) hkind = -1;
+    // element indices of the points in plane 0 (a field has fewer than 2^31 elements)
     const int sz = (int)g.sz;
-    auto at = [&](int px, int py) { return min(py, g.ny - 1) * (int)g.sy + min(px, g.nx - 1); };
-    const int oc = at(x, y), ohc = at(hx, hy);
+    const int oc = own_in ? y * (int)g.sy + x : 0, ohc = hy * (int)g.sy + hx;
+    const int own_bytes = own_in ? 4 : 0;
 
     // Copy the raw fields of this thread's points of plane z into an [nraw][plane]
     // area (cp.async of 4 bytes: the rows of an unpadded FP32 field are not
@@ -279,7 +282,7 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
 #pragma unroll
         for (int f = 0; f < NRAW; f++) {
             const unsigned dst = (unsigned)__cvta_generic_to_shared(to + f * kPlane + pc);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(a.U.p[f] + i) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(a.U.p[f] + i), "r"(own_bytes) : "memory");
         }
         if (hkind >= 0) {
             const int j = z * sz + ohc;
@@ -293,7 +296,7 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
     };
     // the tile's rows of a plane of the register and FT into L2: 32 doubles lie in
     // two or three 128-byte lines, the last of which the next tile's rows share
-    const bool fetch = (tx & 15) == 0;
+    const bool fetch = (tx & 15) == 0 && own_in;
     auto prefetch = [&](int z) {
         if (fetch && z < g.nz - 1) {
 #pragma unroll
@@ -427,15 +430,15 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
         if (active) {
             const float* R = row(z);
             // the register: its loads (L2 hits, prefetched) are under way meanwhile; without
-            // lMag from after the momentum terms on (before them the 5-row tile spills, a
-            // step at 256x256x128 1101 us instead of 894)
+            // lMag and with the optional terms from after the momentum terms on (before them
+            // the 5-row tile spills, without lMag a step at 256x256x128 1101 us instead of 894)
             const int i = z * sz + oc;
             double zf[NRAW];
             auto load_register = [&] {
 #pragma unroll
                 for (int f = 0; f < NRAW; f++) zf[f] = a.Z.p[f][i];
             };
-            if constexpr (SW::lMag) load_register();
+            if constexpr (SW::lMag && !EXTRA) load_register();
             const double t0z = a.bgT[z], r0z = a.bgR[z];
             // (constant offsets from one pointer per plane)
             const float *c0 = P0 + pc, *cp = Pp + pc, *cm = Pm + pc;
@@ -522,7 +525,7 @@ __device__ __forceinline__ void substage32_tile(const Fused32Args& a, int bx, in
                 fw = fmaf(R[ZF_KQZ], sub(q3p, q3m), fw);
             }
 
-            if constexpr (!SW::lMag) load_register();
+            if constexpr (!SW::lMag || EXTRA) load_register();
             // ---- temperature (deviation stencils plus the profile's derivatives):
             // nadv collects what is subtracted, qr the terms proportional to 1/rho
             const float dTz = sub(ZP(F_DT), ZM(F_DT)), Tz = fmaf(cz, dTz, R[ZF_DZT]);
