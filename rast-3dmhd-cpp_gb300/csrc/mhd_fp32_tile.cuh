@@ -26,8 +26,8 @@
 // in 3 and 11 instructions (mhd_convert.cuh): 1040 instructions per cell and
 // substage with lMag, against 1470 for the version before it, which read the z
 // neighbours' halos and had two barriers per plane.  Measured, with BCON inside:
-// a step at 256x256x128 1630 -> 1262 us, at 64x64x32 98 -> 56 us, a batch of 24
-// instances 2380 -> 1870 us (see the CTA sizes in mhd_fp32.cu).  Two cells per
+// a step at 256x256x128 1630 -> 1262 us, at 64x64x32 98 -> 57 us, a batch of 24
+// instances 2400 -> 1815 us (see the CTA sizes in mhd_fp32.cu).  Two cells per
 // thread packed into f32x2 operations need 730 instructions per cell but 168
 // registers, 12 warps per SM: 620 us per substage against 425; updating the fields
 // of a plane in four groups, each where its right-hand sides are complete, was 2 %

@@ -135,8 +135,8 @@ class Server:
         self.zrange = {"fp64": None, "fp32": None}
         self.balance = balance
         # nominal cell-RK3-updates/s of a batch per precision (the 64-instance batch, measured:
-        # 1.07e9 and 5.47e9)
-        self.rates = dict(rates or {"fp64": 1.07e9, "fp32": 5.5e9})
+        # 1.07e9 and 5.38e9)
+        self.rates = dict(rates or {"fp64": 1.07e9, "fp32": 5.4e9})
         self.progress = progress
         self.progress_s = float(progress_s)
         self.completed = 0
